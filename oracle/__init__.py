@@ -44,7 +44,8 @@ REFERENCE_DIR = os.environ.get("PCX_REFERENCE", "/root/reference")
 def build() -> None:
     """Compile liboracle.so (and the reference shim when the sources exist)."""
     ref = Path(REFERENCE_DIR)
-    args = [f"REF={ref}"] if ref.is_dir() else []
+    here = any((ref / d / "fft.hpp").is_file() for d in (".", "inc", "inc/simd_impl"))    # an empty folder has none
+    args = [f"REF={ref}"] if here else []
     subprocess.run(["make", "-s", "-C", str(HERE), *args], check=True)
 
 
