@@ -278,6 +278,8 @@ static int plan_init_tables(pcx_plan_s* p) {
             v3_args z3{};
             e = pcx_v3_single(f64, log_n, z3, 0, p->sms, true);
             if (e != cudaErrorNotSupported) PCX_CUDA_TRY(e);
+            e = pcx_v3_single_any(f64, log_n, z3, 0, p->sms, true);
+            if (e != cudaErrorNotSupported) PCX_CUDA_TRY(e);
         } else {
             PCX_CUDA_TRY(pcx_v2_stage_twiddles(p->log_n1, nullptr, f64, 0, &e1));
             PCX_CUDA_TRY(pcx_v2_stage_twiddles(p->log_n2, nullptr, f64, 0, &e2));
@@ -323,7 +325,8 @@ static int plan_init_tables(pcx_plan_s* p) {
             PCX_CUDA_TRY(pcx_fourstep_tables(p->log_n2, p->fst2, f64, 0, &f2));
             // N = 8192 in FP32 also has a one-pass form (64 KB rows in shared memory)
             v3_args z3{};
-            if (pcx_v3_single(f64, log_n, z3, 0, p->sms, true) == cudaSuccess) {
+            if (pcx_v3_single(f64, log_n, z3, 0, p->sms, true) == cudaSuccess &&
+                pcx_v3_single_any(f64, log_n, z3, 0, p->sms, true) == cudaSuccess) {
                 int e3 = 0;
                 PCX_CUDA_TRY(pcx_v2_stage_twiddles(log_n, nullptr, f64, 0, &e3));
                 PCX_CUDA_TRY(cudaMalloc(&p->stw_one, (size_t)std::max(e3, 2) * eb));
@@ -774,26 +777,35 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
     h.conj_out = io.conj_out;
     h.scale    = io.scale;
 
+    // One-pass TMA-fed kernel (k_single3): its default form at the default packs
+    // and full rows, else its any-pack form.
+    const bool tma_rows    = batch == 1 || (sstride % vreals == 0 && dstride % vreals == 0);
+    auto       run_single3 = [&](const void* stw) {
+        v3_args t3{};
+        t3.src        = src;
+        t3.dst        = dst;
+        t3.src_stride = (long long)sstride;
+        t3.dst_stride = (long long)dstride;
+        t3.batch      = (long long)batch;
+        t3.conj_in    = io.conj_in;
+        t3.conj_out   = io.conj_out;
+        t3.order_in   = io.order_in;
+        t3.order_out  = io.order_out;
+        t3.scale      = io.scale;
+        t3.stw        = stw;
+        t3.error      = p->err;
+        t3.lp_src     = io.lp_src;
+        t3.lp_dst     = io.lp_dst;
+        t3.src_len    = io.src_len;
+        const bool plain = src_len == n && io.lp_src == lp_def && io.lp_dst == lp_def;
+        return plain ? pcx_v3_single(f64, p->log_n, t3, st, p->sms, false)
+                     : pcx_v3_single_any(f64, p->log_n, t3, st, p->sms, false);
+    };
+
     if (!p->two_pass) {
-        // TMA-fed kernel: any order, default pack, full-length rows on 16-byte strides
-        const size_t vr = 16 / (f64 ? sizeof(double) : sizeof(float));
-        const bool   tma = src_len == n && io.lp_src == lp_def && io.lp_dst == lp_def && p->log_n >= 5 &&
-                         (batch == 1 || (sstride % vr == 0 && dstride % vr == 0));
-        if (tma) {
-            v3_args t3{};
-            t3.src        = src;
-            t3.dst        = dst;
-            t3.src_stride = (long long)sstride;
-            t3.dst_stride = (long long)dstride;
-            t3.batch      = (long long)batch;
-            t3.conj_in    = io.conj_in;
-            t3.conj_out   = io.conj_out;
-            t3.order_in   = io.order_in;
-            t3.order_out  = io.order_out;
-            t3.scale      = io.scale;
-            t3.stw        = p->stwL;
-            t3.error      = p->err;
-            cudaError_t e = pcx_v3_single(f64, p->log_n, t3, st, p->sms, false);
+        // TMA-fed kernel: any order and pack width, rows on 16-byte strides
+        if (p->log_n >= 5 && tma_rows) {
+            const cudaError_t e = run_single3(p->stwL);
             if (e != cudaErrorNotSupported) {
                 PCX_CUDA_TRY(e);
                 return PCX_OK;
@@ -823,23 +835,9 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
     }
 
     const bool tuned_one = ws || p->form == PCX_FORM_DEFAULT || p->form == PCX_FORM_ONEPASS;
-    if (p->stw_one && tuned_one && src_len == n && io.lp_src == lp_def && io.lp_dst == lp_def &&
-        (batch == 1 || (sstride % vreals == 0 && dstride % vreals == 0))) {
+    if (p->stw_one && tuned_one && tma_rows) {
         // one-pass form of a two-pass size
-        v3_args t3{};
-        t3.src        = src;
-        t3.dst        = dst;
-        t3.src_stride = (long long)sstride;
-        t3.dst_stride = (long long)dstride;
-        t3.batch      = (long long)batch;
-        t3.conj_in    = io.conj_in;
-        t3.conj_out   = io.conj_out;
-        t3.order_in   = io.order_in;
-        t3.order_out  = io.order_out;
-        t3.scale      = io.scale;
-        t3.stw        = p->stw_one;
-        t3.error      = p->err;
-        cudaError_t e = pcx_v3_single(f64, p->log_n, t3, st, p->sms, false);
+        const cudaError_t e = run_single3(p->stw_one);
         if (e != cudaErrorNotSupported) {
             PCX_CUDA_TRY(e);
             return PCX_OK;

@@ -483,6 +483,10 @@ struct v3_args {
     double      scale;
     const void* stw;
     int*        error;    // set when a bounded wait gives up
+    // the any-pack form only (k_single3 with ANY):
+    int         lp_src;     // log2 pack widths
+    int         lp_dst;
+    int         src_len;    // valid source elements per row (zero-extended to N)
 };
 
 // Read (re, im) stored `pk_off` reals apart at `o`; lanes with bit SW set
@@ -528,14 +532,23 @@ __host__ __device__ constexpr int single3_smem() {
                : single3_base_smem<T, LOGL, NT>();
 }
 
-template<class T, int LOGL, int LP, int NT>
+// ANY: source and destination packs of any width up to N (each its own, given
+// at run time) and rows shorter than N.  The row is the same 2*N contiguous
+// reals at every width and lds_swapped / sts_swapped stay free of bank
+// conflicts at widths 1..16, so the form costs an index per element (none in
+// natural order with packs of at most TT elements: one base per thread).
+// Bound by the load/store pipe and HBM like the default form.  2048 points,
+// 5003 rows, rows of 1500 interleaved samples to packed spectra and packed
+// spectra to interleaved rows: the general kernel (plain loads into one
+// buffer, twiddles from global memory) 170 us, this
+// one 91 us for both.
+template<class T, int LOGL, int LP, int NT, bool ANY = false>
 __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
     using P             = splan<LOGL>;
     constexpr int L     = P::L;
     constexpr int E     = P::E;
     constexpr int TT    = P::TT;
     constexpr int M     = NT / TT;
-    constexpr int PK    = 1 << LP;
     constexpr int PADR  = single3_pad<TT>();
     constexpr int RS    = 2 * L + PADR;    // shared-memory row stride (reals)
     constexpr int TILE  = M * RS;
@@ -562,7 +575,15 @@ __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
     const int        m   = tid / TT;
     const int        t   = tid - m * TT;
     const long long  ntile = (a.batch + M - 1) / M;
-    const bool       contig_in  = PADR == 0 && a.src_stride == 2 * L;
+    const int        lps  = ANY ? a.lp_src : LP;
+    const int        lpd  = ANY ? a.lp_dst : LP;
+    const int        pks  = 1 << lps;
+    const int        pkd  = 1 << lpd;
+    // short rows: copied up to the 16-byte unit of the last valid real
+    const bool       cut  = ANY && a.src_len < L;
+    const uint32_t   rowb = cut ? ((pk_re((uint32_t)a.src_len - 1, lps) + pks + 1) * (uint32_t)sizeof(T) + 15) & ~15u
+                                : (uint32_t)ROWB;
+    const bool       contig_in  = PADR == 0 && a.src_stride == 2 * L && !cut;
     const bool       contig_out = PADR == 0 && a.dst_stride == 2 * L;
 
     if constexpr (SH) stage_tw_to_smem<P, T>(tws, a.stw, tid, NT);
@@ -577,11 +598,11 @@ __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
         const int  rows = (int)min((long long)M, a.batch - tile * M);
         T*         buf  = in0 + s * TILE;
         const T*   g    = src + tile * M * a.src_stride;
-        mbar_arrive_expect_tx(&full[s], (uint32_t)rows * ROWB);
+        mbar_arrive_expect_tx(&full[s], (uint32_t)rows * rowb);
         if (contig_in) {
-            bulk_g2s(buf, g, (uint32_t)rows * ROWB, &full[s]);
+            bulk_g2s(buf, g, (uint32_t)rows * rowb, &full[s]);
         } else {
-            for (int r = 0; r < rows; ++r) bulk_g2s(buf + r * RS, g + r * a.src_stride, ROWB, &full[s]);
+            for (int r = 0; r < rows; ++r) bulk_g2s(buf + r * RS, g + r * a.src_stride, rowb, &full[s]);
         }
     };
     if (tid == 0) {
@@ -606,13 +627,29 @@ __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
         }
         const T* in = in0 + s * TILE;
         cpx<T>   v[E];
-        static_for<E>([&](auto ic) {
-            constexpr int  i  = decltype(ic)::value;
-            const uint32_t p  = order_pos(t + i * TT, a.order_in, LOGL);
-            const int      o  = m * RS + pk<LP>((int)p);
-            const cpx<T>   x  = lds_swapped<T, SW>(in, o, PK);    // halves of a warp on disjoint banks
-            v[i]              = {x.re, a.conj_in ? -x.im : x.im};
-        });
+        if (ANY && a.order_in == 0 && pks <= TT) {
+            // element t + i*TT lies 2*i*TT reals after element t at any such width
+            const int o = m * RS + (int)pk_re(t, lps);
+            static_for<E>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                const cpx<T>  x = lds_swapped<T, SW>(in, o + 2 * i * TT, pks);
+                v[i]            = {x.re, a.conj_in ? -x.im : x.im};
+            });
+        } else {
+            static_for<E>([&](auto ic) {
+                constexpr int  i  = decltype(ic)::value;
+                const uint32_t p  = order_pos(t + i * TT, a.order_in, LOGL);
+                const int      o  = m * RS + (ANY ? (int)pk_re(p, lps) : pk<LP>((int)p));
+                const cpx<T>   x  = lds_swapped<T, SW>(in, o, pks);    // halves of a warp on disjoint banks
+                v[i]              = {x.re, a.conj_in ? -x.im : x.im};
+            });
+        }
+        if (cut) {    // forward only, so the source is in natural order
+            static_for<E>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                if (t + i * TT >= a.src_len) v[i] = {T(0), T(0)};
+            });
+        }
         fence_proxy_async_smem();
         __syncthreads();    // stage s consumed: refill it with the tile after next
         if (tid == 0 && tile + 2 * (long long)gridDim.x < ntile) issue(tile + 2 * (long long)gridDim.x, s);
@@ -627,13 +664,23 @@ __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
             constexpr int G   = E / (1 << P::rbits(S));
             const T       sc  = T(a.scale);
             const T       sim = a.conj_out ? -sc : sc;
-            static_for<E>([&](auto ic) {
-                constexpr int  i = decltype(ic)::value;
-                constexpr int  g = i % G, j = i / G;
-                const uint32_t kf = stage_out_index<P, S>(t, g, j);
-                const int      o  = m * RS + pk<LP>((int)order_pos(kf, a.order_out, LOGL));
-                sts_swapped<T, SW>(stg, o, PK, v[i].re * sc, v[i].im * sim);
-            });
+            if (ANY && a.order_out == 0 && pkd <= TT) {
+                // the last stage leaves frequency t + i*TT in v[i]
+                const int o = m * RS + (int)pk_re(t, lpd);
+                static_for<E>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    sts_swapped<T, SW>(stg, o + 2 * i * TT, pkd, v[i].re * sc, v[i].im * sim);
+                });
+            } else {
+                static_for<E>([&](auto ic) {
+                    constexpr int  i = decltype(ic)::value;
+                    constexpr int  g = i % G, j = i / G;
+                    const uint32_t kf = stage_out_index<P, S>(t, g, j);
+                    const uint32_t p  = order_pos(kf, a.order_out, LOGL);
+                    const int      o  = m * RS + (ANY ? (int)pk_re(p, lpd) : pk<LP>((int)p));
+                    sts_swapped<T, SW>(stg, o, pkd, v[i].re * sc, v[i].im * sim);
+                });
+            }
         }
         __syncthreads();
         const int rows = (int)min((long long)M, a.batch - tile * M);

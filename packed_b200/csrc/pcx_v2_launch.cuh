@@ -32,6 +32,22 @@ inline cudaError_t persistent_grid(K kern, int nt, int bytes, long long tiles, i
     return cudaSuccess;
 }
 
+template<class T, int LOGL, bool ANY>
+cudaError_t launch_single3(const v3_args& a, cudaStream_t st, int sms, bool attr_only) {
+    constexpr int NT    = LOGL >= 13 ? 512 : 256;    // 16 elements per thread
+    constexpr int M     = NT / splan<LOGL>::TT;
+    constexpr int bytes = single3_smem<T, LOGL, NT>();
+    auto          kern  = k_single3<T, LOGL, v2cfg<T>::LP, NT, ANY>;
+    if (attr_only) return set_smem(kern, bytes);
+    const long long tiles = (a.batch + M - 1) / M;
+    if (tiles == 0) return cudaSuccess;
+    unsigned    grid = 0;
+    cudaError_t e    = persistent_grid(kern, NT, bytes, tiles, sms, &grid);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, NT, bytes, st>>>(a);
+    return cudaGetLastError();
+}
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no -lcuda).
 inline cudaError_t encode_tensor_map(CUtensorMap* map, bool f64, int rank, void* base, const cuuint64_t* dims,
                                      const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* estr) {
