@@ -172,45 +172,67 @@ size_t pcx_plan_s::chunk_rows(size_t batch) const {
 
 // Make `v` the plan's one-launch four-step variant: its split's tables (W_N
 // tables, W_{16 N2}, full stage tables), generated again only when the split
-// changes, and its tile counts and resident blocks per SM.
+// changes, and its tile counts and resident blocks per SM.  The first variant
+// chosen is the size's default one and keeps its tables.
 static int fs_select(pcx_plan_s* p, const fs_variant& v) {
     const bool f64 = p->dtype == PCX_F64;
     if (v.l1 + v.l2 != p->log_n) return pcx_fail(PCX_ERR_INVALID, "four-step variant of another size");
-    int tc = 0, tr = 0, per_sm = 0;
-    const cudaError_t ea = pcx_fourstep(f64, v, fs_args{}, 0, p->sms, true, &tc, &tr, &per_sm);
+    fs_choice         c{};
+    const cudaError_t ea = pcx_fourstep(f64, v, fs_args{}, 0, p->sms, true, &c.tc, &c.tr, &c.per_sm);
     if (ea != cudaSuccess) {
         cudaGetLastError();
         return pcx_fail(ea == cudaErrorNotSupported ? PCX_ERR_UNSUPPORTED : PCX_ERR_CUDA,
                         std::string("four-step variant: ") + cudaGetErrorString(ea));
     }
-    if (p->fs_tab_l1 != v.l1 || !p->fs_mem) {
+    const fs_choice* same = nullptr;    // tables of the same split
+    if (p->fs.mem && p->fs.var.l1 == v.l1) same = &p->fs;
+    if (p->fs_def.mem && p->fs_def.var.l1 == v.l1) same = &p->fs_def;
+    if (same) {
+        const int tc = c.tc, tr = c.tr, per_sm = c.per_sm;
+        c        = *same;
+        c.tc     = tc;
+        c.tr     = tr;
+        c.per_sm = per_sm;
+    } else {
         const size_t eb = p->elem_bytes();
         const int    n1 = 1 << v.l1, n2 = 1 << v.l2;
         int          f1 = 0, f2 = 0;
         PCX_CUDA_TRY(pcx_fourstep_tables(v.l1, nullptr, f64, 0, &f1));
         PCX_CUDA_TRY(pcx_fourstep_tables(v.l2, nullptr, f64, 0, &f2));
-        if (p->fs_mem) cudaFree(p->fs_mem);
-        p->fs_mem    = nullptr;
-        p->fs_tab_l1 = 0;
-        const size_t ent = (size_t)n1 + 2 * (size_t)n2 + f1 + f2;
-        PCX_CUDA_TRY(cudaMalloc(&p->fs_mem, ent * eb));
-        char* b    = static_cast<char*>(p->fs_mem);
-        p->fs_thi  = b;
-        p->fs_tlo  = b + (size_t)n1 * eb;
-        p->fs_tb   = b + ((size_t)n1 + n2) * eb;
-        p->fs_st1  = b + ((size_t)n1 + 2 * n2) * eb;
-        p->fs_st2  = b + ((size_t)n1 + 2 * n2 + f1) * eb;
-        PCX_CUDA_TRY(pcx_gen_twiddles(p->fs_thi, n1, p->log_n, n2, f64, 0));
-        PCX_CUDA_TRY(pcx_gen_twiddles(p->fs_tlo, n2, p->log_n, 1, f64, 0));
-        PCX_CUDA_TRY(pcx_gen_twiddles(p->fs_tb, n2, v.l2 + 4, 1, f64, 0));
-        PCX_CUDA_TRY(pcx_fourstep_tables(v.l1, p->fs_st1, f64, 0, &f1));
-        PCX_CUDA_TRY(pcx_fourstep_tables(v.l2, p->fs_st2, f64, 0, &f2));
-        p->fs_tab_l1 = v.l1;
+        // the default variant, which the kernel's other forms run, has their
+        // twiddle table as well, plans of a permuted order a second one by
+        // bit-reversed column
+        const size_t tw = (size_t)(n1 / 16 + 5) * n2;
+        const size_t nt = p->fs_def.mem ? 0 : (p->order != PCX_ORDER_NORMAL ? 2 : 1);
+        PCX_CUDA_TRY(cudaMalloc(&c.mem, ((size_t)n1 + 2 * (size_t)n2 + f1 + f2 + nt * tw) * eb));
+        char* b = static_cast<char*>(c.mem);
+        c.thi   = b;
+        c.tlo   = b + (size_t)n1 * eb;
+        c.tb    = b + ((size_t)n1 + n2) * eb;
+        c.st1   = b + ((size_t)n1 + 2 * n2) * eb;
+        c.st2   = b + ((size_t)n1 + 2 * n2 + f1) * eb;
+        cudaError_t e = pcx_gen_twiddles(c.thi, n1, p->log_n, n2, f64, 0);
+        if (e == cudaSuccess) e = pcx_gen_twiddles(c.tlo, n2, p->log_n, 1, f64, 0);
+        if (e == cudaSuccess) e = pcx_gen_twiddles(c.tb, n2, v.l2 + 4, 1, f64, 0);
+        if (e == cudaSuccess) e = pcx_fourstep_tables(v.l1, c.st1, f64, 0, &f1);
+        if (e == cudaSuccess) e = pcx_fourstep_tables(v.l2, c.st2, f64, 0, &f2);
+        for (size_t i = 0; i < nt && e == cudaSuccess; ++i) {
+            const unsigned grid = (unsigned)((tw + 255) / 256);
+            void*          o    = b + ((size_t)n1 + 2 * (size_t)n2 + f1 + f2 + i * tw) * eb;
+            (i ? c.twr : c.tw)  = o;
+            if (f64) k_fs_twiddles<double><<<grid, 256>>>(static_cast<cpx<double>*>(o), n1 / 16, v.l2, p->log_n, i);
+            else k_fs_twiddles<float><<<grid, 256>>>(static_cast<cpx<float>*>(o), n1 / 16, v.l2, p->log_n, i);
+            e = cudaGetLastError();
+        }
+        if (e != cudaSuccess) {
+            cudaFree(c.mem);
+            PCX_CUDA_TRY(e);
+        }
     }
-    p->fs_var    = v;
-    p->fs_tc     = tc;
-    p->fs_tr     = tr;
-    p->fs_per_sm = per_sm;
+    c.var = v;
+    if (p->fs.mem && p->fs.mem != c.mem && p->fs.mem != p->fs_def.mem) cudaFree(p->fs.mem);
+    p->fs = c;
+    if (!p->fs_def.mem) p->fs_def = c;
     return PCX_OK;
 }
 
@@ -307,12 +329,13 @@ static int plan_init_tables(pcx_plan_s* p) {
                 PCX_CUDA_TRY(cudaEventCreateWithFlags(&p->ev_row[i], cudaEventDisableTiming));
             }
             PCX_CUDA_TRY(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
-            // one launch for all chunks of a batch
             // one launch for a whole batch: the size's first built-in variant
-            p->fs_tc = p->fs_tr = 0;
             for (const fs_variant& v: fs_candidates(p)) {
                 if (fs_select(p, v) == PCX_OK) break;
-                p->fs_tc = p->fs_tr = 0;
+            }
+            // its forms for other packs, short sources and permuted orders (where built)
+            for (auto form: {pcx_fs_any, pcx_fs_out, pcx_fs_in}) {
+                if (form(f64, p->fs_def.var, fs_args{}, 0, p->sms, true) != cudaSuccess) (void)cudaGetLastError();
             }
             // full stage tables of the two sub-transforms (the TMA-fed passes)
             int f1 = 0, f2 = 0;
@@ -391,9 +414,10 @@ void pcx_plan_s::release() {
     if (stw) cudaFree(stw);
     if (stw_one) cudaFree(stw_one);
     if (fst) cudaFree(fst);
-    if (fs_mem) cudaFree(fs_mem);
-    fs_mem    = nullptr;
-    fs_tab_l1 = 0;
+    if (fs.mem && fs.mem != fs_def.mem) cudaFree(fs.mem);
+    if (fs_def.mem) cudaFree(fs_def.mem);
+    fs     = {};
+    fs_def = {};
     if (fs_ctr) cudaFree(fs_ctr);
     if (par_buf) cudaFree(par_buf);
     par_buf   = nullptr;
@@ -461,10 +485,10 @@ pcx_tune_result plan_choice(const pcx_plan_s* p, double ms) {
     r.form          = p->form;
     r.rounds        = p->fs_rounds;
     r.chunk_bytes   = p->chunk_bytes;
-    r.log_n1        = p->fs_var.l1;
-    r.log_n2        = p->fs_var.l2;
-    r.blocks_per_sm = p->fs_var.minb;
-    r.stages        = p->fs_var.st;
+    r.log_n1        = p->fs.var.l1;
+    r.log_n2        = p->fs.var.l2;
+    r.blocks_per_sm = p->fs.var.minb;
+    r.stages        = p->fs.var.st;
     r.ms            = ms;
     return r;
 }
@@ -513,7 +537,7 @@ extern "C" int pcx_plan_tune(pcx_plan plan, size_t batch, void* stream, int* for
         };
         std::vector<cand> cands;
         if (p->stw_one) cands.push_back({PCX_FORM_ONEPASS, 3, 0, {}});
-        if (p->fs_tc > 0) {
+        if (p->fs.tc > 0) {
             for (const fs_variant& v: fs_candidates(p)) {
                 for (int r: {2, 3, 6}) cands.push_back({PCX_FORM_FUSED, r, 0, v});
             }
@@ -530,7 +554,7 @@ extern "C" int pcx_plan_tune(pcx_plan plan, size_t batch, void* stream, int* for
             if (e1) cudaEventDestroy(e1);
         };
         const pcx_tune_result keep = plan_choice(p, 0.0);
-        const fs_variant      keep_var = p->fs_var;
+        const fs_variant      keep_var = p->fs.var;
         auto restore = [&]() {
             if (keep_var.l1 > 0) fs_select(p, keep_var);
             p->form        = keep.form;
@@ -551,7 +575,7 @@ extern "C" int pcx_plan_tune(pcx_plan plan, size_t batch, void* stream, int* for
         float        best_ms = 0.f;
         cand         best{keep.form, keep.rounds, keep.chunk_bytes, keep_var};
         for (const cand& c: cands) {
-            if (c.form == PCX_FORM_FUSED && !(c.v == p->fs_var) && fs_select(p, c.v) != PCX_OK) continue;
+            if (c.form == PCX_FORM_FUSED && !(c.v == p->fs.var) && fs_select(p, c.v) != PCX_OK) continue;
             p->form        = c.form;
             p->fs_rounds   = c.rounds;
             p->chunk_bytes = c.chunk;
@@ -589,7 +613,7 @@ extern "C" int pcx_plan_tune(pcx_plan plan, size_t batch, void* stream, int* for
                 cleanup();
                 return rc;
             }
-        } else if (keep_var.l1 > 0 && !(p->fs_var == keep_var)) {
+        } else if (keep_var.l1 > 0 && !(p->fs.var == keep_var)) {
             fs_select(p, keep_var);
         }
         p->form        = best.form;
@@ -887,19 +911,29 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
     const bool row_hot = direct && io.order_out == 0 && io.lp_dst == lp_def;
 
     // One launch over the whole batch (plan-owned scratch slots and counters);
-    // PCX_FOURSTEP=chunked selects the two-launch chunk pipeline below.
+    // PCX_FOURSTEP=chunked selects the two-launch chunk pipeline below.  The
+    // kernel's other forms take packs up to the default width (at the side
+    // that is in a permuted order: 1 or the default one, whose runs they
+    // read or write in whole 16-byte units) and short sources of at least one
+    // row of the four-step view.
     const char* fs_env = std::getenv("PCX_FOURSTEP");
     const bool tuned_fused = p->form == PCX_FORM_DEFAULT || p->form == PCX_FORM_FUSED;
-    if (!ws && tuned_fused && col_hot && row_hot && use_tma && p->fs_tc > 0 &&
+    const int  perm        = io.order_in ? io.order_in : io.order_out;
+    const int  lp_perm     = io.order_in ? io.lp_src : io.lp_dst;
+    const bool fs_plain    = col_hot && row_hot;
+    const bool fs_form     = !fs_plain && p->fs_def.tc > 0 && (size_t(1) << p->fs_def.var.l2) <= src_len &&
+                         (!perm || lp_perm == 0 || lp_perm == lp_def);
+    if (!ws && tuned_fused && use_tma && p->fs.tc > 0 && (fs_plain || fs_form) &&
         !(fs_env && std::strcmp(fs_env, "chunked") == 0)) {
-        const long long per_t = p->fs_tc + p->fs_tr;
+        const fs_choice& fc    = fs_plain ? p->fs : p->fs_def;
+        const long long  per_t = fc.tc + fc.tr;
         // a row tile runs about `rounds` rounds of items (one item per CTA)
         // after its transform's column tiles, and a slot is rewritten about as
         // long after its row tiles, so both dependencies have usually cleared
         // by the time the copy warp reaches them
         const char*     re     = std::getenv("PCX_FS_ROUNDS");
         const long long rounds = re && std::atol(re) > 0 ? std::atol(re) : p->fs_rounds;
-        const long long ctas   = (long long)p->sms * std::max(1, p->fs_per_sm);
+        const long long ctas   = (long long)p->sms * std::max(1, fc.per_sm);
         long long       lag    = (rounds * ctas + per_t - 1) / per_t;
         lag                    = std::max<long long>(1, std::min<long long>(lag, (long long)batch));
         // slots in use at once: lag transforms between a column tile and its
@@ -933,19 +967,32 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         a.conj_in    = io.conj_in;
         a.conj_out   = io.conj_out;
         a.scale      = io.scale;
-        a.stw1       = p->fs_st1;
-        a.stw2       = p->fs_st2;
-        a.tw_hi      = p->fs_thi;
-        a.tw_lo      = p->fs_tlo;
-        a.tw_b       = p->fs_tb;
+        a.stw1       = fc.st1;
+        a.stw2       = fc.st2;
+        a.tw_hi      = fc.thi;
+        a.tw_lo      = fc.tlo;
+        a.tw_b       = fc.tb;
+        a.tw         = io.order_in ? fc.twr : fc.tw;
         a.scratch    = p->scratch;
         a.nslot      = (int)nslot;
         a.lag        = (int)lag;
         a.col_done   = p->fs_ctr;
         a.row_done   = p->fs_ctr + batch;
         a.error      = p->err;
-        PCX_CUDA_TRY(pcx_fourstep(f64, p->fs_var, a, st, p->sms, false, nullptr, nullptr, nullptr));
-        return PCX_OK;
+        a.lp_src     = io.lp_src;
+        a.lp_dst     = io.lp_dst;
+        a.src_len    = io.src_len;
+        a.order      = perm;
+        if (fs_plain) {
+            PCX_CUDA_TRY(pcx_fourstep(f64, fc.var, a, st, p->sms, false, nullptr, nullptr, nullptr));
+            return PCX_OK;
+        }
+        const cudaError_t e = (io.order_in ? pcx_fs_in : io.order_out ? pcx_fs_out : pcx_fs_any)(f64, fc.var, a, st,
+                                                                                                 p->sms, false);
+        if (e != cudaErrorNotSupported) {
+            PCX_CUDA_TRY(e);
+            return PCX_OK;
+        }
     }
 
     std::unique_lock<std::mutex> lock(p->mu, std::defer_lock);

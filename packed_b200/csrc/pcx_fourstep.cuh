@@ -51,16 +51,97 @@ struct fs_args {
     double      scale;
     const void* stw1;     // full stage tables of the N1 and N2 sub-transforms (fs_full_tw_*)
     const void* stw2;
-    const void* tw_hi;    // W_N^(i*N2), i < N1
+    const void* tw_hi;    // W_N^(i*N2), i < N1 (FS_PLAIN, as tw_lo and tw_b)
     const void* tw_lo;    // W_N^i, i < N2
     const void* tw_b;     // W_{16*N2}^m
+    const void* tw;       // other forms: four-step twiddles (k_fs_twiddles), [row][n2], FS_IN: [row][bitrev(n2)]
     void*       scratch;  // nslot slots of N complex
     int         nslot;    // a power of two: transform r uses slot r & (nslot - 1)
     int         lag;      // transforms between a column pass and its row pass
     int*        col_done;
     int*        row_done;
     int*        error;
+    // forms other than FS_PLAIN only
+    int         lp_src;     // log2 pack widths
+    int         lp_dst;
+    int         src_len;    // valid source elements per transform, at least N2 (zero-extended to N)
+    int         order;      // FS_OUT: the output's order; FS_IN: the input's
 };
+
+// Forms of the kernel.  FS_PLAIN is the hot one: default packs, whole rows,
+// natural order on both sides.  The others run the same items in the same
+// order (one built variant per size, the size's default):
+//  * FS_ANY: source and destination packs of 1 up to the default width, and
+//    short sources.  A column tile's row segment and a row tile's output
+//    segment are the same contiguous reals at every such width, so only the
+//    per-thread base and the distance of the imaginary part change.  Source
+//    rows n1 that are whole come by TMA (the tensor map ends there and fills
+//    the rest with zeros); the one partial row is read by its threads.
+//  * FS_OUT (forward into bit_reversed / unordered order): frequency
+//    k = k2*N1 + k1 goes to position bitrev(k1)*N2 + bitrev(k2), so a row tile's
+//    outputs are whole contiguous rows, and the 16 values of a thread
+//    (k2 = t + i*TT) are 16 consecutive positions of one: they are staged in
+//    the tile's stage with 16-byte stores (8 rows on 8 bank groups by an XOR)
+//    and leave as 16-byte stores, a quarter of the store instructions of the
+//    transposed natural-order output.
+//  * FS_IN (inverse from such an order): the N1 inputs of column n2 are the
+//    contiguous run r = bitrev(n2), so a column tile is C whole source rows
+//    brought in by bulk copies, each thread's 16 inputs one run of it.
+//    The scratch keeps the columns in the order r, and a row tile reads its
+//    n2 from bitrev(n2), again one run of 16 per thread.
+// 2^15, 301 transforms, forward into `unordered` and inverse back: two
+// launches per chunk of general kernels 427 us, these 119 us.
+constexpr int FS_PLAIN = 0;
+constexpr int FS_ANY   = 1;
+constexpr int FS_OUT   = 2;
+constexpr int FS_IN    = 3;
+
+// Register i of the 16 a thread holds (element t + i*TT) at place q of its run
+// of 16 consecutive positions: i = bitrev4(q), or bitrev4(sigma(q)) in the
+// unordered order (sigma moves bits (0,1,2,3) to (2,1,3,0)).
+__host__ __device__ constexpr int run_reg(int q, bool unordered) {
+    const int s = unordered ? (((q & 1) << 2) | (q & 2) | (((q >> 2) & 1) << 3) | ((q >> 3) & 1)) : q;
+    return ((s & 1) << 3) | ((s & 2) << 1) | ((s & 4) >> 1) | ((s & 8) >> 3);
+}
+
+// Real f (0..31) of a run of 16 packed elements at pack width 2^LPX.
+template<int LPX, bool UNORD, class T>
+__device__ __forceinline__ T& run_real(cpx<T> (&v)[16], int f) {
+    const int q = ((f >> (LPX + 1)) << LPX) | (f & ((1 << LPX) - 1));
+    cpx<T>&   x = v[run_reg(q, UNORD)];
+    return (f >> LPX) & 1 ? x.im : x.re;
+}
+template<class T>
+struct alignas(16) vec16 {
+    T x[16 / sizeof(T)];
+};
+// The 16 elements of the run at `p` (16-byte aligned) into the registers they belong to.
+template<int LPX, bool UNORD, class T>
+__device__ __forceinline__ void run_load(cpx<T> (&v)[16], const T* p) {
+    constexpr int W = 16 / (int)sizeof(T);
+    static_for<32 / W>([&](auto jc) {
+        constexpr int  j = decltype(jc)::value;
+        const vec16<T> w = *reinterpret_cast<const vec16<T>*>(p + j * W);
+        static_for<W>([&](auto uc) {
+            constexpr int u                       = decltype(uc)::value;
+            run_real<LPX, UNORD>(v, j * W + u) = w.x[u];
+        });
+    });
+}
+// The run into 16-byte unit j ^ key of its 32 / W units at `p`.
+template<int LPX, bool UNORD, class T>
+__device__ __forceinline__ void run_store(cpx<T> (&v)[16], T* p, int key) {
+    constexpr int W = 16 / (int)sizeof(T);
+    static_for<32 / W>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        vec16<T>      w;
+        static_for<W>([&](auto uc) {
+            constexpr int u = decltype(uc)::value;
+            w.x[u]          = run_real<LPX, UNORD>(v, j * W + u);
+        });
+        *reinterpret_cast<vec16<T>*>(p + (j ^ key) * W) = w;
+    });
+}
 
 // Variant of the one-launch four-step: split N = 2^LOGN1 * 2^LOGN2, MINB
 // resident blocks per SM (tiles of 64 KB / MINB: two blocks of 32 KB tiles
@@ -109,6 +190,9 @@ struct fs_cfg {
     static constexpr bool SH  = stw_fits(BASE, TB1 + TB2, MINB);
     static constexpr int SMEM = SH ? BASE + TB1 + TB2 : BASE;
     static constexpr int BOXY = N1 < 256 ? N1 : 256;
+    // FS_IN: padded shared row of a column tile (reals); 16 bytes in FP32, so
+    // the 16-byte reads of 8 neighbouring columns fall on 8 bank groups
+    static constexpr int RSC  = 2 * N1 + 4;
 };
 
 __device__ __forceinline__ void fence_proxy_async_global() {
@@ -144,6 +228,27 @@ __device__ __forceinline__ void red_release_add(int* p, int v) {
     asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Twiddles of the forms other than FS_PLAIN: W_N^(k1*n2), k1 = t + i*TT, as one
+// table entry W_N^(t*n2) (row t) times powers of u = W_N^(TT*n2) (rows TT..
+// hold u^1, u^2, u^4, u^8 and u^12), all generated in FP64 and rounded once; a
+// row of N2 entries is read by neighbouring columns at once.  Against
+// FS_PLAIN's chains (two half-size tables and one power) this has the error of
+// the general kernels or less (2^15, there and back: 2.2e-7 for 3.6e-7 with
+// the chains and 3.0e-7 before) at the same speed; in FS_PLAIN it cost 0.7 %.
+template<class T>
+__global__ void k_fs_twiddles(cpx<T>* out, int tt, int log_n2, int log_n, int permuted) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= (tt + 5) << log_n2) return;
+    const int       row = q >> log_n2, r = q & ((1 << log_n2) - 1);
+    const long long n2   = permuted ? (int)brev(r, log_n2) : r;
+    const int       j    = row - tt;
+    const long long mult = j < 0 ? row : (long long)tt * (j == 4 ? 12 : 1 << j);
+    const long long e    = (n2 * mult) & ((1LL << log_n) - 1);
+    double          s, c;
+    sincospi(2.0 * (double)e / (double)(1LL << log_n), &s, &c);
+    out[q] = {T(c), T(-s)};
+}
+
 // Item j of the queue (32-bit: the launch holds fewer than 2^31 items).  TC
 // and TR are powers of two, TC + TR a constant: no division is a real one.
 template<int TC, int TR>
@@ -162,7 +267,7 @@ __device__ __forceinline__ fs_item fs_decode(uint32_t j, uint32_t batch, uint32_
     return {1, (int)(batch - lag + j / TR), (int)(j % TR)};
 }
 
-template<class T, int LOGN1, int LOGN2, int MINB, int ST_>
+template<class T, int LOGN1, int LOGN2, int MINB, int ST_, int FORM = FS_PLAIN>
 __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, MINB)
     k_fourstep(const __grid_constant__ CUtensorMap tmap, fs_args a) {
     using F            = fs_cfg<T, LOGN1, LOGN2, MINB, ST_>;
@@ -186,6 +291,8 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
     constexpr int RSI  = F::RSI;
     constexpr int RROW = N2 * (int)sizeof(cpx<T>);
     constexpr bool SH  = F::SH;
+    static_assert(FORM != FS_IN || C * F::RSC * (int)sizeof(T) <= F::STAGE, "a column tile of whole rows fits a stage");
+    static_assert(FORM != FS_OUT || CR * 2 * N2 * (int)sizeof(T) <= (IP ? F::STAGE : F::XB), "a staged row tile fits");
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char*      ring = smem;
     cpx<T>*             tws1 = reinterpret_cast<cpx<T>*>(smem + F::BASE);
@@ -292,7 +399,15 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
             unsigned char* buf = ring + s * F::STAGE;
             if (!it.row) {
                 // the source tile does not depend on anything: copy it first
-                if (lane == 0) {
+                if constexpr (FORM == FS_IN) {
+                    if (lane == 0) mbar_arrive_expect_tx(&full[s], F::COLB);
+                    __syncwarp();
+                    const T* g = reinterpret_cast<const T*>(a.src) + it.r * a.src_stride + (long long)it.tile * C * 2 * N1;
+                    for (int q = lane; q < C; q += 32) {
+                        bulk_g2s(reinterpret_cast<T*>(buf) + q * F::RSC, g + (long long)q * 2 * N1,
+                                 2 * N1 * (int)sizeof(T), &full[s]);
+                    }
+                } else if (lane == 0) {
                     mbar_arrive_expect_tx(&full[s], F::COLB);
 #pragma unroll
                     for (int y = 0; y < N1; y += F::BOXY) {
@@ -363,13 +478,22 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
         };
         // column tile: the four-step twiddle inputs are requested before the
         // tile's data is waited for, and used after the stages
-        cpx<T> th{}, tl{}, tu{};
+        cpx<T> th{}, tl{}, tu[FORM == FS_PLAIN ? 1 : 5]{};
         if (!it.row) {
-            const int      n2 = it.tile * C + tid % C;
-            const uint32_t e0 = (uint32_t)(tid / C) * (uint32_t)n2;
-            th                = ldg_cpx(reinterpret_cast<const cpx<T>*>(a.tw_hi) + (e0 >> LOGN2));
-            tl                = ldg_cpx(reinterpret_cast<const cpx<T>*>(a.tw_lo) + (e0 & (N2 - 1)));
-            tu                = ldg_cpx(reinterpret_cast<const cpx<T>*>(a.tw_b) + n2);
+            const int n2 = it.tile * C + tid % C;    // FS_IN: the column's place in the scratch
+            if constexpr (FORM == FS_PLAIN) {
+                const uint32_t e0 = (uint32_t)(tid / C) * (uint32_t)n2;
+                th                = ldg_cpx(reinterpret_cast<const cpx<T>*>(a.tw_hi) + (e0 >> LOGN2));
+                tl                = ldg_cpx(reinterpret_cast<const cpx<T>*>(a.tw_lo) + (e0 & (N2 - 1)));
+                tu[0]             = ldg_cpx(reinterpret_cast<const cpx<T>*>(a.tw_b) + n2);
+            } else {
+                const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw) + n2;
+                th               = ldg_cpx(tw + (tid / C) * N2);
+                static_for<5>([&](auto qc) {
+                    constexpr int q = decltype(qc)::value;
+                    tu[q]           = ldg_cpx(tw + (P1::TT + q) * N2);
+                });
+            }
         }
         if (!mbar_wait_bounded(&full[s], par)) {
             bad = true;
@@ -381,15 +505,46 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
             constexpr int TT   = P1::TT;
             const int     c    = tid % C;
             const int     t    = tid / C;
-            const int     n2   = it.tile * C + c;
+            const int     n2   = it.tile * C + c;    // FS_IN: the column's place in the scratch
             const T*      in   = reinterpret_cast<const T*>(ring + s * F::STAGE);
             const auto*   stw1 = SH ? tws1 : reinterpret_cast<const cpx<T>*>(gtab1);
             cpx<T>        v[E];
-            static_for<E>([&](auto ic) {
-                constexpr int i = decltype(ic)::value;
-                cpx<T>        x = lds_swapped<T, SW>(in, (t + i * TT) * SEG + pk<LP>(c), PK);
-                v[i]            = {x.re, a.conj_in ? -x.im : x.im};
-            });
+            if constexpr (FORM == FS_IN) {
+                const T* run = in + c * F::RSC + 32 * (int)brev(t, LOGN1 - 4);
+                if (a.lp_src == 0) {
+                    if (a.order == 2) run_load<0, true>(v, run);
+                    else run_load<0, false>(v, run);
+                } else {
+                    if (a.order == 2) run_load<LP, true>(v, run);
+                    else run_load<LP, false>(v, run);
+                }
+                static_for<E>([&](auto ic) { v[decltype(ic)::value].im = -v[decltype(ic)::value].im; });
+            } else if constexpr (FORM != FS_PLAIN) {
+                const int pks = 1 << a.lp_src;
+                const int o   = t * SEG + (int)pk_re(c, a.lp_src);
+                static_for<E>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    cpx<T>        x = lds_swapped<T, SW>(in, o + i * TT * SEG, pks);
+                    v[i]            = {x.re, a.conj_in ? -x.im : x.im};
+                });
+                if (a.src_len < N1 * N2) {    // rows from src_len / N2 on arrived as zeros
+                    const int q = a.src_len >> LOGN2;
+                    static_for<E>([&](auto ic) {
+                        constexpr int i = decltype(ic)::value;
+                        const int     e = q * N2 + n2;
+                        if (t + i * TT == q && e < a.src_len) {
+                            const T* g = reinterpret_cast<const T*>(a.src) + it.r * a.src_stride + pk_re(e, a.lp_src);
+                            v[i]       = {g[0], g[pks]};    // forward: no conjugate
+                        }
+                    });
+                }
+            } else {
+                static_for<E>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    cpx<T>        x = lds_swapped<T, SW>(in, (t + i * TT) * SEG + pk<LP>(c), PK);
+                    v[i]            = {x.re, a.conj_in ? -x.im : x.im};
+                });
+            }
             if constexpr (!IP) release_stage();
             stage_compute_tab<P1, 0>(v, t, stw1);
             if (run_stages_full<P1, typename F::X1, SH, NT, typename F::PT1>(v, xch, c, t, stw1, bad)) return;
@@ -403,10 +558,12 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
             colpar ^= 1u << s;
             if (!bad) {
                 cpx<T>* dst = scr + (it.r & mask) * (long long)(N1 * N2) + (long long)t * N2 + n2;
-                apply_fourstep_tw(v, cmul(th, tl), tu, [&](auto ic, cpx<T> o) {
+                auto    put = [&](auto ic, cpx<T> o) {
                     constexpr int i             = decltype(ic)::value;
                     dst[(long long)i * TT * N2] = o;
-                });
+                };
+                if constexpr (FORM == FS_PLAIN) apply_fourstep_tw(v, cmul(th, tl), tu[0], put);
+                else apply_fourstep_tw5(v, th, tu, put);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&written[s]);
             }
@@ -420,24 +577,80 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
             const int     m    = mhi * G8 + mlo;
             const int     k1   = it.tile * CR + m;
             const auto*   stw2 = SH ? tws2 : reinterpret_cast<const cpx<T>*>(gtab2);
-            const cpx<T>* in   = reinterpret_cast<const cpx<T>*>(ring + s * F::STAGE) + m * RSI + t;
+            const cpx<T>* in   = reinterpret_cast<const cpx<T>*>(ring + s * F::STAGE) + m * RSI +
+                                 (FORM == FS_IN ? 16 * (int)brev(t, LOGN2 - 4) : t);
             cpx<T>        v[E];
-            static_for<E>([&](auto ic) {
-                constexpr int i = decltype(ic)::value;
-                v[i]            = in[i * TT];
-            });
+            if constexpr (FORM == FS_IN) {
+                run_load<0, false>(v, reinterpret_cast<const T*>(in));
+            } else {
+                static_for<E>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    v[i]            = in[i * TT];
+                });
+            }
             if constexpr (!IP) release_stage();
             stage_compute_tab<P2, 0>(v, t, stw2);
             if (run_stages_full<P2, typename F::X2, SH, NT, typename F::PT2>(v, xch, m, t, stw2, bad)) return;
-            if constexpr (IP) release_stage();
-            T*      dst = reinterpret_cast<T*>(a.dst) + it.r * a.dst_stride + pk<LP>(t * N1 + k1);
             const T sc  = T(a.scale);
             const T sim = a.conj_out ? -sc : sc;
-            static_for<E>([&](auto ic) {
-                constexpr int i = decltype(ic)::value;
-                __stcs(dst + 2 * i * TT * N1, v[i].re * sc);
-                __stcs(dst + 2 * i * TT * N1 + PK, v[i].im * sim);
-            });
+            if constexpr (FORM == FS_OUT) {
+                // rows staged in output order, then copied out whole
+                constexpr int W   = 16 / (int)sizeof(T);
+                constexpr int U   = 32 / W;         // 16-byte units per run
+                constexpr int KT  = 8 / G8;         // threads t per bank group turn
+                T*            stg = reinterpret_cast<T*>(xch);
+                auto          key = [](int row, int tt) { return row % G8 + G8 * (tt % KT); };
+                static_for<E>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    v[i]            = {v[i].re * sc, v[i].im * sim};
+                });
+                xch_sync<NT>();    // the exchange buffer is no longer read
+                T* run = stg + m * 2 * N2 + 32 * (int)brev(t, LOGN2 - 4);
+                if (a.lp_dst == 0) {
+                    if (a.order == 2) run_store<0, true>(v, run, key(m, t));
+                    else run_store<0, false>(v, run, key(m, t));
+                } else {
+                    if (a.order == 2) run_store<LP, true>(v, run, key(m, t));
+                    else run_store<LP, false>(v, run, key(m, t));
+                }
+                xch_sync<NT>();
+                T* dst = reinterpret_cast<T*>(a.dst) + it.r * a.dst_stride;
+                for (int q = tid; q < CR * (2 * N2 / W); q += NT) {
+                    const int      row = q / (2 * N2 / W), u = q % (2 * N2 / W);
+                    const int      tt  = (int)brev(u / U, LOGN2 - 4);
+                    const vec16<T> w   = *reinterpret_cast<const vec16<T>*>(
+                        stg + row * 2 * N2 + (u / U) * 32 + ((u % U) ^ key(row, tt)) * W);
+                    const int      k   = (int)brev(it.tile * CR + row, LOGN1);
+                    __stcs(reinterpret_cast<float4*>(dst + (long long)k * 2 * N2 + u * W),
+                           *reinterpret_cast<const float4*>(&w));
+                }
+                if constexpr (IP) release_stage();
+            } else if constexpr (FORM != FS_PLAIN) {
+                if constexpr (IP) release_stage();
+                T* dst = reinterpret_cast<T*>(a.dst) + it.r * a.dst_stride + pk_re(t * N1 + k1, a.lp_dst);
+                if (a.lp_dst == 0) {
+                    using V2 = std::conditional_t<sizeof(T) == 4, float2, double2>;
+                    static_for<E>([&](auto ic) {
+                        constexpr int i = decltype(ic)::value;
+                        __stcs(reinterpret_cast<V2*>(dst + 2 * i * TT * N1), V2{v[i].re * sc, v[i].im * sim});
+                    });
+                } else {
+                    T* dim = dst + (1 << a.lp_dst);
+                    static_for<E>([&](auto ic) {
+                        constexpr int i = decltype(ic)::value;
+                        __stcs(dst + 2 * i * TT * N1, v[i].re * sc);
+                        __stcs(dim + 2 * i * TT * N1, v[i].im * sim);
+                    });
+                }
+            } else {
+                if constexpr (IP) release_stage();
+                T* dst = reinterpret_cast<T*>(a.dst) + it.r * a.dst_stride + pk<LP>(t * N1 + k1);
+                static_for<E>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    __stcs(dst + 2 * i * TT * N1, v[i].re * sc);
+                    __stcs(dst + 2 * i * TT * N1 + PK, v[i].im * sim);
+                });
+            }
         }
     }
 }

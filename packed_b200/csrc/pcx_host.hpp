@@ -62,6 +62,20 @@ struct fs_variant {
     int l1 = 0, l2 = 0, minb = 0, st = 0;
     bool operator==(const fs_variant& o) const { return l1 == o.l1 && l2 == o.l2 && minb == o.minb && st == o.st; }
 };
+// A variant with its tables (one allocation) and tile counts.
+struct fs_choice {
+    fs_variant var{};                 // l1 == 0: none
+    void*      mem = nullptr;         // owns the tables below
+    void*      thi = nullptr;         // W_N^(i*N2), i < N1
+    void*      tlo = nullptr;         // W_N^i, i < N2
+    void*      tb  = nullptr;         // W_{16*N2}^i, i < N2
+    void*      tw  = nullptr;         // twiddles of the forms (the default variant only)
+    void*      twr = nullptr;         // the same by bit-reversed column (plans of a permuted order)
+    void*      st1 = nullptr;         // full stage tables of the N1- and N2-point sub-transforms
+    void*      st2 = nullptr;
+    int        tc = 0, tr = 0;        // column and row tiles per transform
+    int        per_sm = 1;            // resident blocks per SM
+};
 // The variants built into the library (FP32 and FP64), in the order the
 // autotuner tries them; the first one of a size is its untuned default (the
 // fastest one measured on a B200 on 512 MB batches; at 2^15 and 2^17..2^19 an
@@ -136,17 +150,8 @@ struct pcx_plan_s {
     void*  fst      = nullptr;    // one-launch four-step: full stage tables of N1 then N2 (one allocation)
     void*  fst1     = nullptr;
     void*  fst2     = nullptr;
-    pcxg::fs_variant fs_var{};    // one-launch four-step: its variant (l1 == 0: none)
-    void*  fs_mem   = nullptr;    // tables of fs_var's split (one allocation):
-    void*  fs_thi   = nullptr;    //   W_N^(i*N2), i < N1
-    void*  fs_tlo   = nullptr;    //   W_N^i, i < N2
-    void*  fs_tb    = nullptr;    //   W_{16*N2}^i, i < N2
-    void*  fs_st1   = nullptr;    //   full stage tables of the N1- and N2-point sub-transforms
-    void*  fs_st2   = nullptr;
-    int    fs_tab_l1 = 0;         // split the tables belong to
-    int    fs_tc    = 0;          // one-launch four-step: column and row tiles per transform (0: none)
-    int    fs_tr    = 0;
-    int    fs_per_sm = 1;         // its resident blocks per SM
+    pcxg::fs_choice fs{};         // one-launch four-step: the variant in use
+    pcxg::fs_choice fs_def{};     // the size's default one, which the kernel's other forms run
     int*   fs_ctr   = nullptr;    // its dependency counters, 2 per transform
     size_t fs_ctr_n = 0;
     // form of the plan-owned-scratch path for n > 4096, set by pcx_plan_tune
@@ -214,6 +219,14 @@ struct fs_args;
 }
 cudaError_t pcx_fourstep(bool f64, const pcxg::fs_variant& v, const pcxg::fs_args& a, cudaStream_t st, int sms,
                          bool attr_only, int* col_tiles, int* row_tiles, int* blocks_per_sm);
+// Its other forms (pcx_fourstep.cuh: FS_ANY, FS_OUT, FS_IN), built for each
+// size's default variant.
+cudaError_t pcx_fs_any(bool f64, const pcxg::fs_variant& v, const pcxg::fs_args& a, cudaStream_t st, int sms,
+                       bool attr_only);
+cudaError_t pcx_fs_out(bool f64, const pcxg::fs_variant& v, const pcxg::fs_args& a, cudaStream_t st, int sms,
+                       bool attr_only);
+cudaError_t pcx_fs_in(bool f64, const pcxg::fs_variant& v, const pcxg::fs_args& a, cudaStream_t st, int sms,
+                      bool attr_only);
 // Full stage tables of an L = 2^log_l point sub-transform of the one-launch
 // four-step (entries: their count; out == nullptr only counts).
 cudaError_t pcx_fourstep_tables(int log_l, void* out, bool f64, cudaStream_t st, int* entries);
