@@ -86,7 +86,9 @@ __global__ void k_par_scatter(T* const* __restrict__ rows, int lpd, const T* __r
 // kernel parameters (16 bytes a vector, at most 16 KB), so a call copies
 // nothing to the device and needs no workspace.
 // HBM-bound: 16 bytes per point where gather + transform + scatter moved 48.
-// 64 vectors of 250007 elements: 187 us before, 61 us.
+// 64 vectors of 250007 elements: 187 us before, 53.5 us with three blocks an
+// SM in FP32 (two: 61.4, four: 55.3; loads in flight hide the latency, four
+// blocks leave too few registers).
 template<class T, int LOGN>
 struct par_cfg {
     using P                  = splan<LOGN>;
@@ -109,7 +111,7 @@ struct par_args {
 };
 
 template<class T, int LOGN>
-__global__ void __launch_bounds__(par_cfg<T, LOGN>::NT, par_cfg<T, LOGN>::NT > 256 ? 1 : 2)
+__global__ void __launch_bounds__(par_cfg<T, LOGN>::NT, par_cfg<T, LOGN>::NT > 256 ? 1 : (sizeof(T) == 8 ? 2 : 3))
     k_par(const __grid_constant__ par_args<(1 << LOGN)> a) {
     using F          = par_cfg<T, LOGN>;
     using P          = typename F::P;
