@@ -1,6 +1,7 @@
 // Host side of the overlap-save correlator: handle creation (kernel spectrum
 // computed on the device), the fused correlation launch and its adjoint.
 #include "pcx_fxcorr2d.cuh"
+#include "pcx_fxcorr3.cuh"
 #include "pcx_fxcorr_kernels.cuh"
 #include "pcx_host.hpp"
 #include "pcx_v2_launch.cuh"
@@ -27,6 +28,7 @@ struct pcx_fxcorr_s {
     size_t      gscratch_bytes = 0;
     int         sms            = 0;
     int         device         = 0;
+    bool        x3             = false;      // FP32, N <= 2^12: pcx_fxcorr3.cuh (tables: plan->stwL)
     // FP32, N = 2^13 or 2^14: in-CTA four-step form (pcx_fxcorr2d.cuh)
     void*       x2d            = nullptr;    // one allocation: K permuted | stage tables | twiddles
     const void* x2_kperm       = nullptr;
@@ -176,6 +178,60 @@ int launch_xc2_kg(const xc2_kg_args& a, cudaStream_t st, int grid, bool attr_onl
     return PCX_OK;
 }
 
+// The whole-window form (pcx_fxcorr3.cuh): blocks of a launch over `total` windows.
+template<int LOGN, class K>
+int grid_xc3(K kern, long long total, int sms, int* grid) {
+    using C    = xc3_cfg<LOGN>;
+    int per_sm = 0;
+    PCX_CUDA_TRY(smem_attr_cached(reinterpret_cast<const void*>(kern), C::SMEM));
+    PCX_CUDA_TRY(occupancy_cached(reinterpret_cast<const void*>(kern), C::NT, C::SMEM, &per_sm));
+    const long long tiles = (total + C::M - 1) / C::M;
+    *grid = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)std::max(per_sm, 1) * sms));
+    return PCX_OK;
+}
+template<int LOGN>
+int launch_xc3(const xc_args& a, const void* stw, cudaStream_t st, int sms) {
+    using C  = xc3_cfg<LOGN>;
+    int grid = 0;
+    if (int rc = grid_xc3<LOGN>(k_fxcorr3<LOGN>, a.total, sms, &grid)) return rc;
+    if (a.total == 0) return PCX_OK;    // launch attributes only
+    k_fxcorr3<LOGN><<<(unsigned)grid, C::NT, C::SMEM, st>>>(a, stw);
+    PCX_CUDA_TRY(cudaGetLastError());
+    return PCX_OK;
+}
+// grid: given a.acc == nullptr only returned (the rows of the accumulator)
+template<int LOGN>
+int launch_xc3_kg(const kg_args& a, const void* stw, cudaStream_t st, int sms, int* grid) {
+    using C = xc3_cfg<LOGN>;
+    if (int rc = grid_xc3<LOGN>(k_fxcorr3_kgrad<LOGN>, a.total, sms, grid)) return rc;
+    if (!a.acc) return PCX_OK;
+    k_fxcorr3_kgrad<LOGN><<<(unsigned)*grid, C::NT, C::SMEM, st>>>(a, stw);
+    PCX_CUDA_TRY(cudaGetLastError());
+    return PCX_OK;
+}
+int dispatch_xc3(int log_n, const xc_args& a, const void* stw, cudaStream_t st, int sms) {
+    switch (log_n) {
+    case 6: return launch_xc3<6>(a, stw, st, sms);
+    case 7: return launch_xc3<7>(a, stw, st, sms);
+    case 8: return launch_xc3<8>(a, stw, st, sms);
+    case 9: return launch_xc3<9>(a, stw, st, sms);
+    case 10: return launch_xc3<10>(a, stw, st, sms);
+    case 11: return launch_xc3<11>(a, stw, st, sms);
+    default: return launch_xc3<12>(a, stw, st, sms);
+    }
+}
+int dispatch_xc3_kg(int log_n, const kg_args& a, const void* stw, cudaStream_t st, int sms, int* grid) {
+    switch (log_n) {
+    case 6: return launch_xc3_kg<6>(a, stw, st, sms, grid);
+    case 7: return launch_xc3_kg<7>(a, stw, st, sms, grid);
+    case 8: return launch_xc3_kg<8>(a, stw, st, sms, grid);
+    case 9: return launch_xc3_kg<9>(a, stw, st, sms, grid);
+    case 10: return launch_xc3_kg<10>(a, stw, st, sms, grid);
+    case 11: return launch_xc3_kg<11>(a, stw, st, sms, grid);
+    default: return launch_xc3_kg<12>(a, stw, st, sms, grid);
+    }
+}
+
 // Tables of the in-CTA four-step form; false when it does not apply.
 template<int LOGN>
 int init_xc2(pcx_fxcorr_s* h) {
@@ -252,7 +308,6 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
         PCX_CUDA_TRY(cudaMemsetAsync(h->ctl + 2, 0, h->flags_cap * sizeof(unsigned), st));
         h->epoch = 1;
     }
-    PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), st));
 
     xc_args a{};
     a.src         = src;
@@ -280,10 +335,13 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     a.counter     = h->ctl;
     a.error       = reinterpret_cast<int*>(h->ctl + 1);
     a.kspec       = h->kspec;
-    // in-CTA four-step form: FP32, pack 8, windows on whole packs, rows of
-    // packs 16-byte aligned
-    const bool x2 = h->x2d && pack == 8 && a.in_shift % 8 == 0 &&
-                    (channels == 1 || sstride % 4 == 0) && reinterpret_cast<uintptr_t>(src) % 16 == 0;
+    // whole-window and in-CTA four-step forms: FP32, pack 8, windows on whole
+    // packs, rows of packs 16-byte aligned
+    const bool rows = pack == 8 && a.in_shift % 8 == 0 && (channels == 1 || sstride % 4 == 0) &&
+                      reinterpret_cast<uintptr_t>(src) % 16 == 0;
+    if (inplace || !(h->x3 && rows)) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), st));
+    if (h->x3 && rows) return dispatch_xc3(h->log_n, a, h->plan->stwL, st, h->sms);
+    const bool x2 = h->x2d && rows;
     if (x2) {
         xc2_args b{};
         b.base  = a;
@@ -348,6 +406,15 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
         rc = dtype == PCX_F64 ? dispatch_kg<double>(log_n, kg_args{}, nullptr, 0, 0, true)
                               : dispatch_kg<float>(log_n, kg_args{}, nullptr, 0, 0, true);
         if (rc) return fail(rc);
+        if (dtype == PCX_F32 && log_n <= 12 && std::getenv("PCX_XC_GENERAL") == nullptr) {
+            // its launch attributes now, not in a call that may be captured
+            int  grid = 0;
+            auto kg   = kg_args{};
+            rc        = dispatch_xc3_kg(log_n, kg, nullptr, 0, h->sms, &grid);
+            if (!rc) rc = dispatch_xc3(log_n, xc_args{}, nullptr, 0, h->sms);
+            if (rc) return fail(rc);
+            h->x3 = true;
+        }
         if (dtype == PCX_F32 && (log_n == 13 || log_n == 14) && std::getenv("PCX_XC_GENERAL") == nullptr) {
             rc = log_n == 14 ? init_xc2<14>(h) : init_xc2<13>(h);
             if (rc) return fail(rc);
@@ -413,8 +480,21 @@ extern "C" int pcx_fxcorr_vjp(pcx_fxcorr h, void* gx, void* gg, const void* gy, 
         const size_t nblk  = (len + step - 1) / step;
         const size_t total = nblk * channels;
         const size_t eb    = h->dtype == PCX_F64 ? 16 : 8;
-        const int    grid  = (int)std::min<size_t>(total, (size_t)h->sms);
-        const size_t need  = ((size_t)grid * 2 + 2) * n * eb;
+        // FP32 at pack 8 on 16-byte aligned rows: the whole-window form up to
+        // 2^12 points, the in-CTA four-step form with the per-thread spectra in
+        // tensor memory at 2^13 and 2^14
+        const bool rows = pack == 8 && (channels == 1 || stride % 4 == 0) &&
+                          (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gy)) % 16 == 0;
+        const bool x3 = h->x3 && rows, x2 = h->x2d && rows;
+        kg_args    a{};
+        a.total  = (long long)total;
+        int grid = (int)std::min<size_t>(total, (size_t)h->sms);
+        if (x3) {
+            if (int rc = dispatch_xc3_kg(h->log_n, a, nullptr, st, h->sms, &grid)) return rc;
+        }
+        // sums of the blocks, the general form's spectra, the sum and its inverse
+        const size_t rows_s = (size_t)grid * (x3 || x2 ? 1 : 2);
+        const size_t need   = (rows_s + 2) * n * eb;
         if (h->gscratch_bytes < need) {
             if (h->gscratch) cudaFree(h->gscratch);
             h->gscratch       = nullptr;
@@ -423,9 +503,8 @@ extern "C" int pcx_fxcorr_vjp(pcx_fxcorr h, void* gx, void* gg, const void* gy, 
             h->gscratch_bytes = need;
         }
         if (int rc = ensure_flags(h, 1)) return rc;
-        PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), st));
-        char*   base  = static_cast<char*>(h->gscratch);
-        kg_args a{};
+        if (!x3) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), st));
+        char* base = static_cast<char*>(h->gscratch);
         a.x       = x;
         a.gy      = gy;
         a.stride  = (long long)stride;
@@ -433,19 +512,16 @@ extern "C" int pcx_fxcorr_vjp(pcx_fxcorr h, void* gx, void* gg, const void* gy, 
         a.lp      = __builtin_ctz(pack);
         a.step    = (int)step;
         a.nblk    = (int)nblk;
-        a.total   = (long long)total;
         a.counter = h->ctl;
         a.error   = reinterpret_cast<int*>(h->ctl + 1);
         a.acc     = base;
         a.xspec   = base + (size_t)grid * n * eb;
-        void* sum = base + (size_t)grid * 2 * n * eb;
-        void* inv = base + ((size_t)grid * 2 + 1) * n * eb;
-        // FP32 2^13 / 2^14 at pack 8 on 16-byte aligned rows: the in-CTA
-        // four-step form with the per-thread spectra in tensor memory
-        const bool x2 = h->x2d && pack == 8 && (channels == 1 || stride % 4 == 0) &&
-                        (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gy)) % 16 == 0;
+        void* sum = base + rows_s * n * eb;
+        void* inv = base + (rows_s + 1) * n * eb;
         int rc;
-        if (x2) {
+        if (x3) {
+            rc = dispatch_xc3_kg(h->log_n, a, h->plan->stwL, st, h->sms, &grid);
+        } else if (x2) {
             xc2_kg_args b{};
             b.base = a;
             b.stw1 = h->x2_stw1;
@@ -458,10 +534,10 @@ extern "C" int pcx_fxcorr_vjp(pcx_fxcorr h, void* gx, void* gg, const void* gy, 
         }
         if (rc) return rc;
         if (h->dtype == PCX_F64) {
-            k_kgrad_reduce<double><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+            k_kgrad_reduce<double><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
                 static_cast<const cpx<double>*>(a.acc), grid, (int)n, static_cast<cpx<double>*>(sum));
         } else {
-            k_kgrad_reduce<float><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+            k_kgrad_reduce<float><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
                 static_cast<const cpx<float>*>(a.acc), grid, (int)n, static_cast<cpx<float>*>(sum));
         }
         PCX_CUDA_TRY(cudaGetLastError());
