@@ -282,6 +282,12 @@ int pcx_fft_vjp(pcx_plan plan, void* g_in, const void* g_out, int pack, int dire
  */
 int pcx_fxcorr_create(pcx_fxcorr* h, const void* g, size_t k, int pack_g, size_t n_fft, int dtype);
 int pcx_fxcorr_destroy(pcx_fxcorr h);
+/*
+ * Destroyed handles' device memory and tables are kept for the next create of
+ * the same type and FFT size (at most 4 handles and 64 MB of their scratch);
+ * this frees what is kept.
+ */
+int pcx_fxcorr_release_idle(void);
 
 /*
  * y[n] = sum_{j<k} x[n+j] * conj(g[j]) (x zero past its end) for `channels`

@@ -52,6 +52,7 @@ SIGNATURES: dict[str, tuple] = {
     "pcx_fft_exec_noalloc": (_i, [_vp, _vp, _vp, _sz, _i, _i, _i, _i, _sz, _sz, _sz, _vp]),
     "pcx_fxcorr_create": (_i, [ctypes.POINTER(_vp), _vp, _sz, _i, _sz, _i]),
     "pcx_fxcorr_destroy": (_i, [_vp]),
+    "pcx_fxcorr_release_idle": (_i, []),
     "pcx_fxcorr_exec": (_i, [_vp, _vp, _vp, _sz, _i, _sz, _sz, _sz, _vp]),
     "pcx_fxcorr_vjp": (_i, [_vp, _vp, _vp, _vp, _vp, _sz, _i, _sz, _sz, _vp]),
     "pcx_fxcorr_status": (_i, [_vp]),

@@ -8,6 +8,8 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <list>
+#include <mutex>
 #include <string>
 
 using namespace pcxg;
@@ -35,6 +37,13 @@ struct pcx_fxcorr_s {
     const void* x2_stw1        = nullptr;
     const void* x2_stw2        = nullptr;
     const void* x2_tws         = nullptr;
+    // for reuse (see handle_pool): created with PCX_XC_GENERAL; the last call's
+    // end on its stream, unless calls went to several streams or into a capture
+    bool         general = false;
+    cudaEvent_t  done    = nullptr;
+    cudaStream_t last    = nullptr;
+    bool         used    = false;
+    bool         unsure  = false;
 };
 
 namespace {
@@ -250,7 +259,6 @@ int init_xc2(pcx_fxcorr_s* h) {
     auto* s1     = kp + C::N;
     auto* s2     = s1 + e1;
     auto* tws    = s2 + e2;
-    PCX_CUDA_TRY(pcx_xc2_perm_spectrum(h->kspec, kp, C::LOGN1, C::LOGN2, 0));
     PCX_CUDA_TRY(pcx_fourstep_tables(C::LOGN1, s1, false, 0, &e1));
     PCX_CUDA_TRY(pcx_fourstep_tables(C::LOGN2, s2, false, 0, &e2));
     PCX_CUDA_TRY(pcx_gen_twiddles(tws, C::NB, LOGN, 1, false, 0));
@@ -357,6 +365,147 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
 
 }    // namespace
 
+namespace {
+
+void free_handle(pcx_fxcorr_s* h) {
+    if (h->plan) pcx_plan_destroy(h->plan);
+    if (h->tw) cudaFree(h->tw);
+    if (h->kspec) cudaFree(h->kspec);
+    if (h->ctl) cudaFree(h->ctl);
+    if (h->gscratch) cudaFree(h->gscratch);
+    if (h->x2d) cudaFree(h->x2d);
+    if (h->done) cudaEventDestroy(h->done);
+    delete h;
+}
+
+// Handles that were destroyed, kept for the next create of the same kind
+// (device, type, FFT size, form).  A correlation whose kernel changes with
+// every call (a trained filter) creates a handle per call, and seven device
+// allocations and frees, each of which waits for the device, cost it more than
+// ten times its kernels.  What is reused is memory and the tables that depend
+// on the size alone; a handle has one owner at a time, and the kernel's
+// spectrum is computed anew for each.  At most 4 idle handles and 64 MB of
+// their growing buffers are kept, the oldest goes first, and all go when an
+// allocation fails.
+class handle_pool {
+public:
+    static constexpr size_t MAX_IDLE  = 4;
+    static constexpr size_t MAX_BYTES = size_t(64) << 20;
+
+    // An idle handle of this kind, or null.
+    pcx_fxcorr_s* take(int device, int dtype, size_t n, bool general) {
+        std::lock_guard<std::mutex> g(mu_);
+        for (auto it = idle_.begin(); it != idle_.end(); ++it) {
+            pcx_fxcorr_s* h = *it;
+            if (h->device == device && h->dtype == dtype && h->n == n && h->general == general) {
+                idle_.erase(it);
+                return h;
+            }
+        }
+        return nullptr;
+    }
+    void give(pcx_fxcorr_s* h) {
+        std::list<pcx_fxcorr_s*> out;
+        {
+            std::lock_guard<std::mutex> g(mu_);
+            idle_.push_back(h);
+            size_t sum = 0;
+            for (auto it = idle_.end(); it != idle_.begin();) {    // newest first
+                --it;
+                sum += bytes(*it);
+                if (sum > MAX_BYTES || (size_t)std::distance(it, idle_.end()) > MAX_IDLE) {
+                    out.splice(out.begin(), idle_, idle_.begin(), std::next(it));
+                    break;
+                }
+            }
+        }
+        for (pcx_fxcorr_s* o: out) free_handle(o);
+    }
+    void drain() {
+        std::list<pcx_fxcorr_s*> out;
+        {
+            std::lock_guard<std::mutex> g(mu_);
+            out.swap(idle_);
+        }
+        for (pcx_fxcorr_s* o: out) free_handle(o);
+    }
+
+private:
+    static size_t bytes(const pcx_fxcorr_s* h) {
+        return h->flags_cap * sizeof(unsigned) + h->gscratch_bytes + (h->plan ? h->plan->scratch_bytes : 0);
+    }
+    std::mutex               mu_;
+    std::list<pcx_fxcorr_s*> idle_;
+};
+// never destroyed: at process exit the CUDA context may be gone first
+handle_pool& pool() {
+    static handle_pool* p = new handle_pool;
+    return *p;
+}
+
+// Remember where the handle's last call ends.
+void note_call(pcx_fxcorr_s* h, cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        h->unsure = true;
+        return;
+    }
+    if (h->used && st != h->last) h->unsure = true;
+    if (cudaEventRecord(h->done, st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        h->unsure = true;
+    }
+    h->last = st;
+    h->used = true;
+}
+
+// K = FFT(g zero-padded to N) / N, natural order, interleaved (fxcorr.hpp:62-69),
+// and its reordered copy for the in-CTA four-step form.
+int set_kernel(pcx_fxcorr_s* h, const void* g) {
+    if (int rc = pcx_fft_run(h->plan, h->kspec, g, h->k, 1, h->pack_g, PCX_FORWARD, 0, 1, 2 * h->n,
+                             (h->k + h->pack_g - 1) / h->pack_g * 2 * h->pack_g, nullptr, 0, 0, 1.0 / (double)h->n)) {
+        return rc;
+    }
+    if (h->x2d) {
+        const int l1 = (h->log_n + 1) / 2, l2 = h->log_n / 2;
+        PCX_CUDA_TRY(pcx_xc2_perm_spectrum(h->kspec, h->x2d, l1, l2, 0));
+    }
+    return PCX_OK;
+}
+
+// Device memory, tables and launch attributes of a new handle.
+int init_handle(pcx_fxcorr_s* h) {
+    const int    log_n = h->log_n;
+    const bool   f64   = h->dtype == PCX_F64;
+    const size_t eb    = f64 ? 16 : 8;
+    PCX_CUDA_TRY(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device));
+    PCX_CUDA_TRY(cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming));
+    if (int rc = pcx_plan_create(&h->plan, h->n, h->dtype, PCX_ORDER_NORMAL, 2048)) return rc;
+    PCX_CUDA_TRY(cudaMalloc(&h->tw, h->n * eb));
+    PCX_CUDA_TRY(cudaMalloc(&h->kspec, h->n * eb));
+    PCX_CUDA_TRY(pcx_gen_twiddles(h->tw, (int)h->n, log_n, 1, f64, 0));
+    if (int rc = f64 ? dispatch_xc<double>(log_n, xc_args{}, nullptr, 0, 0, true)
+                     : dispatch_xc<float>(log_n, xc_args{}, nullptr, 0, 0, true)) {
+        return rc;
+    }
+    if (int rc = f64 ? dispatch_kg<double>(log_n, kg_args{}, nullptr, 0, 0, true)
+                     : dispatch_kg<float>(log_n, kg_args{}, nullptr, 0, 0, true)) {
+        return rc;
+    }
+    if (!f64 && log_n <= 12 && !h->general) {
+        // its launch attributes now, not in a call that may be captured
+        int grid = 0;
+        if (int rc = dispatch_xc3_kg(log_n, kg_args{}, nullptr, 0, h->sms, &grid)) return rc;
+        if (int rc = dispatch_xc3(log_n, xc_args{}, nullptr, 0, h->sms)) return rc;
+        h->x3 = true;
+    }
+    if (!f64 && log_n >= 13 && !h->general) return log_n == 14 ? init_xc2<14>(h) : init_xc2<13>(h);
+    return PCX_OK;
+}
+
+}    // namespace
+
 extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int pack_g, size_t n_fft, int dtype) {
     return pcx_guard([&]() -> int {
         if (!out) return pcx_fail(PCX_ERR_INVALID, "handle pointer is null");
@@ -377,73 +526,75 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
             return pcx_fail(PCX_ERR_UNSUPPORTED, "fused correlator supports fft sizes 2^6..2^" + std::to_string(maxlog));
         }
         if (!g) return pcx_fail(PCX_ERR_INVALID, "null kernel pointer");
-        auto h    = new pcx_fxcorr_s{};
-        h->dtype  = dtype;
-        h->k      = k;
-        h->n      = n_fft;
-        h->log_n  = log_n;
-        h->pack_g = pack_g;
-        cudaGetDevice(&h->device);
-        auto fail = [&](int rc) {
-            pcx_fxcorr_destroy(h);
-            return rc;
+        const bool general = std::getenv("PCX_XC_GENERAL") != nullptr;
+        int        device  = 0;
+        PCX_CUDA_TRY(cudaGetDevice(&device));
+        auto make = [&](pcx_fxcorr_s*& h) -> int {
+            h = pool().take(device, dtype, n_fft, general);
+            if (h) {
+                // its last owner's kernels may still read what is set below
+                cudaError_t e = cudaSuccess;
+                if (h->unsure) e = cudaDeviceSynchronize();
+                else if (h->used) e = cudaStreamWaitEvent(0, h->done, 0);
+                if (e == cudaSuccess && h->ctl) e = cudaMemsetAsync(h->ctl, 0, 2 * sizeof(unsigned), 0);
+                PCX_CUDA_TRY(e);
+                h->used = h->unsure = false;
+            } else {
+                h          = new pcx_fxcorr_s{};
+                h->dtype   = dtype;
+                h->n       = n_fft;
+                h->log_n   = log_n;
+                h->device  = device;
+                h->general = general;
+                if (int rc = init_handle(h)) return rc;
+            }
+            h->k      = k;
+            h->pack_g = pack_g;
+            if (int rc = set_kernel(h, g)) return rc;
+            PCX_CUDA_TRY(cudaStreamSynchronize(0));    // g is read, the tables and K are there
+            return PCX_OK;
         };
-        PCX_CUDA_TRY(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device));
-        int rc = pcx_plan_create(&h->plan, n_fft, dtype, PCX_ORDER_NORMAL, 2048);
-        if (rc) return fail(rc);
-        const size_t eb = dtype == PCX_F64 ? 16 : 8;
-        cudaError_t  e  = cudaMalloc(&h->tw, n_fft * eb);
-        if (e == cudaSuccess) e = cudaMalloc(&h->kspec, n_fft * eb);
-        if (e == cudaSuccess) e = pcx_gen_twiddles(h->tw, (int)n_fft, log_n, 1, dtype == PCX_F64, 0);
-        if (e != cudaSuccess) return fail(pcx_fail(PCX_ERR_CUDA, cudaGetErrorString(e)));
-        // K = FFT(g zero-padded to N) / N, natural order, interleaved (fxcorr.hpp:62-69)
-        rc = pcx_fft_run(h->plan, h->kspec, g, k, 1, pack_g, PCX_FORWARD, 0, 1, 2 * n_fft,
-                         (k + pack_g - 1) / pack_g * 2 * pack_g, nullptr, 0, 0, 1.0 / (double)n_fft);
-        if (rc) return fail(rc);
-        rc = dtype == PCX_F64 ? dispatch_xc<double>(log_n, xc_args{}, nullptr, 0, 0, true)
-                              : dispatch_xc<float>(log_n, xc_args{}, nullptr, 0, 0, true);
-        if (rc) return fail(rc);
-        rc = dtype == PCX_F64 ? dispatch_kg<double>(log_n, kg_args{}, nullptr, 0, 0, true)
-                              : dispatch_kg<float>(log_n, kg_args{}, nullptr, 0, 0, true);
-        if (rc) return fail(rc);
-        if (dtype == PCX_F32 && log_n <= 12 && std::getenv("PCX_XC_GENERAL") == nullptr) {
-            // its launch attributes now, not in a call that may be captured
-            int  grid = 0;
-            auto kg   = kg_args{};
-            rc        = dispatch_xc3_kg(log_n, kg, nullptr, 0, h->sms, &grid);
-            if (!rc) rc = dispatch_xc3(log_n, xc_args{}, nullptr, 0, h->sms);
-            if (rc) return fail(rc);
-            h->x3 = true;
+        pcx_fxcorr_s* h  = nullptr;
+        int           rc = make(h);
+        if (rc == PCX_ERR_CUDA) {
+            // out of memory, perhaps: once more without the idle handles' memory
+            (void)cudaGetLastError();
+            if (h) free_handle(h);
+            h = nullptr;
+            pool().drain();
+            rc = make(h);
         }
-        if (dtype == PCX_F32 && (log_n == 13 || log_n == 14) && std::getenv("PCX_XC_GENERAL") == nullptr) {
-            rc = log_n == 14 ? init_xc2<14>(h) : init_xc2<13>(h);
-            if (rc) return fail(rc);
+        if (rc) {
+            if (h) free_handle(h);
+            return rc;
         }
-        e = cudaDeviceSynchronize();
-        if (e != cudaSuccess) return fail(pcx_fail(PCX_ERR_CUDA, cudaGetErrorString(e)));
         *out = h;
         return PCX_OK;
     });
 }
 
 extern "C" int pcx_fxcorr_destroy(pcx_fxcorr h) {
-    if (!h) return PCX_OK;
-    if (h->plan) pcx_plan_destroy(h->plan);
-    if (h->tw) cudaFree(h->tw);
-    if (h->kspec) cudaFree(h->kspec);
-    if (h->ctl) cudaFree(h->ctl);
-    if (h->gscratch) cudaFree(h->gscratch);
-    if (h->x2d) cudaFree(h->x2d);
-    delete h;
-    return PCX_OK;
+    return pcx_guard([&]() -> int {
+        if (h) pool().give(h);
+        return PCX_OK;
+    });
+}
+
+extern "C" int pcx_fxcorr_release_idle(void) {
+    return pcx_guard([&]() -> int {
+        pool().drain();
+        return PCX_OK;
+    });
 }
 
 extern "C" int pcx_fxcorr_exec(pcx_fxcorr h, void* dst, const void* src, size_t len, int pack, size_t channels,
                                size_t dst_stride, size_t src_stride, void* stream) {
     return pcx_guard([&]() -> int {
         if (!h) return pcx_fail(PCX_ERR_INVALID, "handle is null");
-        return run_xc(h, dst, src, len, pack, channels, dst_stride, src_stride, false,
-                      static_cast<cudaStream_t>(stream));
+        const cudaStream_t st = static_cast<cudaStream_t>(stream);
+        const int          rc = run_xc(h, dst, src, len, pack, channels, dst_stride, src_stride, false, st);
+        note_call(h, st);
+        return rc;
     });
 }
 
@@ -461,98 +612,105 @@ extern "C" int pcx_fxcorr_status(pcx_fxcorr h) {
     });
 }
 
+static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const void* x, size_t len, int pack,
+                   size_t channels, size_t stride, cudaStream_t st) {
+    // d/dx: convolution of gy with g
+    if (gx) {
+        int rc = run_xc(h, gx, gy, len, pack, channels, stride, stride, true, st);
+        if (rc) return rc;
+    }
+    if (!gg) return PCX_OK;
+    if (!x) return pcx_fail(PCX_ERR_INVALID, "kernel gradient needs the forward input x");
+    if (int rc = check_pack(pack)) return rc;
+    const size_t n    = h->n;
+    const size_t step = (n - (h->k - 1)) / pack * pack;
+    if (step == 0 || len == 0 || channels == 0) return pcx_fail(PCX_ERR_INVALID, "nothing to differentiate");
+    const size_t nblk  = (len + step - 1) / step;
+    const size_t total = nblk * channels;
+    const size_t eb    = h->dtype == PCX_F64 ? 16 : 8;
+    // FP32 at pack 8 on 16-byte aligned rows: the whole-window form up to
+    // 2^12 points, the in-CTA four-step form with the per-thread spectra in
+    // tensor memory at 2^13 and 2^14
+    const bool rows = pack == 8 && (channels == 1 || stride % 4 == 0) &&
+                      (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gy)) % 16 == 0;
+    const bool x3 = h->x3 && rows, x2 = h->x2d && rows;
+    kg_args    a{};
+    a.total  = (long long)total;
+    int grid = (int)std::min<size_t>(total, (size_t)h->sms);
+    if (x3) {
+        if (int rc = dispatch_xc3_kg(h->log_n, a, nullptr, st, h->sms, &grid)) return rc;
+    }
+    // sums of the blocks, the general form's spectra, the sum and its inverse
+    const size_t rows_s = (size_t)grid * (x3 || x2 ? 1 : 2);
+    const size_t need   = (rows_s + 2) * n * eb;
+    if (h->gscratch_bytes < need) {
+        if (h->gscratch) cudaFree(h->gscratch);
+        h->gscratch       = nullptr;
+        h->gscratch_bytes = 0;
+        PCX_CUDA_TRY(cudaMalloc(&h->gscratch, need));
+        h->gscratch_bytes = need;
+    }
+    if (int rc = ensure_flags(h, 1)) return rc;
+    if (!x3) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), st));
+    char* base = static_cast<char*>(h->gscratch);
+    a.x       = x;
+    a.gy      = gy;
+    a.stride  = (long long)stride;
+    a.len     = (long long)len;
+    a.lp      = __builtin_ctz(pack);
+    a.step    = (int)step;
+    a.nblk    = (int)nblk;
+    a.counter = h->ctl;
+    a.error   = reinterpret_cast<int*>(h->ctl + 1);
+    a.acc     = base;
+    a.xspec   = base + (size_t)grid * n * eb;
+    void* sum = base + rows_s * n * eb;
+    void* inv = base + (rows_s + 1) * n * eb;
+    int rc;
+    if (x3) {
+        rc = dispatch_xc3_kg(h->log_n, a, h->plan->stwL, st, h->sms, &grid);
+    } else if (x2) {
+        xc2_kg_args b{};
+        b.base = a;
+        b.stw1 = h->x2_stw1;
+        b.stw2 = h->x2_stw2;
+        b.tws  = h->x2_tws;
+        rc     = h->log_n == 14 ? launch_xc2_kg<14>(b, st, grid, false) : launch_xc2_kg<13>(b, st, grid, false);
+    } else {
+        rc = h->dtype == PCX_F64 ? dispatch_kg<double>(h->log_n, a, h->tw, st, grid, false)
+                                 : dispatch_kg<float>(h->log_n, a, h->tw, st, grid, false);
+    }
+    if (rc) return rc;
+    if (h->dtype == PCX_F64) {
+        k_kgrad_reduce<double><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
+            static_cast<const cpx<double>*>(a.acc), grid, (int)n, static_cast<cpx<double>*>(sum));
+    } else {
+        k_kgrad_reduce<float><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
+            static_cast<const cpx<float>*>(a.acc), grid, (int)n, static_cast<cpx<float>*>(sum));
+    }
+    PCX_CUDA_TRY(cudaGetLastError());
+    // gg[j] = (1/N) sum_k S[k] e^{+2 pi i jk/N}, j < K
+    rc = pcx_fft_run(h->plan, inv, sum, 0, 1, 1, PCX_INVERSE, 1, 1, 2 * n, 2 * n, nullptr, 0, st, 1.0);
+    if (rc) return rc;
+    const int lpg = __builtin_ctz(h->pack_g);
+    if (h->dtype == PCX_F64) {
+        k_scale_pack<double><<<(unsigned)((h->k + 255) / 256), 256, 0, st>>>(
+            static_cast<const cpx<double>*>(inv), (int)h->k, lpg, static_cast<double*>(gg));
+    } else {
+        k_scale_pack<float><<<(unsigned)((h->k + 255) / 256), 256, 0, st>>>(
+            static_cast<const cpx<float>*>(inv), (int)h->k, lpg, static_cast<float*>(gg));
+    }
+    PCX_CUDA_TRY(cudaGetLastError());
+    return PCX_OK;
+}
+
 extern "C" int pcx_fxcorr_vjp(pcx_fxcorr h, void* gx, void* gg, const void* gy, const void* x, size_t len, int pack,
                               size_t channels, size_t stride, void* stream) {
     return pcx_guard([&]() -> int {
         if (!h) return pcx_fail(PCX_ERR_INVALID, "handle is null");
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        // d/dx: convolution of gy with g
-        if (gx) {
-            int rc = run_xc(h, gx, gy, len, pack, channels, stride, stride, true, st);
-            if (rc) return rc;
-        }
-        if (!gg) return PCX_OK;
-        if (!x) return pcx_fail(PCX_ERR_INVALID, "kernel gradient needs the forward input x");
-        if (int rc = check_pack(pack)) return rc;
-        const size_t n    = h->n;
-        const size_t step = (n - (h->k - 1)) / pack * pack;
-        if (step == 0 || len == 0 || channels == 0) return pcx_fail(PCX_ERR_INVALID, "nothing to differentiate");
-        const size_t nblk  = (len + step - 1) / step;
-        const size_t total = nblk * channels;
-        const size_t eb    = h->dtype == PCX_F64 ? 16 : 8;
-        // FP32 at pack 8 on 16-byte aligned rows: the whole-window form up to
-        // 2^12 points, the in-CTA four-step form with the per-thread spectra in
-        // tensor memory at 2^13 and 2^14
-        const bool rows = pack == 8 && (channels == 1 || stride % 4 == 0) &&
-                          (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gy)) % 16 == 0;
-        const bool x3 = h->x3 && rows, x2 = h->x2d && rows;
-        kg_args    a{};
-        a.total  = (long long)total;
-        int grid = (int)std::min<size_t>(total, (size_t)h->sms);
-        if (x3) {
-            if (int rc = dispatch_xc3_kg(h->log_n, a, nullptr, st, h->sms, &grid)) return rc;
-        }
-        // sums of the blocks, the general form's spectra, the sum and its inverse
-        const size_t rows_s = (size_t)grid * (x3 || x2 ? 1 : 2);
-        const size_t need   = (rows_s + 2) * n * eb;
-        if (h->gscratch_bytes < need) {
-            if (h->gscratch) cudaFree(h->gscratch);
-            h->gscratch       = nullptr;
-            h->gscratch_bytes = 0;
-            PCX_CUDA_TRY(cudaMalloc(&h->gscratch, need));
-            h->gscratch_bytes = need;
-        }
-        if (int rc = ensure_flags(h, 1)) return rc;
-        if (!x3) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), st));
-        char* base = static_cast<char*>(h->gscratch);
-        a.x       = x;
-        a.gy      = gy;
-        a.stride  = (long long)stride;
-        a.len     = (long long)len;
-        a.lp      = __builtin_ctz(pack);
-        a.step    = (int)step;
-        a.nblk    = (int)nblk;
-        a.counter = h->ctl;
-        a.error   = reinterpret_cast<int*>(h->ctl + 1);
-        a.acc     = base;
-        a.xspec   = base + (size_t)grid * n * eb;
-        void* sum = base + rows_s * n * eb;
-        void* inv = base + (rows_s + 1) * n * eb;
-        int rc;
-        if (x3) {
-            rc = dispatch_xc3_kg(h->log_n, a, h->plan->stwL, st, h->sms, &grid);
-        } else if (x2) {
-            xc2_kg_args b{};
-            b.base = a;
-            b.stw1 = h->x2_stw1;
-            b.stw2 = h->x2_stw2;
-            b.tws  = h->x2_tws;
-            rc     = h->log_n == 14 ? launch_xc2_kg<14>(b, st, grid, false) : launch_xc2_kg<13>(b, st, grid, false);
-        } else {
-            rc = h->dtype == PCX_F64 ? dispatch_kg<double>(h->log_n, a, h->tw, st, grid, false)
-                                     : dispatch_kg<float>(h->log_n, a, h->tw, st, grid, false);
-        }
-        if (rc) return rc;
-        if (h->dtype == PCX_F64) {
-            k_kgrad_reduce<double><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
-                static_cast<const cpx<double>*>(a.acc), grid, (int)n, static_cast<cpx<double>*>(sum));
-        } else {
-            k_kgrad_reduce<float><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
-                static_cast<const cpx<float>*>(a.acc), grid, (int)n, static_cast<cpx<float>*>(sum));
-        }
-        PCX_CUDA_TRY(cudaGetLastError());
-        // gg[j] = (1/N) sum_k S[k] e^{+2 pi i jk/N}, j < K
-        rc = pcx_fft_run(h->plan, inv, sum, 0, 1, 1, PCX_INVERSE, 1, 1, 2 * n, 2 * n, nullptr, 0, st, 1.0);
-        if (rc) return rc;
-        const int lpg = __builtin_ctz(h->pack_g);
-        if (h->dtype == PCX_F64) {
-            k_scale_pack<double><<<(unsigned)((h->k + 255) / 256), 256, 0, st>>>(
-                static_cast<const cpx<double>*>(inv), (int)h->k, lpg, static_cast<double*>(gg));
-        } else {
-            k_scale_pack<float><<<(unsigned)((h->k + 255) / 256), 256, 0, st>>>(
-                static_cast<const cpx<float>*>(inv), (int)h->k, lpg, static_cast<float*>(gg));
-        }
-        PCX_CUDA_TRY(cudaGetLastError());
-        return PCX_OK;
+        const cudaStream_t st = static_cast<cudaStream_t>(stream);
+        const int          rc = run_vjp(h, gx, gg, gy, x, len, pack, channels, stride, st);
+        note_call(h, st);
+        return rc;
     });
 }

@@ -467,6 +467,11 @@ class fxcorr_unit:
                 pass
             self._h = None
 
+    @staticmethod
+    def release_idle() -> None:
+        """Free the device memory kept from destroyed correlators (pcx_fxcorr_release_idle)."""
+        _lib.check(_lib.lib().pcx_fxcorr_release_idle())
+
     def fft_size(self) -> int:
         return self._n
 
