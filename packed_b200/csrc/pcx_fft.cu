@@ -294,14 +294,11 @@ static int plan_init_tables(pcx_plan_s* p) {
             PCX_CUDA_TRY(cudaMalloc(&p->stw, (size_t)std::max(e1, 2) * eb));
             p->stwL = p->stw;
             PCX_CUDA_TRY(pcx_v2_stage_twiddles(log_n, p->stwL, f64, 0, &e1));
-            v2_args z{};
-            cudaError_t e = pcx_v2_single(f64, log_n, z, 0, true);
-            if (e != cudaErrorNotSupported) PCX_CUDA_TRY(e);
-            v3_args z3{};
-            e = pcx_v3_single(f64, log_n, z3, 0, p->sms, true);
-            if (e != cudaErrorNotSupported) PCX_CUDA_TRY(e);
-            e = pcx_v3_single_any(f64, log_n, z3, 0, p->sms, true);
-            if (e != cudaErrorNotSupported) PCX_CUDA_TRY(e);
+            for (cudaError_t e: {pcx_rows(f64, log_n, {}, 0, true), pcx_rows_any(f64, log_n, {}, 0, true),
+                                 pcx_v3_single(f64, log_n, {}, 0, p->sms, true),
+                                 pcx_v3_single_any(f64, log_n, {}, 0, p->sms, true)}) {
+                if (e != cudaErrorNotSupported) PCX_CUDA_TRY(e);
+            }
         } else {
             PCX_CUDA_TRY(pcx_v2_stage_twiddles(p->log_n1, nullptr, f64, 0, &e1));
             PCX_CUDA_TRY(pcx_v2_stage_twiddles(p->log_n2, nullptr, f64, 0, &e2));
@@ -346,10 +343,12 @@ static int plan_init_tables(pcx_plan_s* p) {
             p->fst2 = static_cast<char*>(p->fst) + (size_t)f1 * eb;
             PCX_CUDA_TRY(pcx_fourstep_tables(p->log_n1, p->fst1, f64, 0, &f1));
             PCX_CUDA_TRY(pcx_fourstep_tables(p->log_n2, p->fst2, f64, 0, &f2));
-            // N = 8192 in FP32 also has a one-pass form (64 KB rows in shared memory)
-            v3_args z3{};
-            if (pcx_v3_single(f64, log_n, z3, 0, p->sms, true) == cudaSuccess &&
-                pcx_v3_single_any(f64, log_n, z3, 0, p->sms, true) == cudaSuccess) {
+            // 2^13 has a one-pass form (a block of 512 threads a row)
+            if (pcx_rows(f64, log_n, {}, 0, true) == cudaSuccess && pcx_rows_any(f64, log_n, {}, 0, true) == cudaSuccess) {
+                for (cudaError_t e: {pcx_v3_single(f64, log_n, {}, 0, p->sms, true),
+                                     pcx_v3_single_any(f64, log_n, {}, 0, p->sms, true)}) {
+                    if (e != cudaErrorNotSupported) PCX_CUDA_TRY(e);
+                }
                 int e3 = 0;
                 PCX_CUDA_TRY(pcx_v2_stage_twiddles(log_n, nullptr, f64, 0, &e3));
                 PCX_CUDA_TRY(cudaMalloc(&p->stw_one, (size_t)std::max(e3, 2) * eb));
@@ -801,10 +800,9 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
     h.conj_out = io.conj_out;
     h.scale    = io.scale;
 
-    // One-pass TMA-fed kernel (k_single3): its default form at the default packs
-    // and full rows, else its any-pack form.
-    const bool tma_rows    = batch == 1 || (sstride % vreals == 0 && dstride % vreals == 0);
-    auto       run_single3 = [&](const void* stw) {
+    // One pass: k_rows or k_single3, at the default packs and full rows their
+    // default forms, else their any-pack forms.
+    auto run_rows = [&](const void* stw) {
         v3_args t3{};
         t3.src        = src;
         t3.dst        = dst;
@@ -821,30 +819,25 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         t3.lp_src     = io.lp_src;
         t3.lp_dst     = io.lp_dst;
         t3.src_len    = io.src_len;
-        const bool plain = src_len == n && io.lp_src == lp_def && io.lp_dst == lp_def;
+        const uintptr_t both = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst);
+        t3.pairs             = both % eb == 0 && (batch == 1 || (sstride % 2 == 0 && dstride % 2 == 0));
+        const bool plain     = src_len == n && io.lp_src == lp_def && io.lp_dst == lp_def;
+        const bool natural   = io.order_in == 0 && io.order_out == 0;
+        const bool tma       = batch == 1 || (sstride % vreals == 0 && dstride % vreals == 0);
+        // natural order from 256 points on (FP64: 128) goes straight through
+        // registers; k_single3 is faster below and takes the other orders
+        if (natural && p->log_n >= 7 && (f64 || p->log_n >= 8 || !tma)) {
+            const cudaError_t e = (plain ? pcx_rows : pcx_rows_any)(f64, p->log_n, t3, st, false);
+            if (e != cudaErrorNotSupported) return e;
+        }
+        if (!tma) return cudaErrorNotSupported;
         return plain ? pcx_v3_single(f64, p->log_n, t3, st, p->sms, false)
                      : pcx_v3_single_any(f64, p->log_n, t3, st, p->sms, false);
     };
 
     if (!p->two_pass) {
-        // TMA-fed kernel: any order and pack width, rows on 16-byte strides
-        if (p->log_n >= 5 && tma_rows) {
-            const cudaError_t e = run_single3(p->stwL);
-            if (e != cudaErrorNotSupported) {
-                PCX_CUDA_TRY(e);
-                return PCX_OK;
-            }
-        }
-        const bool hot = io.order_in == 0 && io.order_out == 0 && src_len == n && io.lp_src == lp_def &&
-                         io.lp_dst == lp_def && p->log_n >= 7;
-        if (hot) {
-            h.src        = src;
-            h.dst        = dst;
-            h.src_stride = (long long)sstride;
-            h.dst_stride = (long long)dstride;
-            h.batch      = (long long)batch;
-            h.stw        = p->stwL;
-            cudaError_t e = pcx_v2_single(f64, p->log_n, h, st, false);
+        if (p->log_n >= 5) {
+            const cudaError_t e = run_rows(p->stwL);
             if (e != cudaErrorNotSupported) {
                 PCX_CUDA_TRY(e);
                 return PCX_OK;
@@ -859,9 +852,9 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
     }
 
     const bool tuned_one = ws || p->form == PCX_FORM_DEFAULT || p->form == PCX_FORM_ONEPASS;
-    if (p->stw_one && tuned_one && tma_rows) {
+    if (p->stw_one && tuned_one) {
         // one-pass form of a two-pass size
-        const cudaError_t e = run_single3(p->stw_one);
+        const cudaError_t e = run_rows(p->stw_one);
         if (e != cudaErrorNotSupported) {
             PCX_CUDA_TRY(e);
             return PCX_OK;

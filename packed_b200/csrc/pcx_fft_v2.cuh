@@ -17,6 +17,8 @@
 #include "pcx_fft_kernels.cuh"
 #include "pcx_tma.cuh"
 
+#include <type_traits>
+
 namespace pcxg {
 
 // ---- per-stage twiddle tables ------------------------------------------------
@@ -327,44 +329,122 @@ struct v2_args {
     const void* tw_b;          // W_{16*N2}^m, m < 16*N2
 };
 
+struct v3_args {
+    const void* src;
+    void*       dst;
+    long long   src_stride;
+    long long   dst_stride;
+    long long   batch;
+    int         conj_in;
+    int         conj_out;
+    int         order_in;
+    int         order_out;
+    double      scale;
+    const void* stw;
+    int*        error;    // set when a bounded wait gives up
+    // the any-pack forms only (k_rows and k_single3 with ANY):
+    int         lp_src;     // log2 pack widths
+    int         lp_dst;
+    int         src_len;    // valid source elements per row (zero-extended to N)
+    int         pairs;      // interleaved rows may be moved a complex number at a time (aligned)
+};
+
 // ---------------------------------------------------------------------------
-// Single-pass, natural order, N = 2^LOGL (128 <= N <= 4096), pack 2^LP.
-template<class T, int LOGL, int LP, int NT>
-__global__ void __launch_bounds__(NT) k_single2(v2_args a) {
-    using P          = splan<LOGL>;
+// Single pass, natural order on both sides: rows straight between HBM and
+// registers, 16 points per thread, shared memory for the exchanges only.
+//
+// Bound by HBM: what counts is warps in flight.  A thread keeps to 64
+// registers in FP32 (32 of them data) and 128 in FP64, so 32 (16) warps fit an
+// SM; their loads cover the latency without a copy ring, which at 16 warps
+// an SM was the faster form only with the ring's help, and a block's barriers
+// stall 128 threads at a time where a row allows it (256 for 4096 points).
+// Stage factors come through L1.  GB/s (16 B per point, 32 B in FP64), 512 MB
+// a buffer, of 6544 measured copy; before: the TMA-fed kernel (k_single3),
+// rows staged in shared memory both ways, 16 warps an SM (FP64: 8):
+//   N            256  512 1024 2048 4096 8192   FP64: 128  256  512 1024 2048 4096 8192
+//   before      5917 4944 4436 4544 4526 3255        4364 4982 4073 3516 3658 3860 1833
+//   this        6687 6237 5578 6014 5660 4225        6799 6779 5929 5044 5317 5092 3320
+//   256 threads 6729 6168 5582 5773                  6587 6798 5576 4557 4901
+// (8192 before: the four-step's tuned form reached 3500 in FP32.)  With 3 and
+// 2 blocks of 256 threads in FP32: 4096 5480 and 4430.  At 128 points in FP32
+// a row's eight threads cover single 32-byte sectors and k_single3 is faster
+// (6270 against 5630); 16384 in one pass is slower (3043) than the four-step.
+template<class T, int LOGL>
+struct rows_cfg {
+    using P                   = splan<LOGL>;
+    static constexpr int NT   = P::TT > 128 ? P::TT : 128;
+    static constexpr int M    = NT / P::TT;
+    static constexpr int MINB = (sizeof(T) == 8 ? 512 : 1024) / NT;
+    using X                   = xch_blocked<P::L, M>;
+    static constexpr int SMEM = X::size * (int)sizeof(cpx<T>);
+};
+
+template<class T, int LOGL, int LP, bool ANY>
+__global__ void __launch_bounds__(rows_cfg<T, LOGL>::NT, rows_cfg<T, LOGL>::MINB) k_rows(v3_args a) {
+    using F          = rows_cfg<T, LOGL>;
+    using P          = typename F::P;
     constexpr int L  = P::L;
     constexpr int E  = P::E;
     constexpr int TT = P::TT;
-    constexpr int M  = NT / TT;
-    constexpr int PK = 1 << LP;
-    static_assert(TT % PK == 0, "pack must divide threads per row");
-    using X = xch_blocked<L, M>;
+    using V2         = std::conditional_t<sizeof(T) == 4, float2, double2>;
+    static_assert(TT % (1 << LP) == 0, "pack must divide threads per row");
     extern __shared__ __align__(16) unsigned char smem[];
-    cpx<T>*       xch = reinterpret_cast<cpx<T>*>(smem);
-    const auto*   stw = reinterpret_cast<const cpx<T>*>(a.stw);
-    const int     tid = threadIdx.x;
-    const int     m   = tid / TT;
-    const int     t   = tid - m * TT;
-    const long long row = (long long)blockIdx.x * M + m;
-    const bool    live  = row < a.batch;
-    const T*      src = reinterpret_cast<const T*>(a.src) + (live ? row : 0) * a.src_stride + pk<LP>(t);
-    T*            dst = reinterpret_cast<T*>(a.dst) + row * a.dst_stride + pk<LP>(t);
+    cpx<T>*         xch  = reinterpret_cast<cpx<T>*>(smem);
+    const auto*     stw  = reinterpret_cast<const cpx<T>*>(a.stw);
+    const int       m    = threadIdx.x / TT;
+    const int       t    = threadIdx.x - m * TT;
+    const long long row  = (long long)blockIdx.x * F::M + m;
+    const bool      live = row < a.batch;
+    const T*        src  = reinterpret_cast<const T*>(a.src) + (live ? row : 0) * a.src_stride;
+    T*              dst  = reinterpret_cast<T*>(a.dst) + row * a.dst_stride;
+    const int       lps  = ANY ? a.lp_src : LP;
+    const int       lpd  = ANY ? a.lp_dst : LP;
 
     cpx<T> v[E];
-    static_for<E>([&](auto ic) {
-        constexpr int i = decltype(ic)::value;
-        const T       re = src[2 * i * TT], im = src[2 * i * TT + PK];
-        v[i]           = {re, a.conj_in ? -im : im};
-    });
-    stage_compute_tab<P, 0>(v, t, stw);
-    run_stages_tab<P, X>(v, xch, m, t, stw);
-    if (live) {
-        const T sc  = T(a.scale);
-        const T sim = a.conj_out ? -sc : sc;
+    if (ANY && (a.src_len < L || (1 << lps) > TT)) {
         static_for<E>([&](auto ic) {
-            constexpr int i   = decltype(ic)::value;
-            dst[2 * i * TT]      = v[i].re * sc;
-            dst[2 * i * TT + PK] = v[i].im * sim;
+            constexpr int i = decltype(ic)::value;
+            const int     e = t + i * TT, o = (int)pk_re(e, lps);
+            v[i]            = {T(0), T(0)};
+            if (e < a.src_len) v[i] = {src[o], src[o + (1 << lps)]};
+        });
+    } else if (ANY && lps == 0 && a.pairs) {
+        static_for<E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            const V2      x = reinterpret_cast<const V2*>(src)[t + i * TT];
+            v[i]            = {x.x, x.y};
+        });
+    } else {
+        const T* s = src + (ANY ? (int)pk_re(t, lps) : pk<LP>(t));
+        static_for<E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            v[i]            = {s[2 * i * TT], s[2 * i * TT + (ANY ? 1 << lps : 1 << LP)]};
+        });
+    }
+    if (a.conj_in) static_for<E>([&](auto ic) { v[decltype(ic)::value].im = -v[decltype(ic)::value].im; });
+    stage_compute_tab<P, 0>(v, t, stw);
+    run_stages_tab<P, typename F::X, false, (TT <= 32 ? -1 : 0)>(v, xch, m, t, stw);
+    if (!live) return;
+    const T sc  = T(a.scale);
+    const T sim = a.conj_out ? -sc : sc;
+    if (ANY && (1 << lpd) > TT) {
+        static_for<E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            const int     o = (int)pk_re(t + i * TT, lpd);
+            dst[o]              = v[i].re * sc;
+            dst[o + (1 << lpd)] = v[i].im * sim;
+        });
+    } else if (ANY && lpd == 0 && a.pairs) {
+        static_for<E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            __stcs(reinterpret_cast<V2*>(dst) + t + i * TT, V2{v[i].re * sc, v[i].im * sim});
+        });
+    } else {
+        T* d = dst + (ANY ? (int)pk_re(t, lpd) : pk<LP>(t));
+        static_for<E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            __stcs(d + 2 * i * TT, v[i].re * sc);
+            __stcs(d + 2 * i * TT + (ANY ? 1 << lpd : 1 << LP), v[i].im * sim);
         });
     }
 }
@@ -480,30 +560,13 @@ __global__ void __launch_bounds__(NT, 2) k_row2(v2_args a) {
 // TMA-fed single pass.  Persistent CTAs; each tile (M rows) is brought into
 // shared memory by one-dimensional bulk copies through a two-stage ring, so
 // the next tiles are in flight while this one is transformed.  Stage 0 reads
-// the packed rows from shared memory (any input order), the last stage
-// writes packed rows into a staging area (any output order) that the threads
-// copy out with 16-byte stores.  Rows are padded in shared memory so that
-// the rows of one warp fall into different banks.
+// the packed rows from shared memory (any input order); outputs in natural
+// order are stored from registers (s3_cfg::DIRECT), in another order the last
+// stage writes packed rows into a staging area that the threads copy out with
+// 16-byte stores.  Rows are padded in shared memory so that the rows of one
+// warp fall into different banks.
 namespace pcxg {
 
-struct v3_args {
-    const void* src;
-    void*       dst;
-    long long   src_stride;
-    long long   dst_stride;
-    long long   batch;
-    int         conj_in;
-    int         conj_out;
-    int         order_in;
-    int         order_out;
-    double      scale;
-    const void* stw;
-    int*        error;    // set when a bounded wait gives up
-    // the any-pack form only (k_single3 with ANY):
-    int         lp_src;     // log2 pack widths
-    int         lp_dst;
-    int         src_len;    // valid source elements per row (zero-extended to N)
-};
 
 // Read (re, im) stored `pk_off` reals apart at `o`; lanes with bit SW set
 // fetch the imaginary part first, so the two halves of each shared-memory
@@ -527,63 +590,60 @@ template<int TT>
 __host__ __device__ constexpr int single3_pad() {
     return TT >= 32 ? 0 : (TT >= 8 ? 8 : 4);
 }
-// Resident CTAs per SM a single-pass launch is built for (registers: 128 per
-// thread either way).
-__host__ __device__ constexpr int single3_minb(int nt) { return nt >= 512 ? 1 : 2; }
-template<class T, int LOGL, int NT>
-__host__ __device__ constexpr int single3_base_smem() {
-    using P          = splan<LOGL>;
-    constexpr int M  = NT / P::TT;
-    constexpr int RS = 2 * P::L + single3_pad<P::TT>();
-    return 2 * M * RS * (int)sizeof(T) + xch_blocked<P::L, M>::size * (int)sizeof(cpx<T>);
-}
-template<class T, int LOGL, int NT>
-__host__ __device__ constexpr bool single3_tws() {
-    return stw_fits(single3_base_smem<T, LOGL, NT>(), stage_tw_smem_bytes<splan<LOGL>, T>(), single3_minb(NT));
-}
-template<class T, int LOGL, int NT>
-__host__ __device__ constexpr int single3_smem() {
-    return single3_tws<T, LOGL, NT>()
-               ? smem_align16(single3_base_smem<T, LOGL, NT>()) + stage_tw_smem_bytes<splan<LOGL>, T>()
-               : single3_base_smem<T, LOGL, NT>();
-}
+// Shape of the TMA-fed one-pass kernel at a size: four warps a block at 32
+// and 64 points (GB/s, 512 MB, 128 and 256 threads: FP32 4784 and 3411, 5877
+// and 4820; FP64 5085 and 3360, 6098 and 5518), else eight.
+template<class T, int LOGL>
+struct s3_cfg {
+    using P                    = splan<LOGL>;
+    static constexpr bool F64  = sizeof(T) == 8;
+    static constexpr int  NT   = LOGL >= 13 ? 512 : (LOGL <= 6 ? 128 : 256);
+    static constexpr int  MINB = NT == 512 ? 1 : (NT == 128 && !F64 ? 5 : 2);    // blocks per SM
+    // natural-order outputs straight from registers; with fewer than eight
+    // threads a row in FP32 they would cover parts of sectors (64 points: 4680
+    // against 5877 GB/s staged), else they save a staging pass (128: 6270, 5305)
+    static constexpr bool DIRECT = F64 || LOGL > 6;
+    static constexpr int  M    = NT / P::TT;                        // rows per tile
+    static constexpr int  RS   = 2 * P::L + single3_pad<P::TT>();    // shared-memory row stride (reals)
+    using X                    = xch_blocked<P::L, M>;
+    static constexpr int  STAGE = M * RS * (int)sizeof(T);
+    static constexpr int  XB   = X::size * (int)sizeof(cpx<T>);
+    static constexpr int  BASE = smem_align16(2 * STAGE + XB);
+    static constexpr int  TAB  = stage_tw_smem_bytes<P, T>();
+    static constexpr bool SH   = stw_fits(BASE, TAB, MINB);    // stage factors in shared memory
+    static constexpr int  SMEM = SH ? BASE + TAB : BASE;
+    static_assert(XB >= STAGE, "staging fits the exchange buffer");
+    static_assert((RS * (int)sizeof(T)) % 16 == 0, "rows stay 16-byte aligned");
+};
 
 // ANY: source and destination packs of any width up to N (each its own, given
 // at run time) and rows shorter than N.  The row is the same 2*N contiguous
 // reals at every width and lds_swapped / sts_swapped stay free of bank
 // conflicts at widths 1..16, so the form costs an index per element (none in
 // natural order with packs of at most TT elements: one base per thread).
-// Bound by the load/store pipe and HBM like the default form.  2048 points,
-// 5003 rows, rows of 1500 interleaved samples to packed spectra and packed
-// spectra to interleaved rows: the general kernel (plain loads into one
-// buffer, twiddles from global memory) 170 us, this
-// one 91 us for both.
-template<class T, int LOGL, int LP, int NT, bool ANY = false>
-__global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
-    using P             = splan<LOGL>;
+// Bound by the load/store pipe and HBM like the default form.
+template<class T, int LOGL, int LP, bool ANY>
+__global__ void __launch_bounds__(s3_cfg<T, LOGL>::NT, s3_cfg<T, LOGL>::MINB) k_single3(v3_args a) {
+    using F             = s3_cfg<T, LOGL>;
+    using P             = typename F::P;
+    using X             = typename F::X;
     constexpr int L     = P::L;
     constexpr int E     = P::E;
     constexpr int TT    = P::TT;
-    constexpr int M     = NT / TT;
-    constexpr int PADR  = single3_pad<TT>();
-    constexpr int RS    = 2 * L + PADR;    // shared-memory row stride (reals)
-    constexpr int TILE  = M * RS;
+    constexpr int NT    = F::NT;
+    constexpr int M     = F::M;
+    constexpr int RS    = F::RS;
     constexpr int ROWB  = 2 * L * (int)sizeof(T);
     constexpr int V     = 16 / (int)sizeof(T);
     // a warp inside one row: its two halves read reals / imaginaries on
     // disjoint banks by swapping the order in half of the lanes (rows of fewer
     // than 32 threads keep the plain order: their rows are padded instead)
-    constexpr int SW    = TT >= 32 ? (sizeof(T) == 8 ? 8 : 16) : 0;
-    using X             = xch_blocked<L, M>;
-    static_assert(X::size * 2 >= TILE, "staging fits the exchange buffer");
-    static_assert((RS * (int)sizeof(T)) % 16 == 0, "rows stay 16-byte aligned");
+    constexpr int  SW   = TT >= 32 ? (sizeof(T) == 8 ? 8 : 16) : 0;
+    constexpr bool SH   = F::SH;
     extern __shared__ __align__(128) unsigned char smem[];
-    T*               in0 = reinterpret_cast<T*>(smem);
-    cpx<T>*          xch = reinterpret_cast<cpx<T>*>(in0 + 2 * TILE);
-    T*               stg = reinterpret_cast<T*>(xch);
     __shared__ uint64_t full[2];
-    constexpr bool   SH  = single3_tws<T, LOGL, NT>();
-    cpx<T>*          tws = reinterpret_cast<cpx<T>*>(smem + smem_align16(single3_base_smem<T, LOGL, NT>()));
+    cpx<T>*          xch = reinterpret_cast<cpx<T>*>(smem + 2 * F::STAGE);
+    cpx<T>*          tws = reinterpret_cast<cpx<T>*>(smem + F::BASE);
     const auto*      stw = SH ? tws : reinterpret_cast<const cpx<T>*>(a.stw);
     const T*         src = reinterpret_cast<const T*>(a.src);
     T*               dst = reinterpret_cast<T*>(a.dst);
@@ -599,8 +659,8 @@ __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
     const bool       cut  = ANY && a.src_len < L;
     const uint32_t   rowb = cut ? ((pk_re((uint32_t)a.src_len - 1, lps) + pks + 1) * (uint32_t)sizeof(T) + 15) & ~15u
                                 : (uint32_t)ROWB;
-    const bool       contig_in  = PADR == 0 && a.src_stride == 2 * L && !cut;
-    const bool       contig_out = PADR == 0 && a.dst_stride == 2 * L;
+    const bool       contig_in  = RS == 2 * L && a.src_stride == 2 * L && !cut;
+    const bool       contig_out = RS == 2 * L && a.dst_stride == 2 * L;
 
     if constexpr (SH) stage_tw_to_smem<P, T>(tws, a.stw, tid, NT);
     if (tid == 0) {
@@ -612,7 +672,7 @@ __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
 
     auto issue = [&](long long tile, int s) {    // thread 0 only
         const int  rows = (int)min((long long)M, a.batch - tile * M);
-        T*         buf  = in0 + s * TILE;
+        T*         buf  = reinterpret_cast<T*>(smem + s * F::STAGE);
         const T*   g    = src + tile * M * a.src_stride;
         mbar_arrive_expect_tx(&full[s], (uint32_t)rows * rowb);
         if (contig_in) {
@@ -626,23 +686,12 @@ __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
         if ((long long)blockIdx.x + gridDim.x < ntile) issue(blockIdx.x + gridDim.x, 1);
     }
 
-    long long k = 0;
-    for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x, ++k) {
-        const int      s   = (int)(k & 1);
-        const uint32_t par = (uint32_t)((k >> 1) & 1);
-        const bool     ok  = mbar_wait_bounded(&full[s], par);
-        if (__syncthreads_or(!ok)) {
-            // give up: record it, let the other stage's copy land, leave together
-            if (tid == 0) {
-                atomicExch(a.error, 1);
-                mbar_wait_bounded(&full[s], par, 100000000ull);
-                mbar_wait_bounded(&full[s ^ 1], par ^ (s ? 1u : 0u), 100000000ull);
-            }
-            __syncthreads();
-            return;
-        }
-        const T* in = in0 + s * TILE;
-        cpx<T>   v[E];
+    int      s   = 0;
+    uint32_t par = 0;
+    for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x, s ^= 1, par ^= s == 0) {
+        const bool ok  = mbar_wait_bounded(&full[s], par);
+        const T*   in  = reinterpret_cast<const T*>(smem + s * F::STAGE);
+        cpx<T>     v[E];
         if (ANY && a.order_in == 0 && pks <= TT) {
             // element t + i*TT lies 2*i*TT reals after element t at any such width
             const int o = m * RS + (int)pk_re(t, lps);
@@ -667,21 +716,65 @@ __global__ void __launch_bounds__(NT, single3_minb(NT)) k_single3(v3_args a) {
             });
         }
         fence_proxy_async_smem();
-        __syncthreads();    // stage s consumed: refill it with the tile after next
+        // every thread has read the tile (this barrier is also the vote on a
+        // copy that did not land in time)
+        if (__syncthreads_or(!ok)) {
+            // give up: record it, let the other stage's copy land, leave together
+            if (tid == 0) {
+                atomicExch(a.error, 1);
+                mbar_wait_bounded(&full[s], par, 100000000ull);
+                mbar_wait_bounded(&full[s ^ 1], par ^ (s ? 1u : 0u), 100000000ull);
+            }
+            __syncthreads();
+            return;
+        }
+        // the stage is consumed: refill it with the tile after next
         if (tid == 0 && tile + 2 * (long long)gridDim.x < ntile) issue(tile + 2 * (long long)gridDim.x, s);
         stage_compute_tab<P, 0>(v, t, stw);
         // a transform's TT <= 32 threads share one warp and its own exchange
-        // block: its exchanges need only that warp's barrier (the block-wide
-        // barriers before and after them order the stage and staging reuse)
+        // block: its exchanges need only that warp's barrier
         run_stages_tab<P, X, SH, (TT <= 32 ? -1 : 0)>(v, xch, m, t, stw);
-        __syncthreads();    // exchange reads done: reuse the buffer as staging
+        const T sc  = T(a.scale);
+        const T sim = a.conj_out ? -sc : sc;
+        if (F::DIRECT && a.order_out == 0) {
+            // v[i] is frequency t + i*TT: neighbouring threads store neighbouring reals
+            if (tile * M + m < a.batch) {
+                T* d = dst + (tile * M + m) * a.dst_stride;
+                if (!ANY || pkd <= TT) {
+                    d += ANY ? (int)pk_re(t, lpd) : 0;
+                    if (ANY && lpd == 0) {
+                        using V2 = std::conditional_t<sizeof(T) == 4, float2, double2>;
+                        static_for<E>([&](auto ic) {
+                            constexpr int i = decltype(ic)::value;
+                            __stcs(reinterpret_cast<V2*>(d + 2 * i * TT), V2{v[i].re * sc, v[i].im * sim});
+                        });
+                    } else {
+                        static_for<E>([&](auto ic) {
+                            constexpr int i = decltype(ic)::value;
+                            T*            o = d + (ANY ? 2 * i * TT : pk<LP>(t + i * TT));
+                            __stcs(o, v[i].re * sc);
+                            __stcs(o + pkd, v[i].im * sim);
+                        });
+                    }
+                } else {
+                    static_for<E>([&](auto ic) {
+                        constexpr int i = decltype(ic)::value;
+                        T*            o = d + pk_re(t + i * TT, lpd);
+                        __stcs(o, v[i].re * sc);
+                        __stcs(o + pkd, v[i].im * sim);
+                    });
+                }
+            }
+            continue;
+        }
+        // other orders (and the smallest sizes): rows staged in the exchange
+        // buffer in output order, then copied out in 16-byte units
+        T* stg = reinterpret_cast<T*>(xch);
+        __syncthreads();    // exchange reads done
         {
-            constexpr int S   = P::NST - 1;
-            constexpr int G   = E / (1 << P::rbits(S));
-            const T       sc  = T(a.scale);
-            const T       sim = a.conj_out ? -sc : sc;
+            constexpr int S = P::NST - 1;
+            constexpr int G = E / (1 << P::rbits(S));
             if (ANY && a.order_out == 0 && pkd <= TT) {
-                // the last stage leaves frequency t + i*TT in v[i]
                 const int o = m * RS + (int)pk_re(t, lpd);
                 static_for<E>([&](auto ic) {
                     constexpr int i = decltype(ic)::value;

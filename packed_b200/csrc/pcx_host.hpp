@@ -210,7 +210,8 @@ cudaError_t pcx_tc_list_launch(int precision, const pcxg::tc_item* items, int ni
                                const void* tw, int tw_lg, int* error, int sms, cudaStream_t st);
 
 // Hot-path launches (pcx_v2_*.cu); cudaErrorNotSupported when no variant exists.
-cudaError_t pcx_v2_single(bool f64, int log_n, const pcxg::v2_args& a, cudaStream_t st, bool attr_only);
+cudaError_t pcx_rows(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, bool attr_only);
+cudaError_t pcx_rows_any(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, bool attr_only);
 cudaError_t pcx_v3_single(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, int sms, bool attr_only);
 // the same kernel for any pack widths and short rows
 cudaError_t pcx_v3_single_any(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, int sms, bool attr_only);

@@ -33,12 +33,23 @@ inline cudaError_t persistent_grid(K kern, int nt, int bytes, long long tiles, i
 }
 
 template<class T, int LOGL, bool ANY>
+cudaError_t launch_rows(const v3_args& a, cudaStream_t st, bool attr_only) {
+    using F   = rows_cfg<T, LOGL>;
+    auto kern = k_rows<T, LOGL, v2cfg<T>::LP, ANY>;
+    if (attr_only) return smem_attr_cached(reinterpret_cast<const void*>(kern), F::SMEM);
+    if (a.batch == 0) return cudaSuccess;
+    kern<<<(unsigned)((a.batch + F::M - 1) / F::M), F::NT, F::SMEM, st>>>(a);
+    return cudaGetLastError();
+}
+
+template<class T, int LOGL, bool ANY>
 cudaError_t launch_single3(const v3_args& a, cudaStream_t st, int sms, bool attr_only) {
-    constexpr int NT    = LOGL >= 13 ? 512 : 256;    // 16 elements per thread
-    constexpr int M     = NT / splan<LOGL>::TT;
-    constexpr int bytes = single3_smem<T, LOGL, NT>();
-    auto          kern  = k_single3<T, LOGL, v2cfg<T>::LP, NT, ANY>;
-    if (attr_only) return set_smem(kern, bytes);
+    using F             = s3_cfg<T, LOGL>;
+    constexpr int NT    = F::NT;
+    constexpr int M     = F::M;
+    constexpr int bytes = F::SMEM;
+    auto          kern  = k_single3<T, LOGL, v2cfg<T>::LP, ANY>;
+    if (attr_only) return smem_attr_cached(reinterpret_cast<const void*>(kern), bytes);
     const long long tiles = (a.batch + M - 1) / M;
     if (tiles == 0) return cudaSuccess;
     unsigned    grid = 0;
