@@ -20,11 +20,12 @@
 //    copies into the ST-stage ring (for a column tile it also tells the
 //    compute warps when the slot may be written);
 //  * the publisher warp walks the same items and publishes each completion as
-//    soon as it happens (col_done once the compute warps wrote a column tile;
-//    row_done once a row tile's scratch rows have landed in shared memory and
-//    their L2 lines are dropped unwritten).  It never waits on another CTA, so
-//    the completions other CTAs wait for are never held up behind this CTA's
-//    own dependency waits.
+//    soon as it happens (col_done once a column tile is written; row_done once
+//    a row tile's scratch rows have landed in shared memory and their L2 lines
+//    are dropped unwritten).  Where outputs are stored by TMA (fs_cfg::TS) it
+//    also issues those copies, a column tile's once its slot may be written
+//    (a wait for earlier items, as every wait is); else it never waits on
+//    another CTA.
 // A stage is refilled after the compute warps are done with it and the
 // publisher has passed its item (empty[s] counts both), so no barrier phase is
 // ever overtaken.  With three stages the exchanges of the sub-transforms run
@@ -174,6 +175,20 @@ struct fs_cfg {
     static constexpr int XB   = smem_align16((X1::size > X2::size ? X1::size : X2::size) * (int)sizeof(cpx<T>));
     static constexpr int ST   = ST_;
     static constexpr bool IP  = ST == 3;
+    // Outputs of both passes staged in the item's stage and stored by TMA.  A
+    // row tile's transposed stores are four 32-byte sectors in four lines per
+    // instruction, 32 instructions a thread, and held the load/store queue
+    // (lg_throttle the first stall at 2^20).  The exchange layout is a TMA box
+    // already: 17 rows of 64 bytes (or of the columns) per 16, the 17th, the
+    // bank padding, outside the tensor view and so not written; each thread
+    // puts its outputs over values that it (row tiles: a lane beside it) read
+    // last, without a block barrier, and the publisher issues one to eight
+    // copies a tile.  The stage is held until its copy has read it, which costs
+    // the short tiles more than it saves.  GB/s at 512 MB, from registers and
+    // staged: FP32 2^14 3405 3261, 2^15 3459 3249, 2^16 3313 3015, 2^17 2947
+    // 3043, 2^18 2867 2950, 2^19 2523 2818, 2^20 2541 2830; FP64 2^14 3429 3502,
+    // 2^15 3372 3399, 2^16 3351 3508, 2^17 2691 3254, 2^18 2429 2928.
+    static constexpr bool TS  = IP && (sizeof(T) == 8 || LOGN1 >= 9 || LOGN2 >= 9);
     static_assert(ST == 2 || ST == 3, "two or three ring stages");
     static constexpr int TILEB = COLB > ROWB ? COLB : ROWB;
     static constexpr int STAGE = ((IP ? (TILEB > XB ? TILEB : XB) : TILEB) + 127) / 128 * 128;
@@ -269,7 +284,8 @@ __device__ __forceinline__ fs_item fs_decode(uint32_t j, uint32_t batch, uint32_
 
 template<class T, int LOGN1, int LOGN2, int MINB, int ST_, int FORM = FS_PLAIN>
 __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, MINB)
-    k_fourstep(const __grid_constant__ CUtensorMap tmap, fs_args a) {
+    k_fourstep(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tscr,
+               const __grid_constant__ CUtensorMap tdst, fs_args a) {
     using F            = fs_cfg<T, LOGN1, LOGN2, MINB, ST_>;
     using P1           = typename F::P1;
     using P2           = typename F::P2;
@@ -291,6 +307,8 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
     constexpr int RSI  = F::RSI;
     constexpr int RROW = N2 * (int)sizeof(cpx<T>);
     constexpr bool SH  = F::SH;
+    constexpr bool TS  = F::TS;                      // outputs staged in the item's stage and stored by TMA
+    constexpr bool TSR = TS && FORM != FS_OUT;       // row tiles too (FS_OUT stores whole rows itself)
     static_assert(FORM != FS_IN || C * F::RSC * (int)sizeof(T) <= F::STAGE, "a column tile of whole rows fits a stage");
     static_assert(FORM != FS_OUT || CR * 2 * N2 * (int)sizeof(T) <= (IP ? F::STAGE : F::XB), "a staged row tile fits");
     extern __shared__ __align__(128) unsigned char smem[];
@@ -301,9 +319,9 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
     const void*         gtab1 = F::ONE && LOGN2 > LOGN1 ? a.stw2 : a.stw1;
     const void*         gtab2 = F::ONE && LOGN1 > LOGN2 ? a.stw1 : a.stw2;
     __shared__ uint64_t full[ST];      // TMA bytes landed
-    __shared__ uint64_t empty[ST];     // compute warps done with the stage, publisher past its item
-    __shared__ uint64_t slotok[ST];    // column tile: its scratch slot may be written
-    __shared__ uint64_t written[ST];   // column tile: compute warps wrote the slot
+    __shared__ uint64_t empty[ST];     // the stage may be refilled
+    __shared__ uint64_t slotok[ST];    // !TS, column tile: its scratch slot may be written
+    __shared__ uint64_t written[ST];   // TS: outputs staged (FS_OUT rows: stored); !TS: column tile written
     cpx<T>*             scr   = reinterpret_cast<cpx<T>*>(a.scratch);
     const int           tid   = threadIdx.x;
     const uint32_t      items = (uint32_t)a.batch * (uint32_t)(TC + TR);    // < 2^31 (host check)
@@ -319,7 +337,7 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
     if (tid == 0) {
         for (int s = 0; s < ST; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], NW + 1);
+            mbar_init(&empty[s], TS ? 1 : NW + 1);
             mbar_init(&slotok[s], 1);
             mbar_init(&written[s], NW);
         }
@@ -330,24 +348,15 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
     if (tid >= NT + 32) {
         // ======================= publisher warp
         const int lane    = tid - NT - 32;
-        uint32_t  colpar  = 0;    // bit s: parity of the next `written` wait on stage s
+        const uint64_t pol = l2_evict_first_policy();    // outputs are written once
+        uint32_t  colpar  = 0;    // !TS, bit s: parity of the next `written` wait on stage s
         bool      fail    = false;
         int       s       = 0;
         uint32_t  par     = 0;
         for (uint32_t j = blockIdx.x; j < items && !fail; j += G, s = s + 1 == ST ? 0 : s + 1, par ^= s == 0) {
             const fs_item  it  = fs_decode<TC, TR>(j, batch, lag);
             int            ok  = 1;
-            if (!it.row) {
-                // the compute warps' stores of the tile are done: make them
-                // visible to other CTAs' TMA reads, then count the tile
-                if (lane == 0) ok = mbar_wait_bounded(&written[s], (colpar >> s) & 1u) ? 1 : 0;
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                colpar ^= 1u << s;
-                if (ok && lane == 0) {
-                    fence_proxy_async_global();
-                    red_release_add(a.col_done + it.r, 1);
-                }
-            } else {
+            if (it.row) {
                 // the tile's scratch rows are in shared memory: drop their L2
                 // lines unwritten and count the tile
                 if (lane == 0) ok = mbar_wait_bounded(&full[s], par) ? 1 : 0;
@@ -360,6 +369,45 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
                     if (lane == 0) red_release_add(a.row_done + it.r, 1);
                 }
             }
+            if constexpr (TS) {
+                // the compute warps' staged outputs leave by TMA: a column
+                // tile to its scratch slot once that may be written (counted
+                // when the copy is complete), a row tile to the destination
+                if (lane == 0 && ok) {
+                    ok = mbar_wait_bounded(&written[s], par) ? 1 : 0;
+                    const unsigned char* buf = ring + s * F::STAGE;
+                    if (ok && !it.row) {
+                        ok = it.r < a.nslot || fs_wait(a.row_done + (it.r - a.nslot), TR);
+                        if (ok) {
+                            fence_proxy_async_global();
+                            tma_store_4d(&tscr, buf, 2 * it.tile * C, 0, 0, (int)(it.r & mask));
+                            bulk_commit();
+                            bulk_wait();
+                            fence_proxy_async_global();
+                            red_release_add(a.col_done + it.r, 1);
+                        }
+                    } else if (ok && TSR) {
+#pragma unroll
+                        for (int h = 0; h < CR / G8; ++h) {
+                            tma_store_4d_hint(&tdst, buf + h * F::X2::LP * G8 * (int)sizeof(cpx<T>),
+                                              2 * (it.tile * CR + h * G8), 0, 0, it.r, pol);
+                        }
+                        bulk_commit();
+                        bulk_wait_read();
+                    }
+                }
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+            } else if (!it.row) {
+                // the compute warps' stores of the tile are done: make them
+                // visible to other CTAs' TMA reads, then count the tile
+                if (lane == 0) ok = mbar_wait_bounded(&written[s], (colpar >> s) & 1u) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                colpar ^= 1u << s;
+                if (ok && lane == 0) {
+                    fence_proxy_async_global();
+                    red_release_add(a.col_done + it.r, 1);
+                }
+            }
             if (!ok) {
                 fail = true;
                 if (lane == 0) atomicExch(a.error, 1);
@@ -367,6 +415,7 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
                 mbar_arrive(&empty[s]);
             }
         }
+        if (TS && lane == 0) bulk_wait();    // nothing is in flight when the block exits
         __syncwarp();
         return;
     }
@@ -416,14 +465,16 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
                     }
                 }
                 issued = k + 1;
-                // the acquire of the slot's counter (or a first use of the
-                // slot) orders the compute warps' writes after the earlier
-                // row tiles' reads, through this arrive and their wait
-                if (!(it.r < a.nslot || need(a.row_done + (it.r - a.nslot), TR))) {
-                    fail = true;
-                    break;
+                if constexpr (!TS) {
+                    // the acquire of the slot's counter (or a first use of the
+                    // slot) orders the compute warps' writes after the earlier
+                    // row tiles' reads, through this arrive and their wait
+                    if (!(it.r < a.nslot || need(a.row_done + (it.r - a.nslot), TR))) {
+                        fail = true;
+                        break;
+                    }
+                    if (lane == 0) mbar_arrive(&slotok[s]);
                 }
-                if (lane == 0) mbar_arrive(&slotok[s]);
             } else {
                 if (!need(a.col_done + it.r, TC)) {
                     fail = true;
@@ -475,6 +526,12 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);
+        };
+        // TS: this warp's part of the staged outputs is in place
+        auto staged = [&]() {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0 && !bad) mbar_arrive(&written[s]);
         };
         // column tile: the four-step twiddle inputs are requested before the
         // tile's data is waited for, and used after the stages
@@ -548,24 +605,33 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
             if constexpr (!IP) release_stage();
             stage_compute_tab<P1, 0>(v, t, stw1);
             if (run_stages_full<P1, typename F::X1, SH, NT, typename F::PT1>(v, xch, c, t, stw1, bad)) return;
-            if constexpr (IP) release_stage();
-            if (!mbar_wait_bounded(&slotok[s], (colpar >> s) & 1u)) {
-                // the producer gave up on this slot: nothing is written, and
-                // the compute warps leave at the next item's vote
-                bad = true;
-                atomicExch(a.error, 1);
-            }
-            colpar ^= 1u << s;
-            if (!bad) {
-                cpx<T>* dst = scr + (it.r & mask) * (long long)(N1 * N2) + (long long)t * N2 + n2;
-                auto    put = [&](auto ic, cpx<T> o) {
-                    constexpr int i             = decltype(ic)::value;
-                    dst[(long long)i * TT * N2] = o;
-                };
+            if constexpr (IP && !TS) release_stage();
+            if constexpr (TS) {
+                // each output over the value this thread read last: the
+                // exchange layout is the box the publisher stores
+                auto put = [&](auto ic, cpx<T> o) { xch[F::X1::idx(c, t + decltype(ic)::value * TT)] = o; };
                 if constexpr (FORM == FS_PLAIN) apply_fourstep_tw(v, cmul(th, tl), tu[0], put);
                 else apply_fourstep_tw5(v, th, tu, put);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&written[s]);
+                staged();
+            } else {
+                if (!mbar_wait_bounded(&slotok[s], (colpar >> s) & 1u)) {
+                    // the producer gave up on this slot: nothing is written, and
+                    // the compute warps leave at the next item's vote
+                    bad = true;
+                    atomicExch(a.error, 1);
+                }
+                colpar ^= 1u << s;
+                if (!bad) {
+                    cpx<T>* dst = scr + (it.r & mask) * (long long)(N1 * N2) + (long long)t * N2 + n2;
+                    auto    put = [&](auto ic, cpx<T> o) {
+                        constexpr int i             = decltype(ic)::value;
+                        dst[(long long)i * TT * N2] = o;
+                    };
+                    if constexpr (FORM == FS_PLAIN) apply_fourstep_tw(v, cmul(th, tl), tu[0], put);
+                    else apply_fourstep_tw5(v, th, tu, put);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&written[s]);
+                }
             }
         } else {
             // ---------------- row tile: N2-point DFTs along CR rows
@@ -624,7 +690,23 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
                     __stcs(reinterpret_cast<float4*>(dst + (long long)k * 2 * N2 + u * W),
                            *reinterpret_cast<const float4*>(&w));
                 }
-                if constexpr (IP) release_stage();
+                // the stage is read: it may be refilled
+                if constexpr (TS) staged();
+                else if constexpr (IP) release_stage();
+            } else if constexpr (TS) {
+                // row k2 of the exchange layout is 8 (FP64: 4) elements of the
+                // transposed output, one segment of 64 bytes, last read by
+                // neighbouring lanes of this warp: they put their values there
+                // in packed order, the box the publisher stores
+                const int lpd = FORM == FS_PLAIN ? LP : a.lp_dst;
+                T*        seg = reinterpret_cast<T*>(xch + F::X2::idx(m - mlo, 0)) + (int)pk_re(mlo, lpd);
+                __syncwarp();
+                static_for<E>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    const int     l = t + i * TT;
+                    sts_swapped<T, SW>(seg, (l + (l >> 4)) * 2 * G8, 1 << lpd, v[i].re * sc, v[i].im * sim);
+                });
+                staged();
             } else if constexpr (FORM != FS_PLAIN) {
                 if constexpr (IP) release_stage();
                 T* dst = reinterpret_cast<T*>(a.dst) + it.r * a.dst_stride + pk_re(t * N1 + k1, a.lp_dst);

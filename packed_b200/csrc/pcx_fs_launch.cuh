@@ -39,10 +39,27 @@ cudaError_t launch_fs(const fs_args& a, cudaStream_t st, int sms, bool attr_only
     const cuuint32_t estr[3]    = {1, 1, 1};
     cudaError_t      e = encode_tensor_map(&map, sizeof(T) == 8, 3, const_cast<void*>(a.src), dims, strides, box, estr);
     if (e != cudaSuccess) return FORM == FS_PLAIN ? e : cudaErrorNotSupported;    // the caller has another path
+    // 4-D views that the outputs are stored through, [.][16-row block][row of it][reals]: the scratch
+    // (rows k1 of slot .) and the destination (rows k2 of transform .).  Boxes are 17 rows high: the
+    // 17th, outside the view, is the padding row of the shared layout and is not written.
+    CUtensorMap      tscr, tdst;
+    const cuuint32_t estr4[4]    = {1, 1, 1, 1};
+    const cuuint64_t sdims[4]    = {(cuuint64_t)2 << LOGN2, 16, (cuuint64_t)F::N1 / 16, (cuuint64_t)a.nslot};
+    const cuuint64_t sstr[3]     = {((cuuint64_t)2 << LOGN2) * sizeof(T), ((cuuint64_t)32 << LOGN2) * sizeof(T),
+                                    ((cuuint64_t)2 << (LOGN1 + LOGN2)) * sizeof(T)};
+    const cuuint32_t sbox[4]     = {(cuuint32_t)(2 * F::C), 17, (cuuint32_t)F::N1 / 16, 1};
+    const long long  ds          = a.batch > 1 ? a.dst_stride : (2LL << (LOGN1 + LOGN2));
+    const cuuint64_t ddims[4]    = {(cuuint64_t)2 << LOGN1, 16, (cuuint64_t)F::N2 / 16, (cuuint64_t)a.batch};
+    const cuuint64_t dstr[3]     = {((cuuint64_t)2 << LOGN1) * sizeof(T), ((cuuint64_t)32 << LOGN1) * sizeof(T),
+                                    (cuuint64_t)ds * sizeof(T)};
+    const cuuint32_t dbox[4]     = {(cuuint32_t)(2 * F::G8), 17, (cuuint32_t)F::N2 / 16, 1};
+    e = encode_tensor_map(&tscr, sizeof(T) == 8, 4, a.scratch, sdims, sstr, sbox, estr4);
+    if (e == cudaSuccess) e = encode_tensor_map(&tdst, sizeof(T) == 8, 4, a.dst, ddims, dstr, dbox, estr4);
+    if (e != cudaSuccess) return FORM == FS_PLAIN ? e : cudaErrorNotSupported;
     unsigned grid = 0;
     e             = persistent_grid(kern, F::NT + 64, F::SMEM, items, sms, &grid);
     if (e != cudaSuccess) return e;
-    kern<<<grid, F::NT + 64, F::SMEM, st>>>(map, a);
+    kern<<<grid, F::NT + 64, F::SMEM, st>>>(map, tscr, tdst, a);
     return cudaGetLastError();
 }
 
@@ -69,15 +86,15 @@ cudaError_t launch_fs(const fs_args& a, cudaStream_t st, int sms, bool attr_only
         PCX_FS_FORM_VARIANT(float, 7, 8, 2, 3)                                                                \
         PCX_FS_FORM_VARIANT(float, 8, 8, 2, 3)                                                                \
         PCX_FS_FORM_VARIANT(float, 8, 9, 2, 3)                                                                \
-        PCX_FS_FORM_VARIANT(float, 8, 10, 1, 3)                                                               \
-        PCX_FS_FORM_VARIANT(float, 9, 10, 1, 3)                                                               \
+        PCX_FS_FORM_VARIANT(float, 9, 9, 2, 3)                                                                \
+        PCX_FS_FORM_VARIANT(float, 10, 9, 1, 3)                                                               \
         PCX_FS_FORM_VARIANT(float, 10, 10, 1, 3)                                                              \
         PCX_FS_FORM_VARIANT(double, 7, 7, 2, 3)                                                               \
         PCX_FS_FORM_VARIANT(double, 8, 7, 2, 3)                                                               \
         PCX_FS_FORM_VARIANT(double, 8, 8, 2, 3)                                                               \
         PCX_FS_FORM_VARIANT(double, 9, 8, 2, 3)                                                               \
         PCX_FS_FORM_VARIANT(double, 9, 9, 2, 3)                                                               \
-        PCX_FS_FORM_VARIANT(double, 10, 9, 1, 2)                                                              \
+        PCX_FS_FORM_VARIANT(double, 10, 9, 1, 3)                                                              \
         PCX_FS_FORM_VARIANT(double, 10, 10, 1, 2)                                                             \
         return cudaErrorNotSupported;                                                                         \
     }

@@ -78,20 +78,22 @@ struct fs_choice {
 };
 // The variants built into the library (FP32 and FP64), in the order the
 // autotuner tries them; the first one of a size is its untuned default (the
-// fastest one measured on a B200 on 512 MB batches; at 2^15 and 2^17..2^19 an
-// uneven split with the longer sub-transform in the row pass is fastest).
+// fastest one measured on a B200 on 512 MB batches: GB/s at 2^18 2950 for
+// 512 x 512 and 2860 for 256 x 1024, at 2^19 2818 for 1024 x 512 and 2769 for
+// 512 x 1024; at 2^15 and 2^17 the longer sub-transform goes in the row pass).
 constexpr fs_variant kFsVariantsF32[] = {
     {7, 6, 2, 3},  {6, 7, 2, 3},                                      // 2^13 (beside the one-pass form)
     {7, 7, 2, 3},  {7, 7, 1, 3},  {6, 8, 2, 3},                       // 2^14
     {7, 8, 2, 3},  {8, 7, 2, 3},  {6, 9, 2, 3},                       // 2^15
     {8, 8, 2, 3},  {8, 8, 1, 3},  {7, 9, 2, 3},  {9, 7, 2, 3},  {6, 10, 1, 3},    // 2^16
     {8, 9, 2, 3},  {9, 8, 2, 3},  {10, 7, 1, 3}, {9, 8, 1, 3},  {7, 10, 1, 3},    // 2^17
-    {8, 10, 1, 3}, {10, 8, 1, 3}, {9, 9, 1, 3},  {9, 9, 2, 3},        // 2^18
-    {9, 10, 1, 3}, {9, 10, 1, 2}, {10, 9, 1, 2}, {10, 9, 1, 3},       // 2^19
+    {9, 9, 2, 3},  {8, 10, 1, 3}, {10, 8, 1, 3}, {9, 9, 1, 3},        // 2^18
+    {10, 9, 1, 3}, {9, 10, 1, 3}, {9, 10, 1, 2}, {10, 9, 1, 2},       // 2^19
     {10, 10, 1, 3}, {10, 10, 1, 2},                                   // 2^20
 };
 constexpr fs_variant kFsVariantsF64[] = {
-    {7, 7, 2, 3}, {8, 7, 2, 3}, {8, 8, 2, 3}, {9, 8, 2, 3}, {9, 9, 2, 3}, {10, 9, 1, 2}, {10, 10, 1, 2},
+    {7, 7, 2, 3}, {8, 7, 2, 3}, {8, 8, 2, 3}, {9, 8, 2, 3}, {9, 9, 2, 3}, {10, 9, 1, 3}, {10, 9, 1, 2},
+    {10, 10, 1, 2},
 };
 }
 

@@ -89,4 +89,25 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
         : "memory");
 }
 
+// 4-D tensor copy shared -> global (elements of the box outside the tensor are
+// not written); counted in this thread's bulk groups.
+__device__ __forceinline__ void tma_store_4d(const void* tmap, const void* src, int x, int y, int z, int w) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(tmap),
+                 "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(src))
+                 : "memory");
+}
+// The same with an L2 eviction-priority policy.
+__device__ __forceinline__ void tma_store_4d_hint(const void* tmap, const void* src, int x, int y, int z, int w,
+                                                  uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group.L2::cache_hint [%0, {%1, %2, %3, %4}], [%5], %6;" ::"l"(
+            tmap),
+        "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(src)), "l"(policy)
+        : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// All of this thread's bulk groups have read their shared memory / are complete.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 }    // namespace pcxg

@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 
 F32, F64 = torch.float32, torch.float64
 # log2 of the row length N2 of each size's default split
-ROW = {13: 6, 14: 7, 15: 8, 16: 8, 17: 9, 18: 10, 19: 10, 20: 10}
+ROW = {13: 6, 14: 7, 15: 8, 16: 8, 17: 9, 18: 9, 19: 9, 20: 10}
 SIZES = [(F32, lg) for lg in range(13, 21)] + [(F64, lg) for lg in (14, 15, 16, 17, 18, 19, 20)]
 
 
