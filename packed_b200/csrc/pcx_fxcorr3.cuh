@@ -172,12 +172,13 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
     }
     __syncthreads();
 
+    bool bad = false;    // this warp gave up a wait
     for (int k = 0;; ++k) {
         const int       s    = k & 1;
         const long long tile = s_tile[s];
         if (tile >= ntile) break;    // claims only grow: nothing is in flight
         const bool ok = mbar_wait_bounded(&full[s], (uint32_t)((k >> 1) & 1));
-        if (__syncthreads_or(!ok)) {
+        if (__syncthreads_or(!ok || bad)) {
             // give up: record it, let the copies in flight land, leave together
             if (tid == 0) {
                 atomicExch(a.error, 1);
@@ -187,7 +188,6 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
             break;
         }
         if (a.inplace && tid == 0) {
-            __threadfence();
             st_release(a.flags + tile, a.epoch);    // this tile's windows are loaded
         }
         const xc3_window x  = win[s][m];
@@ -218,15 +218,19 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
         });
         // in place: the first look at the flags, so that the wait below rarely
         // has to read one
-        bool seen = true;
-        if (a.inplace && tid < htile && tid < tile) seen = ld_acquire(a.flags + (tile - 1 - tid)) == a.epoch;
+        const int lane = tid % 32;
+        bool      seen = true;
+        if (a.inplace && lane < htile && lane < tile) seen = ld_acquire(a.flags + (tile - 1 - lane)) == a.epoch;
         stage_compute_tab<P, 0>(v, t, stw);
         run_stages_tab<P, X, true, BAR>(v, xch, m, t, stw);
         if (a.inplace) {
+            // every warp waits for itself, so that no barrier holds the outputs
+            // of those that are done; one that gives up stores nothing, and the
+            // block leaves at the next tile's vote
             bool late = false;
-            for (long long d = tid; d < htile && d < tile && !late; d += NT) {
+            for (long long d = lane; d < htile && d < tile && !late; d += 32) {
                 const unsigned* f = a.flags + (tile - 1 - d);
-                if ((d == tid && seen) || ld_acquire(f) == a.epoch) continue;
+                if ((d == lane && seen) || ld_acquire(f) == a.epoch) continue;
                 const unsigned long long t0 = globaltimer_ns();
                 while (ld_acquire(f) != a.epoch) {
                     if (globaltimer_ns() - t0 > XC_WAIT_NS) {
@@ -236,13 +240,10 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
                     __nanosleep(128);
                 }
             }
-            if (__syncthreads_or(late)) {
-                if (tid == 0) {
-                    atomicExch(a.error, 1);
-                    if (s_tile[s ^ 1] < ntile) mbar_wait_bounded(&full[s ^ 1], (uint32_t)(((k + 1) >> 1) & 1), 100000000ull);
-                    if (s_tile[s] < ntile) mbar_wait_bounded(&full[s], (uint32_t)(((k + 2) >> 1) & 1), 100000000ull);
-                }
-                break;
+            if (__any_sync(0xffffffffu, late)) {
+                if (lane == 0) atomicExch(a.error, 1);
+                bad = true;
+                continue;
             }
         }
         // v[i] = conj of circular output t + i*TT, output t + i*TT - out_shift of the block
