@@ -2,6 +2,7 @@
 // computed on the device), the fused correlation launch and its adjoint.
 #include "pcx_fxcorr2d.cuh"
 #include "pcx_fxcorr3.cuh"
+#include "pcx_fxcorr_ip.cuh"
 #include "pcx_fxcorr_kernels.cuh"
 #include "pcx_host.hpp"
 #include "pcx_v2_launch.cuh"
@@ -31,9 +32,10 @@ struct pcx_fxcorr_s {
     int         sms            = 0;
     int         device         = 0;
     bool        x3             = false;      // FP32, N <= 2^12: pcx_fxcorr3.cuh (tables: plan->stwL)
-    // FP32, N = 2^13 or 2^14: in-CTA four-step form (pcx_fxcorr2d.cuh)
-    void*       x2d            = nullptr;    // one allocation: K permuted | stage tables | twiddles
-    const void* x2_kperm       = nullptr;
+    // FP32, N = 2^13 or 2^14: three-step form (pcx_fxcorr_ip.cuh), kernel
+    // gradient in the in-CTA four-step form (pcx_fxcorr2d.cuh)
+    void*       x2d            = nullptr;    // one allocation: K permuted | twiddles | stage tables | twiddles
+    const void* xi_tw          = nullptr;
     const void* x2_stw1        = nullptr;
     const void* x2_stw2        = nullptr;
     const void* x2_tws         = nullptr;
@@ -159,15 +161,13 @@ cudaError_t pcx_xc2_perm_spectrum(const void* ks, void* kp, int log_n1, int log_
 namespace {
 
 template<int LOGN>
-int launch_xc2(const xc2_args& a, cudaStream_t st, int sms, bool attr_only) {
-    using C   = xc2_cfg<LOGN>;
-    auto kern = k_fxcorr2d<LOGN>;
-    if (attr_only) {
-        PCX_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-        return PCX_OK;
-    }
+int launch_xci(const xci_args& a, cudaStream_t st, int sms, bool attr_only) {
+    using C    = xci_cfg<LOGN>;
+    auto kern  = k_fxcorr_ip<LOGN>;
     int per_sm = 0;
+    PCX_CUDA_TRY(smem_attr_cached(reinterpret_cast<const void*>(kern), C::SMEM));
     PCX_CUDA_TRY(occupancy_cached(reinterpret_cast<const void*>(kern), C::NT, C::SMEM, &per_sm));
+    if (attr_only) return PCX_OK;
     const long long grid = std::max<long long>(1, std::min<long long>(a.base.total, (long long)std::max(per_sm, 1) * sms));
     kern<<<(unsigned)grid, C::NT, C::SMEM, st>>>(a);
     PCX_CUDA_TRY(cudaGetLastError());
@@ -252,11 +252,13 @@ int init_xc2(pcx_fxcorr_s* h) {
     e1                  = (e1 + 1) / 2 * 2;    // 16-byte sections
     e2                  = (e2 + 1) / 2 * 2;
     const size_t ntw    = (size_t)C::NB + C::N2 + C::N1;
-    const size_t entries = (size_t)C::N + e1 + e2 + ntw;
+    const size_t entries = (size_t)C::N + xci_cfg<LOGN>::TABLE + e1 + e2 + ntw;
     PCX_CUDA_TRY(cudaMalloc(&h->x2d, entries * sizeof(cpx<float>)));
     auto* base   = static_cast<cpx<float>*>(h->x2d);
-    auto* kp     = base;
-    auto* s1     = kp + C::N;
+    auto* xt     = base + C::N;
+    auto* s1     = xt + xci_cfg<LOGN>::TABLE;
+    k_xci_twiddles<<<(xci_cfg<LOGN>::TABLE + 255) / 256, 256>>>(xt, LOGN);
+    PCX_CUDA_TRY(cudaGetLastError());
     auto* s2     = s1 + e1;
     auto* tws    = s2 + e2;
     PCX_CUDA_TRY(pcx_fourstep_tables(C::LOGN1, s1, false, 0, &e1));
@@ -264,12 +266,12 @@ int init_xc2(pcx_fxcorr_s* h) {
     PCX_CUDA_TRY(pcx_gen_twiddles(tws, C::NB, LOGN, 1, false, 0));
     PCX_CUDA_TRY(pcx_gen_twiddles(tws + C::NB, C::N2, LOGN, C::TT1, false, 0));
     PCX_CUDA_TRY(pcx_gen_twiddles(tws + C::NB + C::N2, C::N1, LOGN, C::TT2, false, 0));
-    h->x2_kperm = kp;
+    h->xi_tw    = xt;
     h->x2_stw1  = s1;
     h->x2_stw2  = s2;
     h->x2_tws   = tws;
     if (int rc = launch_xc2_kg<LOGN>(xc2_kg_args{}, 0, 0, true)) return rc;
-    return launch_xc2<LOGN>(xc2_args{}, 0, 0, true);
+    return launch_xci<LOGN>(xci_args{}, 0, 0, true);
 }
 
 int check_pack(int pack) {
@@ -343,7 +345,7 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     a.counter     = h->ctl;
     a.error       = reinterpret_cast<int*>(h->ctl + 1);
     a.kspec       = h->kspec;
-    // whole-window and in-CTA four-step forms: FP32, pack 8, windows on whole
+    // whole-window and three-step forms: FP32, pack 8, windows on whole
     // packs, rows of packs 16-byte aligned
     const bool rows = pack == 8 && a.in_shift % 8 == 0 && (channels == 1 || sstride % 4 == 0) &&
                       reinterpret_cast<uintptr_t>(src) % 16 == 0;
@@ -351,13 +353,11 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     if (h->x3 && rows) return dispatch_xc3(h->log_n, a, h->plan->stwL, st, h->sms);
     const bool x2 = h->x2d && rows;
     if (x2) {
-        xc2_args b{};
+        xci_args b{};
         b.base  = a;
-        b.kperm = h->x2_kperm;
-        b.stw1  = h->x2_stw1;
-        b.stw2  = h->x2_stw2;
-        b.tws   = h->x2_tws;
-        return h->log_n == 14 ? launch_xc2<14>(b, st, h->sms, false) : launch_xc2<13>(b, st, h->sms, false);
+        b.kperm = h->x2d;
+        b.tw    = h->xi_tw;
+        return h->log_n == 14 ? launch_xci<14>(b, st, h->sms, false) : launch_xci<13>(b, st, h->sms, false);
     }
     return h->dtype == PCX_F64 ? dispatch_xc<double>(h->log_n, a, h->tw, st, h->sms, false)
                                : dispatch_xc<float>(h->log_n, a, h->tw, st, h->sms, false);
@@ -461,15 +461,16 @@ void note_call(pcx_fxcorr_s* h, cudaStream_t st) {
 }
 
 // K = FFT(g zero-padded to N) / N, natural order, interleaved (fxcorr.hpp:62-69),
-// and its reordered copy for the in-CTA four-step form.
+// and its reordered copy for the three-step form.
 int set_kernel(pcx_fxcorr_s* h, const void* g) {
     if (int rc = pcx_fft_run(h->plan, h->kspec, g, h->k, 1, h->pack_g, PCX_FORWARD, 0, 1, 2 * h->n,
                              (h->k + h->pack_g - 1) / h->pack_g * 2 * h->pack_g, nullptr, 0, 0, 1.0 / (double)h->n)) {
         return rc;
     }
     if (h->x2d) {
-        const int l1 = (h->log_n + 1) / 2, l2 = h->log_n / 2;
-        PCX_CUDA_TRY(pcx_xc2_perm_spectrum(h->kspec, h->x2d, l1, l2, 0));
+        k_xci_spectrum<<<(unsigned)(h->n / 256), 256>>>(static_cast<const cpx<float>*>(h->kspec),
+                                                       static_cast<cpx<float>*>(h->x2d), h->log_n);
+        PCX_CUDA_TRY(cudaGetLastError());
     }
     return PCX_OK;
 }

@@ -71,322 +71,6 @@ struct xc2_cfg {
     static_assert(WIN % 16 == 0 && XB % 16 == 0 && TB1 % 16 == 0 && TB2 % 16 == 0, "16-byte sections");
 };
 
-struct xc2_args {
-    xc_args     base;
-    const void* kperm;    // K[k1 + N1*k2] / N at [k1*N2 + k2]
-    const void* stw1;     // stage tables of the N1- and N2-point FFTs
-    const void* stw2;
-    const void* tws;      // W_N^e (e < N/16), W_N^(TT1*n2) (n2 < N2), W_N^(TT2*k1) (k1 < N1)
-};
-
-template<int LOGN>
-__global__ void __launch_bounds__(512, 1) k_fxcorr2d(xc2_args A) {
-    using F            = xc2_cfg<LOGN>;
-    using P1           = typename F::P1;
-    using P2           = typename F::P2;
-    constexpr int N1   = F::N1;
-    constexpr int N2   = F::N2;
-    constexpr int NT   = F::NT;
-    constexpr int TT1  = F::TT1;
-    constexpr int TT2  = F::TT2;
-    constexpr int RS   = F::RS;
-    constexpr int E    = 16;
-    const xc_args& a   = A.base;
-    extern __shared__ __align__(128) unsigned char smem[];
-    cpx<float>*          win  = reinterpret_cast<cpx<float>*>(smem);
-    cpx<float>*          xch  = reinterpret_cast<cpx<float>*>(smem + F::WIN);
-    cpx<float>*          tw1  = reinterpret_cast<cpx<float>*>(smem + F::WIN + F::XB);
-    cpx<float>*          tw2  = tw1 + F::TB1 / 8;
-    cpx<float>*          fwb  = tw2 + F::TB2 / 8;    // W_N^e
-    cpx<float>*          fwu1 = fwb + F::NBP;        // W_N^(TT1*n2)
-    cpx<float>*          fwu2 = fwu1 + N2;           // W_N^(TT2*k1)
-    __shared__ uint64_t  full;
-    __shared__ long long s_item;
-    __shared__ int       s_rlo;
-    __shared__ int       s_rhi;
-    __shared__ int       s_abort;
-    __shared__ uint32_t  s_tmem;
-    const int            tid  = threadIdx.x;
-    const float*         src  = reinterpret_cast<const float*>(a.src);
-    float*               dst  = reinterpret_cast<float*>(a.dst);
-    const cpx<float>*    kp   = reinterpret_cast<const cpx<float>*>(A.kperm);
-
-    // constant tables into shared memory
-    copy_table_to_smem<F::TB1>(tw1, A.stw1, tid, NT);
-    copy_table_to_smem<F::TB2>(tw2, A.stw2, tid, NT);
-    const cpx<float>* tws = reinterpret_cast<const cpx<float>*>(A.tws);
-    for (int e = tid; e < F::NB; e += NT) fwb[e + (e >> 4)] = ldg_cpx(tws + e);
-    for (int i = tid; i < (N2 + N1) / 2; i += NT) {
-        reinterpret_cast<uint4*>(fwu1)[i] = __ldg(reinterpret_cast<const uint4*>(tws + F::NB) + i);
-    }
-    if (tid == 0) {
-        mbar_init(&full, 1);
-        fence_barrier_init();
-    }
-    // step 2's row groups: the U groups of a half-warp take rows S apart, so
-    // their window rows fall in disjoint banks (RS = 2 mod 16)
-    constexpr int S2 = TT2 / 2;
-    constexpr int U2 = 16 / TT2;
-    const int     g2 = tid / TT2, t2 = tid % TT2;
-    const int     r2 = ((g2 / U2) / S2) * 8 + ((g2 / U2) % S2) + (g2 % U2) * S2;
-    // The kernel spectrum values a thread multiplies by are the same for every
-    // block (its rows k1 = rd*G2 + r2, columns k2 = t2 + i*TT2): they are read
-    // once into the thread's tensor-memory lane (otherwise idle in this kernel),
-    // 32 columns per row round, instead of from global memory in every block.
-    constexpr uint32_t TCOLS = 128 * F::R2;    // four warps share each lane quarter
-    static_assert(TCOLS == 128 || TCOLS == 256, "a power-of-two TMEM allocation");
-    if (tid < 32) {
-        tmem_alloc(&s_tmem, TCOLS);
-        tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tbase = s_tmem;
-    const uint32_t tcol  = tbase + ((uint32_t)(32 * ((tid / 32) % 4)) << 16) + (uint32_t)((tid / 128) * 32 * F::R2);
-    for (int rd = 0; rd < F::R2; ++rd) {
-        const int k1 = rd * F::G2 + r2;
-        uint32_t  kr[32];
-        static_for<E>([&](auto ic) {
-            constexpr int    i = decltype(ic)::value;
-            const cpx<float> k = ldg_cpx(kp + k1 * N2 + t2 + i * TT2);
-            kr[2 * i]          = __float_as_uint(k.re);
-            kr[2 * i + 1]      = __float_as_uint(k.im);
-        });
-        tmem_st32(tcol + 32 * rd, kr);
-    }
-
-    // channel and window start (samples) of an item
-    auto item_pos = [&](long long item, long long& ch, long long& b0) {
-        ch = item / a.nblk;
-        b0 = (item - ch * a.nblk) * a.step - a.in_shift;
-    };
-    // warp 0: thread 0 claims the next item; the warp's lanes start the
-    // copies of its rows that lie inside [0, len), a row each in turn; the
-    // threads fill the others
-    auto claim_and_copy = [&]() {
-        if (tid == 0) {
-            const long long item = (long long)atomicAdd(a.counter, 1u);
-            s_item               = item;
-            if (item < a.total) {
-                long long ch, b0;
-                item_pos(item, ch, b0);
-                long long r_lo = b0 >= 0 ? 0 : (-b0 + N2 - 1) / N2;
-                long long r_hi = b0 + (long long)N1 * N2 <= a.len ? N1 : (a.len - b0) / N2;
-                r_lo           = r_lo > N1 ? N1 : r_lo;
-                r_hi           = r_hi < r_lo ? r_lo : (r_hi > N1 ? N1 : r_hi);
-                s_rlo          = (int)r_lo;
-                s_rhi          = (int)r_hi;
-                mbar_arrive_expect_tx(&full, (uint32_t)(r_hi - r_lo) * (N2 * 8));
-            }
-        }
-        __syncwarp();
-        const long long item = s_item;
-        if (item >= a.total) return;
-        long long ch, b0;
-        item_pos(item, ch, b0);
-        const float* base = src + ch * a.src_stride + 2 * b0;    // packed: 2 reals per sample
-        for (int r = s_rlo + tid; r < s_rhi; r += 32) bulk_g2s(win + r * RS, base + 2LL * r * N2, N2 * 8, &full);
-    };
-
-    __syncthreads();
-    if (tid < 32) claim_and_copy();
-    uint32_t phase = 0;
-    for (;;) {
-        __syncthreads();
-        const long long item = s_item;
-        if (item >= a.total) break;
-        const int r_lo = s_rlo, r_hi = s_rhi;
-        long long ch, b0;
-        item_pos(item, ch, b0);
-        // rows outside the copied range: packed samples, zeros outside [0, len)
-        if (r_hi - r_lo < N1) {
-            for (int q = tid; q < N1 * N2; q += NT) {
-                const int r = q / N2, c = q - r * N2;
-                if (r >= r_lo && r < r_hi) continue;
-                const long long pos = b0 + q;
-                float           re = 0.f, im = 0.f;
-                if (pos >= 0 && pos < a.len) {
-                    const long long o = ch * a.src_stride + ((pos >> 3) << 4) + (pos & 7);
-                    re                = src[o];
-                    im                = src[o + 8];
-                }
-                float* row                         = reinterpret_cast<float*>(win + r * RS);
-                row[((c >> 3) << 4) + (c & 7)]     = re;
-                row[((c >> 3) << 4) + (c & 7) + 8] = im;
-            }
-        }
-        const bool ok = mbar_wait_bounded(&full, phase);
-        if (__syncthreads_or(!ok)) {
-            // give up: record it and let the copies in flight land first
-            if (tid == 0) {
-                atomicExch(a.error, 1);
-                mbar_wait_bounded(&full, phase, 100000000ull);
-            }
-            __syncthreads();
-            break;    // every thread leaves the loop together; TMEM is freed below
-        }
-        phase ^= 1;
-        if (a.inplace && tid == 0) {
-            __threadfence();
-            st_release(a.flags + item, a.epoch);    // this window is loaded
-        }
-        // packed -> interleaved, in place, one 64-byte pack per thread and step;
-        // consecutive threads take consecutive rows (row stride 65 x 16 bytes),
-        // so each quarter-warp's 16-byte accesses hit eight distinct bank groups
-        for (int q = tid; q < N1 * N2 / 8; q += NT) {
-            const int    r  = q % N1, p = q / N1;
-            float4*      w  = reinterpret_cast<float4*>(win + r * RS + p * 8);
-            const float4 r0 = w[0], r1 = w[1], i0 = w[2], i1 = w[3];
-            w[0]            = make_float4(r0.x, i0.x, r0.y, i0.y);
-            w[1]            = make_float4(r0.z, i0.z, r0.w, i0.w);
-            w[2]            = make_float4(r1.x, i1.x, r1.y, i1.y);
-            w[3]            = make_float4(r1.z, i1.z, r1.w, i1.w);
-        }
-        __syncthreads();
-
-        // ---------------- step 1: columns, forward, times W_N^(k1*n2)
-        {
-            const int g = tid / TT1, t = tid % TT1;
-            for (int rd = 0; rd < F::R1; ++rd) {
-                const int  n2 = rd * F::G1 + g;
-                cpx<float> v[E];
-                static_for<E>([&](auto ic) {
-                    constexpr int i = decltype(ic)::value;
-                    v[i]            = win[(t + i * TT1) * RS + n2];
-                });
-                stage_compute_tab<P1, 0>(v, t, tw1);
-                run_stages_full<P1, typename F::X1, true, -1>(v, xch, g, t, tw1);
-                const int e = t * n2;
-                apply_fourstep_tw(v, fwb[e + (e >> 4)], fwu1[n2], [&](auto ic, cpx<float> o) {
-                    constexpr int i              = decltype(ic)::value;
-                    win[(t + i * TT1) * RS + n2] = o;
-                });
-            }
-        }
-        __syncthreads();
-
-        // in place: thread 0 reads the load flags of the first previous windows
-        // now, so that step 3 rarely has to wait for them
-        unsigned pflag[4] = {0u, 0u, 0u, 0u};
-        if (a.inplace && tid == 0) {
-            const long long blk = item % a.nblk;
-            static_for<4>([&](auto dc) {
-                constexpr int d = decltype(dc)::value + 1;
-                if (d <= a.hwait && d <= blk) pflag[d - 1] = ld_acquire(a.flags + (item - d));
-            });
-        }
-        // ---------------- step 2: rows; spectrum times conj(K) or K; inverse rows
-        {
-            const int g = g2, t = t2;
-            for (int rd = 0; rd < F::R2; ++rd) {
-                const int  k1 = rd * F::G2 + r2;
-                cpx<float> v[E];
-                static_for<E>([&](auto ic) {
-                    constexpr int i = decltype(ic)::value;
-                    v[i]            = win[k1 * RS + t + i * TT2];
-                });
-                stage_compute_tab<P2, 0>(v, t, tw2);
-                run_stages_full<P2, typename F::X2, true, -1>(v, xch, g, t, tw2);
-                // v[i] = X[k1 + N1*k2], k2 = t + i*TT2: conj(X * conj(K)) or conj(X * K),
-                // K from tensor memory eight values at a time
-                static_for<2>([&](auto hc) {
-                    constexpr int h = decltype(hc)::value;
-                    uint32_t      kq[16];
-                    tmem_ld16(tcol + 32 * rd + 16 * h, kq);
-                    static_for<8>([&](auto jc) {
-                        constexpr int    i = 8 * h + decltype(jc)::value;
-                        const cpx<float> k = {__uint_as_float(kq[2 * (i - 8 * h)]), __uint_as_float(kq[2 * (i - 8 * h) + 1])};
-                        const cpx<float> c = {v[i].re, -v[i].im};
-                        v[i]               = a.conj_kernel ? cmul(c, k) : cmulc(c, k);
-                    });
-                });
-                stage_compute_tab<P2, 0>(v, t, tw2);
-                run_stages_full<P2, typename F::X2, true, -1>(v, xch, g, t, tw2);
-                // v[i] at n2 = t + i*TT2, times W_N^(k1*n2) = W_N^(k1*t) * W_N^(TT2*k1)^i
-                const int e = k1 * t;
-                apply_fourstep_tw(v, fwb[e + (e >> 4)], fwu2[k1], [&](auto ic, cpx<float> o) {
-                    constexpr int i           = decltype(ic)::value;
-                    win[k1 * RS + t + i * TT2] = o;
-                });
-            }
-        }
-        __syncthreads();
-
-        // ---------------- step 3: columns again; outputs y = conj(.)
-        if (a.inplace) {
-            // the outputs overwrite samples of the windows of the hwait
-            // previous blocks of this channel: wait until those are loaded
-            if (tid == 0) {
-                s_abort              = 0;
-                const long long blk  = item % a.nblk;
-                for (int d = 1; d <= a.hwait && d <= blk && !s_abort; ++d) {
-                    const unsigned* f = a.flags + (item - d);
-                    if (d <= 4) {
-                        unsigned pv = 0u;
-                        static_for<4>([&](auto ic) {
-                            if (decltype(ic)::value == d - 1) pv = pflag[decltype(ic)::value];
-                        });
-                        if (pv == a.epoch) continue;
-                    }
-                    if (ld_acquire(f) == a.epoch) continue;
-                    const unsigned long long t0 = globaltimer_ns();
-                    while (ld_acquire(f) != a.epoch) {
-                        if (globaltimer_ns() - t0 > XC_WAIT_NS) {
-                            atomicExch(a.error, 1);
-                            s_abort = 1;
-                            break;
-                        }
-                        __nanosleep(256);
-                    }
-                }
-            }
-            __syncthreads();
-            if (s_abort) break;    // every thread leaves together; no copy is in flight
-        }
-        {
-            const int       g    = tid / TT1, t = tid % TT1;
-            // window index n is output position e0 + n; it is written when
-            // out_shift <= n < out_shift + step and e0 + n < len.  e0 and every
-            // row start are whole packs, so the packed offset of e0 + row*N2 + n2
-            // is 2*(e0 + row*N2) + pk(n2).
-            const long long e0 = b0 + a.in_shift - a.out_shift;
-            const int       lo = a.out_shift;
-            const long long hl = min((long long)a.out_shift + a.step, a.len - e0);
-            const int       hi = (int)max(0LL, min(hl, (long long)N1 * N2));
-            float*          d  = dst + ch * a.dst_stride + 2 * e0;
-            for (int rd = 0; rd < F::R1; ++rd) {
-                const int  n2 = rd * F::G1 + g;
-                cpx<float> v[E];
-                static_for<E>([&](auto ic) {
-                    constexpr int i = decltype(ic)::value;
-                    v[i]            = win[(t + i * TT1) * RS + n2];
-                });
-                if (rd == F::R1 - 1) {
-                    // the window is read: start the next block's copies
-                    fence_proxy_async_smem();
-                    __syncthreads();
-                    if (tid < 32) claim_and_copy();
-                }
-                stage_compute_tab<P1, 0>(v, t, tw1);
-                run_stages_full<P1, typename F::X1, true, -1>(v, xch, g, t, tw1);
-                float* drow = d + 2 * t * N2 + ((n2 >> 3) << 4) + (n2 & 7);
-                static_for<E>([&](auto ic) {
-                    constexpr int i = decltype(ic)::value;
-                    const int     n = (t + i * TT1) * N2 + n2;    // window index
-                    if (n >= lo && n < hi) {
-                        __stcs(drow + 2 * i * TT1 * N2, v[i].re);
-                        __stcs(drow + 2 * i * TT1 * N2 + 8, -v[i].im);
-                    }
-                });
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (tid < 32) tmem_dealloc(tbase, TCOLS);
-}
-
 // ---------------------------------------------------------------------------
 // Kernel-gradient pass in the same form (the counterpart of k_fxcorr_kgrad for
 // FP32 N = 2^13 / 2^14, pack 8): per block, the gy block (zero-padded to N)
