@@ -99,7 +99,7 @@ size_t pcx_plan_workspace_size(pcx_plan plan, size_t batch);
 
 /* Forms of a transform larger than 4096 points (pcx_plan_tune). */
 #define PCX_FORM_DEFAULT 0  /* built-in choice */
-#define PCX_FORM_ONEPASS 1  /* one shared-memory pass (FP32 n = 8192) */
+#define PCX_FORM_ONEPASS 1  /* one shared-memory pass (n = 8192, FP32 16384) */
 #define PCX_FORM_FUSED 2    /* four-step, the whole batch in one persistent launch */
 #define PCX_FORM_CHUNKED 3  /* four-step, two launches per L2-sized scratch chunk */
 
@@ -108,7 +108,7 @@ size_t pcx_plan_workspace_size(pcx_plan plan, size_t batch);
  * schedule at compile time, fft.hpp:546-575, 1856-1958).  Times the forms
  * this plan supports on `batch` rows of scratch data (forward, natural order,
  * default pack; at most 512 MB per buffer) on `stream`: the one-pass form
- * (FP32 n = 8192), every built-in variant of the one-launch four-step for this
+ * (n = 8192, FP32 16384), every built-in variant of the one-launch four-step for this
  * size (split N1 x N2, i.e. the radix schedule of both passes; tile shape as
  * blocks per SM; ring stages) at three dependency distances, and the chunked
  * four-step at two scratch sizes; it makes the fastest the plan's form for

@@ -160,6 +160,25 @@ struct splan {
     }
 };
 
+// The same with 32 values per thread and radices of up to 32, as equal as they
+// come (larger first): 512 = 32*16, 1024 = 32*32, 8192 = 32*16*16,
+// 16384 = 32*32*16 in one stage less than radix 16 takes.
+template<int LOGL_>
+struct splan32 {
+    static constexpr int LOGL = LOGL_;
+    static constexpr int L    = 1 << LOGL;
+    static constexpr int E    = 32;
+    static constexpr int TT   = L / E;
+    static constexpr int NST  = (LOGL + 4) / 5;
+    static_assert(LOGL >= 5, "at least 32 points");
+    __host__ __device__ static constexpr int rbits(int s) { return LOGL / NST + (s < LOGL % NST ? 1 : 0); }
+    __host__ __device__ static constexpr int nsbits(int s) {
+        int b = 0;
+        for (int i = 0; i < s; ++i) b += rbits(i);
+        return b;
+    }
+};
+
 // Butterflies of stage S.  twL: table W_L^i (i < L).
 template<class P, int S, class T, int E>
 __device__ __forceinline__ void stage_compute(cpx<T> (&v)[E], int t, const cpx<T>* __restrict__ twL) {

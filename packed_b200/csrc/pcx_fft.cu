@@ -343,7 +343,7 @@ static int plan_init_tables(pcx_plan_s* p) {
             p->fst2 = static_cast<char*>(p->fst) + (size_t)f1 * eb;
             PCX_CUDA_TRY(pcx_fourstep_tables(p->log_n1, p->fst1, f64, 0, &f1));
             PCX_CUDA_TRY(pcx_fourstep_tables(p->log_n2, p->fst2, f64, 0, &f2));
-            // 2^13 has a one-pass form (a block of 512 threads a row)
+            // 2^13 and in FP32 2^14 have a one-pass form (a block a row)
             if (pcx_rows(f64, log_n, {}, 0, true) == cudaSuccess && pcx_rows_any(f64, log_n, {}, 0, true) == cudaSuccess) {
                 for (cudaError_t e: {pcx_v3_single(f64, log_n, {}, 0, p->sms, true),
                                      pcx_v3_single_any(f64, log_n, {}, 0, p->sms, true)}) {
@@ -355,6 +355,12 @@ static int plan_init_tables(pcx_plan_s* p) {
                 PCX_CUDA_TRY(pcx_v2_stage_twiddles(log_n, p->stw_one, f64, 0, &e3));
             }
         }
+    }
+    int er = 0;
+    PCX_CUDA_TRY(pcx_rows_twiddles(f64, log_n, nullptr, 0, &er));
+    if (er > 0 && (!p->two_pass || p->stw_one)) {
+        PCX_CUDA_TRY(cudaMalloc(&p->stw_rows, (size_t)er * eb));
+        PCX_CUDA_TRY(pcx_rows_twiddles(f64, log_n, p->stw_rows, 0, &er));
     }
     PCX_CUDA_TRY(cudaDeviceSynchronize());
     return PCX_OK;
@@ -412,6 +418,7 @@ void pcx_plan_s::release() {
     if (tw) cudaFree(tw);
     if (stw) cudaFree(stw);
     if (stw_one) cudaFree(stw_one);
+    if (stw_rows) cudaFree(stw_rows);
     if (fst) cudaFree(fst);
     if (fs.mem && fs.mem != fs_def.mem) cudaFree(fs.mem);
     if (fs_def.mem) cudaFree(fs_def.mem);
@@ -433,6 +440,7 @@ void pcx_plan_s::release() {
     tw      = nullptr;
     stw     = nullptr;
     stw_one  = nullptr;
+    stw_rows = nullptr;
     fst      = nullptr;
     fst1     = nullptr;
     fst2     = nullptr;
@@ -827,7 +835,9 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         // natural order from 256 points on (FP64: 128) goes straight through
         // registers; k_single3 is faster below and takes the other orders
         if (natural && p->log_n >= 7 && (f64 || p->log_n >= 8 || !tma)) {
+            if (p->stw_rows) t3.stw = p->stw_rows;
             const cudaError_t e = (plain ? pcx_rows : pcx_rows_any)(f64, p->log_n, t3, st, false);
+            t3.stw              = stw;
             if (e != cudaErrorNotSupported) return e;
         }
         if (!tma) return cudaErrorNotSupported;

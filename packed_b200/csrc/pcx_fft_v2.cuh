@@ -26,6 +26,7 @@ namespace pcxg {
 // R.  Its twiddles are W^(j*k), W = W_{Ns*R}, j = 1..R-1.  Writing j = 4m + i
 // (i, m < 4), W^(jk) = W^(ik) * W^(4mk), so the table keeps, per position k,
 // only the factors (generated in FP64, rounded once):
+//   R = 32: W^k, W^2k, W^3k, W^4k, W^8k, ..., W^28k
 //   R = 16: W^k, W^2k, W^3k, W^4k, W^8k, W^12k
 //   R = 8:  W^k, W^2k, W^3k, W^4k
 //   R = 4:  W^k, W^2k, W^3k, 1
@@ -33,9 +34,9 @@ namespace pcxg {
 // and a butterfly forms each twiddle as one entry or the product of two.  That
 // is 48 bytes per radix-16 butterfly instead of 120, and the entries of
 // consecutive positions are contiguous (16-byte vector loads).
-__host__ __device__ constexpr int stw_q(int rb) { return rb == 4 ? 6 : (rb == 1 ? 2 : 4); }
+__host__ __device__ constexpr int stw_q(int rb) { return rb == 5 ? 10 : (rb == 4 ? 6 : (rb == 1 ? 2 : 4)); }
 __host__ __device__ constexpr int stw_mult(int rb, int q) {
-    return q < 3 ? ((q + 1) < (1 << rb) ? q + 1 : 0) : (rb == 4 ? 4 * (q - 2) : (rb == 3 && q == 3 ? 4 : 0));
+    return q < 3 ? ((q + 1) < (1 << rb) ? q + 1 : 0) : (rb >= 4 ? 4 * (q - 2) : (rb == 3 && q == 3 ? 4 : 0));
 }
 template<class P>
 __host__ __device__ constexpr int stage_tw_offset(int S) {
@@ -349,33 +350,46 @@ struct v3_args {
     int         pairs;      // interleaved rows may be moved a complex number at a time (aligned)
 };
 
+// Exchange layout of 32-point stages: one slot of padding per 32.
+template<int L, int M>
+struct xch_blocked32 {
+    static constexpr int LP   = L + L / 32;
+    static constexpr int size = M * LP;
+    __device__ static __forceinline__ int idx(int m, int l) { return m * LP + l + (l >> 5); }
+};
+
 // ---------------------------------------------------------------------------
 // Single pass, natural order on both sides: rows straight between HBM and
-// registers, 16 points per thread, shared memory for the exchanges only.
+// registers, 16 or 32 points per thread, shared memory for the exchanges only.
 //
-// Bound by HBM: what counts is warps in flight.  A thread keeps to 64
-// registers in FP32 (32 of them data) and 128 in FP64, so 32 (16) warps fit an
-// SM; their loads cover the latency without a copy ring, which at 16 warps
-// an SM was the faster form only with the ring's help, and a block's barriers
-// stall 128 threads at a time where a row allows it (256 for 4096 points).
-// Stage factors come through L1.  GB/s (16 B per point, 32 B in FP64), 512 MB
-// a buffer, of 6544 measured copy; before: the TMA-fed kernel (k_single3),
-// rows staged in shared memory both ways, 16 warps an SM (FP64: 8):
-//   N            256  512 1024 2048 4096 8192   FP64: 128  256  512 1024 2048 4096 8192
-//   before      5917 4944 4436 4544 4526 3255        4364 4982 4073 3516 3658 3860 1833
-//   this        6687 6237 5578 6014 5660 4225        6799 6779 5929 5044 5317 5092 3320
-//   256 threads 6729 6168 5582 5773                  6587 6798 5576 4557 4901
-// (8192 before: the four-step's tuned form reached 3500 in FP32.)  With 3 and
-// 2 blocks of 256 threads in FP32: 4096 5480 and 4430.  At 128 points in FP32
-// a row's eight threads cover single 32-byte sectors and k_single3 is faster
-// (6270 against 5630); 16384 in one pass is slower (3043) than the four-step.
+// Bound by HBM: what counts is warps in flight and stages.  With 16 points a
+// thread keeps to 64 registers in FP32 (32 of them data) and 128 in FP64, so
+// 32 (16) warps fit an SM; their loads cover the latency without a copy ring,
+// which at 16 warps an SM was the faster form only with the ring's help, and a
+// block's barriers stall 128 threads at a time where a row allows it (256 for
+// 4096 points).  Where 32 points a thread (128 registers, 16 warps) save a
+// stage and its exchange they are faster still: FP32 512, 1024, 8192, 16384
+// (2048 and 4096 take three stages either way: 5450 and 5523).  Stage factors
+// come through L1.  GB/s (16 B per point, 32 B in FP64), 512 MB a buffer, of
+// 6544 measured copy; before: the TMA-fed kernel (k_single3), rows staged in
+// shared memory both ways, 16 warps an SM (FP64: 8):
+//   N            256  512 1024 2048 4096 8192 16384  FP64: 128  256  512 1024 2048 4096 8192
+//   before      5917 4944 4436 4544 4526 3255  3404       4364 4982 4073 3516 3658 3860 1833
+//   this        6703 6470 6488 6026 5654 5092  3690       6726 6722 5954 5049 5309 5095 3316
+//   16 points   6703 6220 5575           4228  3043
+//   256 threads 6729 5690 5720 5773                       6587 6798 5576 4557 4901
+// (8192 and 16384 before: 3500 and 3404 in the four-step's tuned form.)  4096
+// points with 3 and 2 blocks of 256 threads an SM: 5480 and 4430.  At 128
+// points in FP32 a row's eight threads cover single 32-byte sectors and
+// k_single3 is faster (6270 against 5630).
 template<class T, int LOGL>
 struct rows_cfg {
-    using P                   = splan<LOGL>;
+    static constexpr bool W   = sizeof(T) == 4 && (LOGL == 9 || LOGL == 10 || LOGL >= 13);    // 32 points per thread
+    using P                   = std::conditional_t<W, splan32<LOGL>, splan<LOGL>>;
     static constexpr int NT   = P::TT > 128 ? P::TT : 128;
     static constexpr int M    = NT / P::TT;
-    static constexpr int MINB = (sizeof(T) == 8 ? 512 : 1024) / NT;
-    using X                   = xch_blocked<P::L, M>;
+    static constexpr int MINB = (sizeof(T) == 8 || W ? 512 : 1024) / NT;
+    using X                   = std::conditional_t<W, xch_blocked32<P::L, M>, xch_blocked<P::L, M>>;
     static constexpr int SMEM = X::size * (int)sizeof(cpx<T>);
 };
 

@@ -13,11 +13,49 @@ static cudaError_t dispatch_rows(int log_n, const v3_args& a, cudaStream_t st, b
     case 11: return launch_rows<T, 11, false>(a, st, attr_only);
     case 12: return launch_rows<T, 12, false>(a, st, attr_only);
     case 13: return launch_rows<T, 13, false>(a, st, attr_only);
+    case 14:
+        if constexpr (sizeof(T) == 4) return launch_rows<T, 14, false>(a, st, attr_only);
+        return cudaErrorNotSupported;
     default: return cudaErrorNotSupported;
     }
 }
 
+template<class T, int LOGL>
+static cudaError_t rows_twiddles(void* out, cudaStream_t st, int* entries) {
+    using P  = typename rows_cfg<T, LOGL>::P;
+    *entries = rows_cfg<T, LOGL>::W ? stage_tw_size<P>() : 0;
+    if (!out || *entries == 0) return cudaSuccess;
+    for (int s = 1; s < P::NST; ++s) {
+        const int ns = 1 << P::nsbits(s), nq = stw_q(P::rbits(s));
+        k_stage_twiddles<T><<<(ns * nq + 255) / 256, 256, 0, st>>>(static_cast<cpx<T>*>(out) + stage_tw_offset<P>(s), ns,
+                                                                  P::rbits(s), P::nsbits(s) + P::rbits(s));
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+template<class T>
+static cudaError_t dispatch_twiddles(int log_n, void* out, cudaStream_t st, int* entries) {
+    *entries = 0;
+    switch (log_n) {
+    case 7: return rows_twiddles<T, 7>(out, st, entries);
+    case 8: return rows_twiddles<T, 8>(out, st, entries);
+    case 9: return rows_twiddles<T, 9>(out, st, entries);
+    case 10: return rows_twiddles<T, 10>(out, st, entries);
+    case 11: return rows_twiddles<T, 11>(out, st, entries);
+    case 12: return rows_twiddles<T, 12>(out, st, entries);
+    case 13: return rows_twiddles<T, 13>(out, st, entries);
+    case 14: return rows_twiddles<T, 14>(out, st, entries);
+    default: return cudaSuccess;
+    }
+}
+
 }    // namespace pcxg
+
+cudaError_t pcx_rows_twiddles(bool f64, int log_n, void* out, cudaStream_t st, int* entries) {
+    return f64 ? pcxg::dispatch_twiddles<double>(log_n, out, st, entries)
+               : pcxg::dispatch_twiddles<float>(log_n, out, st, entries);
+}
 
 cudaError_t pcx_rows(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, bool attr_only) {
     return f64 ? pcxg::dispatch_rows<double>(log_n, a, st, attr_only)

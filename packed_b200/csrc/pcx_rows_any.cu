@@ -13,6 +13,9 @@ static cudaError_t dispatch_rows(int log_n, const v3_args& a, cudaStream_t st, b
     case 11: return launch_rows<T, 11, true>(a, st, attr_only);
     case 12: return launch_rows<T, 12, true>(a, st, attr_only);
     case 13: return launch_rows<T, 13, true>(a, st, attr_only);
+    case 14:
+        if constexpr (sizeof(T) == 4) return launch_rows<T, 14, true>(a, st, attr_only);
+        return cudaErrorNotSupported;
     default: return cudaErrorNotSupported;
     }
 }

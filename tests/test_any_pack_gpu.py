@@ -21,7 +21,7 @@ def _stride(n, pack, vec):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-@pytest.mark.parametrize("lg", [5, 6, 8, 9, 11, 12, 13])
+@pytest.mark.parametrize("lg", [5, 6, 7, 8, 9, 10, 11, 12, 13, 14])
 @pytest.mark.parametrize("ps,pd", [(1, 8), (8, 1), (1, 1), (2, 4), (16, 2), (4, 16)])
 def test_widths_and_short_rows(dtype, lg, ps, pd):
     npd = np.float32 if dtype == torch.float32 else np.float64
