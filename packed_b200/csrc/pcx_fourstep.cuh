@@ -92,6 +92,7 @@ struct fs_args {
 //    n2 from bitrev(n2), again one run of 16 per thread.
 // 2^15, 301 transforms, forward into `unordered` and inverse back: two
 // launches per chunk of general kernels 427 us, these 119 us.
+constexpr int FS_TS_ROUNDS = 12;
 constexpr int FS_PLAIN = 0;
 constexpr int FS_ANY   = 1;
 constexpr int FS_OUT   = 2;
@@ -184,7 +185,9 @@ struct fs_cfg {
     // puts its outputs over values that it (row tiles: a lane beside it) read
     // last, without a block barrier, and the publisher issues one to eight
     // copies a tile.  The stage is held until its copy has read it, which costs
-    // the short tiles more than it saves.  GB/s at 512 MB, from registers and
+    // the short tiles more than it saves, and the two tensor maps cost a call
+    // 3.5 us on the host: launch_fs takes it from FS_TS_ROUNDS items a block on.
+    // GB/s at 512 MB, from registers and
     // staged: FP32 2^14 3405 3261, 2^15 3459 3249, 2^16 3313 3015, 2^17 2947
     // 3043, 2^18 2867 2950, 2^19 2523 2818, 2^20 2541 2830; FP64 2^14 3429 3502,
     // 2^15 3372 3399, 2^16 3351 3508, 2^17 2691 3254, 2^18 2429 2928.
@@ -282,7 +285,7 @@ __device__ __forceinline__ fs_item fs_decode(uint32_t j, uint32_t batch, uint32_
     return {1, (int)(batch - lag + j / TR), (int)(j % TR)};
 }
 
-template<class T, int LOGN1, int LOGN2, int MINB, int ST_, int FORM = FS_PLAIN>
+template<class T, int LOGN1, int LOGN2, int MINB, int ST_, int FORM, bool TS>
 __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, MINB)
     k_fourstep(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tscr,
                const __grid_constant__ CUtensorMap tdst, fs_args a) {
@@ -307,7 +310,7 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
     constexpr int RSI  = F::RSI;
     constexpr int RROW = N2 * (int)sizeof(cpx<T>);
     constexpr bool SH  = F::SH;
-    constexpr bool TS  = F::TS;                      // outputs staged in the item's stage and stored by TMA
+    static_assert(!TS || F::TS, "outputs staged in the item's stage and stored by TMA");
     constexpr bool TSR = TS && FORM != FS_OUT;       // row tiles too (FS_OUT stores whole rows itself)
     static_assert(FORM != FS_IN || C * F::RSC * (int)sizeof(T) <= F::STAGE, "a column tile of whole rows fits a stage");
     static_assert(FORM != FS_OUT || CR * 2 * N2 * (int)sizeof(T) <= (IP ? F::STAGE : F::XB), "a staged row tile fits");

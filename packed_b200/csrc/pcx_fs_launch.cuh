@@ -17,11 +17,16 @@ cudaError_t launch_fs(const fs_args& a, cudaStream_t st, int sms, bool attr_only
     static_assert(F::SMEM <= 232448, "shared memory per block");
     static_assert(F::MINB * (F::SMEM + 1024 + 256) <= 233472, "blocks per SM fit the shared memory");
     static_assert(F::STAGE % 128 == 0, "TMA destinations stay 128-byte aligned");
-    auto kern = k_fourstep<T, LOGN1, LOGN2, MINB, ST, FORM>;
+    auto kern = k_fourstep<T, LOGN1, LOGN2, MINB, ST, FORM, false>;
     if (tc) *tc = F::TC;
     if (tr) *tr = F::TR;
     if (attr_only) {
         cudaError_t e = smem_attr_cached(reinterpret_cast<const void*>(kern), F::SMEM);
+        if constexpr (F::TS) {
+            if (e == cudaSuccess) {
+                e = smem_attr_cached(reinterpret_cast<const void*>(k_fourstep<T, LOGN1, LOGN2, MINB, ST, FORM, true>), F::SMEM);
+            }
+        }
         if (e == cudaSuccess && per_sm) e = occupancy_cached(reinterpret_cast<const void*>(kern), F::NT + 64, F::SMEM, per_sm);
         return e;
     }
@@ -39,26 +44,33 @@ cudaError_t launch_fs(const fs_args& a, cudaStream_t st, int sms, bool attr_only
     const cuuint32_t estr[3]    = {1, 1, 1};
     cudaError_t      e = encode_tensor_map(&map, sizeof(T) == 8, 3, const_cast<void*>(a.src), dims, strides, box, estr);
     if (e != cudaSuccess) return FORM == FS_PLAIN ? e : cudaErrorNotSupported;    // the caller has another path
-    // 4-D views that the outputs are stored through, [.][16-row block][row of it][reals]: the scratch
-    // (rows k1 of slot .) and the destination (rows k2 of transform .).  Boxes are 17 rows high: the
-    // 17th, outside the view, is the padding row of the shared layout and is not written.
-    CUtensorMap      tscr, tdst;
-    const cuuint32_t estr4[4]    = {1, 1, 1, 1};
-    const cuuint64_t sdims[4]    = {(cuuint64_t)2 << LOGN2, 16, (cuuint64_t)F::N1 / 16, (cuuint64_t)a.nslot};
-    const cuuint64_t sstr[3]     = {((cuuint64_t)2 << LOGN2) * sizeof(T), ((cuuint64_t)32 << LOGN2) * sizeof(T),
-                                    ((cuuint64_t)2 << (LOGN1 + LOGN2)) * sizeof(T)};
-    const cuuint32_t sbox[4]     = {(cuuint32_t)(2 * F::C), 17, (cuuint32_t)F::N1 / 16, 1};
-    const long long  ds          = a.batch > 1 ? a.dst_stride : (2LL << (LOGN1 + LOGN2));
-    const cuuint64_t ddims[4]    = {(cuuint64_t)2 << LOGN1, 16, (cuuint64_t)F::N2 / 16, (cuuint64_t)a.batch};
-    const cuuint64_t dstr[3]     = {((cuuint64_t)2 << LOGN1) * sizeof(T), ((cuuint64_t)32 << LOGN1) * sizeof(T),
-                                    (cuuint64_t)ds * sizeof(T)};
-    const cuuint32_t dbox[4]     = {(cuuint32_t)(2 * F::G8), 17, (cuuint32_t)F::N2 / 16, 1};
-    e = encode_tensor_map(&tscr, sizeof(T) == 8, 4, a.scratch, sdims, sstr, sbox, estr4);
-    if (e == cudaSuccess) e = encode_tensor_map(&tdst, sizeof(T) == 8, 4, a.dst, ddims, dstr, dbox, estr4);
-    if (e != cudaSuccess) return FORM == FS_PLAIN ? e : cudaErrorNotSupported;
     unsigned grid = 0;
     e             = persistent_grid(kern, F::NT + 64, F::SMEM, items, sms, &grid);
     if (e != cudaSuccess) return e;
+    // outputs through TMA: F::TS and enough items for the load/store queue to matter
+    CUtensorMap tscr{}, tdst{};
+    if constexpr (F::TS) {
+        if (items >= (long long)FS_TS_ROUNDS * grid) {
+            // 4-D views that the outputs are stored through, [.][16-row block][row of it][reals]: the scratch
+            // (rows k1 of slot .) and the destination (rows k2 of transform .).  Boxes are 17 rows high: the
+            // 17th, outside the view, is the padding row of the shared layout and is not written.
+            const cuuint32_t estr4[4]    = {1, 1, 1, 1};
+            const cuuint64_t sdims[4]    = {(cuuint64_t)2 << LOGN2, 16, (cuuint64_t)F::N1 / 16, (cuuint64_t)a.nslot};
+            const cuuint64_t sstr[3]     = {((cuuint64_t)2 << LOGN2) * sizeof(T), ((cuuint64_t)32 << LOGN2) * sizeof(T),
+                                            ((cuuint64_t)2 << (LOGN1 + LOGN2)) * sizeof(T)};
+            const cuuint32_t sbox[4]     = {(cuuint32_t)(2 * F::C), 17, (cuuint32_t)F::N1 / 16, 1};
+            const long long  ds          = a.batch > 1 ? a.dst_stride : (2LL << (LOGN1 + LOGN2));
+            const cuuint64_t ddims[4]    = {(cuuint64_t)2 << LOGN1, 16, (cuuint64_t)F::N2 / 16, (cuuint64_t)a.batch};
+            const cuuint64_t dstr[3]     = {((cuuint64_t)2 << LOGN1) * sizeof(T), ((cuuint64_t)32 << LOGN1) * sizeof(T),
+                                            (cuuint64_t)ds * sizeof(T)};
+            const cuuint32_t dbox[4]     = {(cuuint32_t)(2 * F::G8), 17, (cuuint32_t)F::N2 / 16, 1};
+            e = encode_tensor_map(&tscr, sizeof(T) == 8, 4, a.scratch, sdims, sstr, sbox, estr4);
+            if (e == cudaSuccess) e = encode_tensor_map(&tdst, sizeof(T) == 8, 4, a.dst, ddims, dstr, dbox, estr4);
+            if (e != cudaSuccess) return FORM == FS_PLAIN ? e : cudaErrorNotSupported;
+            k_fourstep<T, LOGN1, LOGN2, MINB, ST, FORM, true><<<grid, F::NT + 64, F::SMEM, st>>>(map, tscr, tdst, a);
+            return cudaGetLastError();
+        }
+    }
     kern<<<grid, F::NT + 64, F::SMEM, st>>>(map, tscr, tdst, a);
     return cudaGetLastError();
 }
@@ -94,7 +106,7 @@ cudaError_t launch_fs(const fs_args& a, cudaStream_t st, int sms, bool attr_only
         PCX_FS_FORM_VARIANT(double, 8, 8, 2, 3)                                                               \
         PCX_FS_FORM_VARIANT(double, 9, 8, 2, 3)                                                               \
         PCX_FS_FORM_VARIANT(double, 9, 9, 2, 3)                                                               \
-        PCX_FS_FORM_VARIANT(double, 10, 9, 1, 3)                                                              \
+        PCX_FS_FORM_VARIANT(double, 10, 9, 1, 2)                                                              \
         PCX_FS_FORM_VARIANT(double, 10, 10, 1, 2)                                                             \
         return cudaErrorNotSupported;                                                                         \
     }

@@ -92,8 +92,7 @@ constexpr fs_variant kFsVariantsF32[] = {
     {10, 10, 1, 3}, {10, 10, 1, 2},                                   // 2^20
 };
 constexpr fs_variant kFsVariantsF64[] = {
-    {7, 7, 2, 3}, {8, 7, 2, 3}, {8, 8, 2, 3}, {9, 8, 2, 3}, {9, 9, 2, 3}, {10, 9, 1, 3}, {10, 9, 1, 2},
-    {10, 10, 1, 2},
+    {7, 7, 2, 3}, {8, 7, 2, 3}, {8, 8, 2, 3}, {9, 8, 2, 3}, {9, 9, 2, 3}, {10, 9, 1, 2}, {10, 10, 1, 2},
 };
 }
 
