@@ -957,10 +957,11 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
             if (p->fs_ctr) cudaFree(p->fs_ctr);
             p->fs_ctr   = nullptr;
             p->fs_ctr_n = 0;
-            PCX_CUDA_TRY(cudaMalloc(&p->fs_ctr, 2 * batch * sizeof(int)));
+            PCX_CUDA_TRY(cudaMalloc(&p->fs_ctr, (2 * batch + 1) * sizeof(int)));
             p->fs_ctr_n = 2 * batch;
+            // from here on every launch leaves them zero
+            PCX_CUDA_TRY(cudaMemsetAsync(p->fs_ctr, 0, (2 * batch + 1) * sizeof(int), st));
         }
-        PCX_CUDA_TRY(cudaMemsetAsync(p->fs_ctr, 0, 2 * batch * sizeof(int), st));
         fs_args a{};
         a.src        = src;
         a.dst        = dst;
@@ -979,8 +980,9 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         a.scratch    = p->scratch;
         a.nslot      = (int)nslot;
         a.lag        = (int)lag;
-        a.col_done   = p->fs_ctr;
-        a.row_done   = p->fs_ctr + batch;
+        a.ticket     = p->fs_ctr;
+        a.col_done   = p->fs_ctr + 1;
+        a.row_done   = p->fs_ctr + 1 + batch;
         a.error      = p->err;
         a.lp_src     = io.lp_src;
         a.lp_dst     = io.lp_dst;

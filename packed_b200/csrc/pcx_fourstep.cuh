@@ -59,8 +59,9 @@ struct fs_args {
     void*       scratch;  // nslot slots of N complex
     int         nslot;    // a power of two: transform r uses slot r & (nslot - 1)
     int         lag;      // transforms between a column pass and its row pass
-    int*        col_done;
-    int*        row_done;
+    int*        col_done;    // one per transform, zero at the start and at the end of a launch
+    int*        row_done;    // the same, right behind col_done
+    int*        ticket;      // blocks that are done with the counters, likewise zero outside a launch
     int*        error;
     // forms other than FS_PLAIN only
     int         lp_src;     // log2 pack widths
@@ -418,8 +419,22 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
                 mbar_arrive(&empty[s]);
             }
         }
-        if (TS && lane == 0) bulk_wait();    // nothing is in flight when the block exits
-        __syncwarp();
+        // nothing is in flight when the block exits; the last block to get
+        // here (every one does, also after giving up) leaves the counters zero
+        // for the next launch, which a memset before each call did for one more
+        // launch and 2-3 us of a short call
+        int last = 0;
+        if (lane == 0) {
+            if (TS) bulk_wait();
+            __threadfence();
+            last = atomicAdd(a.ticket, 1) == (int)gridDim.x - 1;
+            __threadfence();
+        }
+        if (__shfl_sync(0xffffffffu, last, 0)) {
+#pragma unroll 4
+            for (uint32_t q = lane; q < 2 * batch; q += 32) a.col_done[q] = 0;
+            if (lane == 0) *a.ticket = 0;
+        }
         return;
     }
 

@@ -24,7 +24,7 @@ struct pcx_fxcorr_s {
     pcx_plan_s* plan   = nullptr;    // natural-order N-point FFT (kernel spectrum, gradient inverse)
     void*       tw     = nullptr;    // W_N^i, i < N
     void*       kspec  = nullptr;    // FFT(g)/N, interleaved complex, natural order
-    unsigned*   ctl    = nullptr;    // [0] work counter, [1] error flag, [2..] flags
+    unsigned*   ctl    = nullptr;    // [0] work counter, [1] error flag, [2] ticket, [3..] flags
     size_t      flags_cap = 0;
     unsigned    epoch     = 0;
     void*       gscratch  = nullptr;    // kernel-gradient accumulators
@@ -287,8 +287,8 @@ int ensure_flags(pcx_fxcorr_s* h, size_t items) {
     h->ctl       = nullptr;
     h->flags_cap = 0;
     const size_t cap = std::max<size_t>(items, 1024);
-    PCX_CUDA_TRY(cudaMalloc(&h->ctl, (cap + 2) * sizeof(unsigned)));
-    PCX_CUDA_TRY(cudaMemset(h->ctl, 0, (cap + 2) * sizeof(unsigned)));
+    PCX_CUDA_TRY(cudaMalloc(&h->ctl, (cap + 3) * sizeof(unsigned)));
+    PCX_CUDA_TRY(cudaMemset(h->ctl, 0, (cap + 3) * sizeof(unsigned)));
     h->flags_cap = cap;
     h->epoch     = 0;
     return PCX_OK;
@@ -315,7 +315,7 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     if (inplace && convolve) return pcx_fail(PCX_ERR_INVALID, "the adjoint needs distinct input and output buffers");
     if (int rc = ensure_flags(h, inplace ? total : 1)) return rc;
     if (++h->epoch == 0) {
-        PCX_CUDA_TRY(cudaMemsetAsync(h->ctl + 2, 0, h->flags_cap * sizeof(unsigned), st));
+        PCX_CUDA_TRY(cudaMemsetAsync(h->ctl + 3, 0, h->flags_cap * sizeof(unsigned), st));
         h->epoch = 1;
     }
 
@@ -341,15 +341,15 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     a.inplace     = inplace ? 1 : 0;
     a.hwait       = (int)((n + step - 1) / step) - 1;
     a.epoch       = h->epoch;
-    a.flags       = h->ctl + 2;
+    a.flags       = h->ctl + 3;
     a.counter     = h->ctl;
+    a.ticket      = h->ctl + 2;
     a.error       = reinterpret_cast<int*>(h->ctl + 1);
     a.kspec       = h->kspec;
     // whole-window and three-step forms: FP32, pack 8, windows on whole
     // packs, rows of packs 16-byte aligned
     const bool rows = pack == 8 && a.in_shift % 8 == 0 && (channels == 1 || sstride % 4 == 0) &&
                       reinterpret_cast<uintptr_t>(src) % 16 == 0;
-    if (inplace || !(h->x3 && rows)) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), st));
     if (h->x3 && rows) return dispatch_xc3(h->log_n, a, h->plan->stwL, st, h->sms);
     const bool x2 = h->x2d && rows;
     if (x2) {
@@ -537,7 +537,7 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
                 cudaError_t e = cudaSuccess;
                 if (h->unsure) e = cudaDeviceSynchronize();
                 else if (h->used) e = cudaStreamWaitEvent(0, h->done, 0);
-                if (e == cudaSuccess && h->ctl) e = cudaMemsetAsync(h->ctl, 0, 2 * sizeof(unsigned), 0);
+                if (e == cudaSuccess && h->ctl) e = cudaMemsetAsync(h->ctl, 0, 3 * sizeof(unsigned), 0);
                 PCX_CUDA_TRY(e);
                 h->used = h->unsure = false;
             } else {
@@ -652,7 +652,6 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
         h->gscratch_bytes = need;
     }
     if (int rc = ensure_flags(h, 1)) return rc;
-    if (!x3) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), st));
     char* base = static_cast<char*>(h->gscratch);
     a.x       = x;
     a.gy      = gy;
@@ -662,6 +661,7 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
     a.step    = (int)step;
     a.nblk    = (int)nblk;
     a.counter = h->ctl;
+    a.ticket  = h->ctl + 2;
     a.error   = reinterpret_cast<int*>(h->ctl + 1);
     a.acc     = base;
     a.xspec   = base + (size_t)grid * n * eb;

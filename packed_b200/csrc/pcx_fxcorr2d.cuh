@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(512, 1) k_fxcorr2d_kgrad(xc2_kg_args A) {
         }
         if (aborted) break;
     }
+    if (tid == 0) xc_done(a.counter, a.ticket);
     if (!aborted) {
         // this CTA's sum, natural order
         cpx<float>* acc = reinterpret_cast<cpx<float>*>(a.acc) + (long long)blockIdx.x * (N1 * N2);

@@ -329,6 +329,7 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
         }
         item = next;
     }
+    if (tid == 0) xc_done(a.counter, a.ticket);
     tc_fence_before();
     __syncthreads();
     if (tid < 32) tmem_dealloc(tbase, F::TCOLS);

@@ -37,7 +37,8 @@ struct xc_args {
     int           hwait;         // predecessors whose windows overlap this block's outputs
     unsigned      epoch;
     unsigned*     flags;
-    unsigned*     counter;
+    unsigned*     counter;       // work counter, zero outside a launch
+    unsigned*     ticket;        // blocks done claiming, likewise
     int*          error;
     const void*   kspec;         // K / N_fft, natural order, interleaved complex
 };
@@ -54,6 +55,18 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 }
 __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// One thread of a block that claims no more work: the last block of the launch
+// leaves the work counter (and the ticket it counts blocks with) zero for the
+// next one.
+__device__ __forceinline__ void xc_done(unsigned* counter, unsigned* ticket) {
+    __threadfence();
+    if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+        __threadfence();
+        *counter = 0u;
+        *ticket  = 0u;
+    }
 }
 
 constexpr unsigned long long XC_WAIT_NS = 1000000000ull;    // 1 s
@@ -108,7 +121,10 @@ __global__ void __launch_bounds__(M * splan<LOGN, EPT>::TT) k_fxcorr(xc_args a, 
         }
         __syncthreads();
         const long long item0 = s_item;
-        if (item0 >= a.total) break;
+        if (item0 >= a.total) {
+            if (tid == 0) xc_done(a.counter, a.ticket);
+            break;
+        }
         xc_load<T, L, NT>(buf, a, item0, M);
         __syncthreads();
         if (a.inplace && tid == 0) {
@@ -156,7 +172,10 @@ __global__ void __launch_bounds__(M * splan<LOGN, EPT>::TT) k_fxcorr(xc_args a, 
                 }
             }
             __syncthreads();
-            if (s_abort) return;    // every thread of the CTA leaves together
+            if (s_abort) {    // every thread of the CTA leaves together
+                if (tid == 0) xc_done(a.counter, a.ticket);
+                return;
+            }
         }
         if (item < a.total) {
             const long long ch  = item / a.nblk;
@@ -197,7 +216,8 @@ struct kg_args {
     int         step;
     int         nblk;
     long long   total;
-    unsigned*   counter;
+    unsigned*   counter;      // work counter, zero outside a launch
+    unsigned*   ticket;       // blocks done claiming, likewise
     void*       acc;          // [gridDim.x][N] complex
     void*       xspec;        // [gridDim.x][N] complex, per-CTA spectrum scratch
     int*        error;        // set when a bounded wait gave up (forms with bulk copies)
@@ -230,7 +250,10 @@ __global__ void __launch_bounds__(splan<LOGN, EPT>::TT) k_fxcorr_kgrad(kg_args a
         if (t == 0) s_item = (long long)atomicAdd(a.counter, 1u);
         __syncthreads();
         const long long item = s_item;
-        if (item >= a.total) break;
+        if (item >= a.total) {
+            if (t == 0) xc_done(a.counter, a.ticket);
+            break;
+        }
         // x window [b*step, b*step + N)
         xc_load<T, L, TT>(buf, la, item, 1);
         __syncthreads();

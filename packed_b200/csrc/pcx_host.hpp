@@ -154,7 +154,7 @@ struct pcx_plan_s {
     void*  fst2     = nullptr;
     pcxg::fs_choice fs{};         // one-launch four-step: the variant in use
     pcxg::fs_choice fs_def{};     // the size's default one, which the kernel's other forms run
-    int*   fs_ctr   = nullptr;    // its dependency counters, 2 per transform
+    int*   fs_ctr   = nullptr;    // a ticket and its dependency counters, 2 per transform
     size_t fs_ctr_n = 0;
     // form of the plan-owned-scratch path for n > 4096, set by pcx_plan_tune
     int    form        = 0;    // PCX_FORM_*: 0 built-in choice
