@@ -1,6 +1,5 @@
 // Host side of the overlap-save correlator: handle creation (kernel spectrum
 // computed on the device), the fused correlation launch and its adjoint.
-#include "pcx_fxcorr2d.cuh"
 #include "pcx_fxcorr3.cuh"
 #include "pcx_fxcorr_ip.cuh"
 #include "pcx_fxcorr_kernels.cuh"
@@ -32,13 +31,9 @@ struct pcx_fxcorr_s {
     int         sms            = 0;
     int         device         = 0;
     bool        x3             = false;      // FP32, N <= 2^12: pcx_fxcorr3.cuh (tables: plan->stwL)
-    // FP32, N = 2^13 or 2^14: three-step form (pcx_fxcorr_ip.cuh), kernel
-    // gradient in the in-CTA four-step form (pcx_fxcorr2d.cuh)
-    void*       x2d            = nullptr;    // one allocation: K permuted | twiddles | stage tables | twiddles
+    // FP32, N = 2^13 or 2^14: three-step form (pcx_fxcorr_ip.cuh)
+    void*       xi             = nullptr;    // one allocation: K in its order | twiddles
     const void* xi_tw          = nullptr;
-    const void* x2_stw1        = nullptr;
-    const void* x2_stw2        = nullptr;
-    const void* x2_tws         = nullptr;
     // for reuse (see handle_pool): created with PCX_XC_GENERAL; the last call's
     // end on its stream, unless calls went to several streams or into a capture
     bool         general = false;
@@ -174,15 +169,17 @@ int launch_xci(const xci_args& a, cudaStream_t st, int sms, bool attr_only) {
     return PCX_OK;
 }
 
+// grid: given a.acc == nullptr only returned (the rows of the accumulator)
 template<int LOGN>
-int launch_xc2_kg(const xc2_kg_args& a, cudaStream_t st, int grid, bool attr_only) {
-    using C   = xc2_cfg<LOGN>;
-    auto kern = k_fxcorr2d_kgrad<LOGN>;
-    if (attr_only) {
-        PCX_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-        return PCX_OK;
-    }
-    kern<<<(unsigned)grid, C::NT, C::SMEM, st>>>(a);
+int launch_xci_kg(const xci_kg_args& a, cudaStream_t st, int sms, int* grid) {
+    using C    = xci_cfg<LOGN>;
+    auto kern  = k_fxcorr_ip_kgrad<LOGN>;
+    int per_sm = 0;
+    PCX_CUDA_TRY(smem_attr_cached(reinterpret_cast<const void*>(kern), xci_kg_cfg<LOGN>::SMEM));
+    PCX_CUDA_TRY(occupancy_cached(reinterpret_cast<const void*>(kern), C::NT, xci_kg_cfg<LOGN>::SMEM, &per_sm));
+    *grid = (int)std::max<long long>(1, std::min<long long>(a.base.total, (long long)std::max(per_sm, 1) * sms));
+    if (!a.base.acc) return PCX_OK;
+    kern<<<(unsigned)*grid, C::NT, xci_kg_cfg<LOGN>::SMEM, st>>>(a);
     PCX_CUDA_TRY(cudaGetLastError());
     return PCX_OK;
 }
@@ -241,36 +238,17 @@ int dispatch_xc3_kg(int log_n, const kg_args& a, const void* stw, cudaStream_t s
     }
 }
 
-// Tables of the in-CTA four-step form; false when it does not apply.
+// Tables and launch attributes of the three-step form.
 template<int LOGN>
-int init_xc2(pcx_fxcorr_s* h) {
-    using C         = xc2_cfg<LOGN>;
-    int e1 = 0, e2 = 0;
-    // full stage tables of the two sub-transforms (one entry per twiddle)
-    PCX_CUDA_TRY(pcx_fourstep_tables(C::LOGN1, nullptr, false, 0, &e1));
-    PCX_CUDA_TRY(pcx_fourstep_tables(C::LOGN2, nullptr, false, 0, &e2));
-    e1                  = (e1 + 1) / 2 * 2;    // 16-byte sections
-    e2                  = (e2 + 1) / 2 * 2;
-    const size_t ntw    = (size_t)C::NB + C::N2 + C::N1;
-    const size_t entries = (size_t)C::N + xci_cfg<LOGN>::TABLE + e1 + e2 + ntw;
-    PCX_CUDA_TRY(cudaMalloc(&h->x2d, entries * sizeof(cpx<float>)));
-    auto* base   = static_cast<cpx<float>*>(h->x2d);
-    auto* xt     = base + C::N;
-    auto* s1     = xt + xci_cfg<LOGN>::TABLE;
-    k_xci_twiddles<<<(xci_cfg<LOGN>::TABLE + 255) / 256, 256>>>(xt, LOGN);
+int init_xci(pcx_fxcorr_s* h) {
+    using C = xci_cfg<LOGN>;
+    PCX_CUDA_TRY(cudaMalloc(&h->xi, (size_t)(C::N + C::TABLE) * sizeof(cpx<float>)));
+    auto* tw = static_cast<cpx<float>*>(h->xi) + C::N;
+    k_xci_twiddles<<<(C::TABLE + 255) / 256, 256>>>(tw, LOGN);
     PCX_CUDA_TRY(cudaGetLastError());
-    auto* s2     = s1 + e1;
-    auto* tws    = s2 + e2;
-    PCX_CUDA_TRY(pcx_fourstep_tables(C::LOGN1, s1, false, 0, &e1));
-    PCX_CUDA_TRY(pcx_fourstep_tables(C::LOGN2, s2, false, 0, &e2));
-    PCX_CUDA_TRY(pcx_gen_twiddles(tws, C::NB, LOGN, 1, false, 0));
-    PCX_CUDA_TRY(pcx_gen_twiddles(tws + C::NB, C::N2, LOGN, C::TT1, false, 0));
-    PCX_CUDA_TRY(pcx_gen_twiddles(tws + C::NB + C::N2, C::N1, LOGN, C::TT2, false, 0));
-    h->xi_tw    = xt;
-    h->x2_stw1  = s1;
-    h->x2_stw2  = s2;
-    h->x2_tws   = tws;
-    if (int rc = launch_xc2_kg<LOGN>(xc2_kg_args{}, 0, 0, true)) return rc;
+    h->xi_tw = tw;
+    int grid = 0;
+    if (int rc = launch_xci_kg<LOGN>(xci_kg_args{}, 0, h->sms, &grid)) return rc;
     return launch_xci<LOGN>(xci_args{}, 0, 0, true);
 }
 
@@ -351,11 +329,10 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     const bool rows = pack == 8 && a.in_shift % 8 == 0 && (channels == 1 || sstride % 4 == 0) &&
                       reinterpret_cast<uintptr_t>(src) % 16 == 0;
     if (h->x3 && rows) return dispatch_xc3(h->log_n, a, h->plan->stwL, st, h->sms);
-    const bool x2 = h->x2d && rows;
-    if (x2) {
+    if (h->xi && rows) {
         xci_args b{};
         b.base  = a;
-        b.kperm = h->x2d;
+        b.kperm = h->xi;
         b.tw    = h->xi_tw;
         return h->log_n == 14 ? launch_xci<14>(b, st, h->sms, false) : launch_xci<13>(b, st, h->sms, false);
     }
@@ -373,7 +350,7 @@ void free_handle(pcx_fxcorr_s* h) {
     if (h->kspec) cudaFree(h->kspec);
     if (h->ctl) cudaFree(h->ctl);
     if (h->gscratch) cudaFree(h->gscratch);
-    if (h->x2d) cudaFree(h->x2d);
+    if (h->xi) cudaFree(h->xi);
     if (h->done) cudaEventDestroy(h->done);
     delete h;
 }
@@ -467,9 +444,9 @@ int set_kernel(pcx_fxcorr_s* h, const void* g) {
                              (h->k + h->pack_g - 1) / h->pack_g * 2 * h->pack_g, nullptr, 0, 0, 1.0 / (double)h->n)) {
         return rc;
     }
-    if (h->x2d) {
+    if (h->xi) {
         k_xci_spectrum<<<(unsigned)(h->n / 256), 256>>>(static_cast<const cpx<float>*>(h->kspec),
-                                                       static_cast<cpx<float>*>(h->x2d), h->log_n);
+                                                       static_cast<cpx<float>*>(h->xi), h->log_n);
         PCX_CUDA_TRY(cudaGetLastError());
     }
     return PCX_OK;
@@ -501,7 +478,7 @@ int init_handle(pcx_fxcorr_s* h) {
         if (int rc = dispatch_xc3(log_n, xc_args{}, nullptr, 0, h->sms)) return rc;
         h->x3 = true;
     }
-    if (!f64 && log_n >= 13 && !h->general) return log_n == 14 ? init_xc2<14>(h) : init_xc2<13>(h);
+    if (!f64 && log_n >= 13 && !h->general) return log_n == 14 ? init_xci<14>(h) : init_xci<13>(h);
     return PCX_OK;
 }
 
@@ -630,19 +607,26 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
     const size_t total = nblk * channels;
     const size_t eb    = h->dtype == PCX_F64 ? 16 : 8;
     // FP32 at pack 8 on 16-byte aligned rows: the whole-window form up to
-    // 2^12 points, the in-CTA four-step form with the per-thread spectra in
-    // tensor memory at 2^13 and 2^14
+    // 2^12 points, the three-step form at 2^13 and 2^14
     const bool rows = pack == 8 && (channels == 1 || stride % 4 == 0) &&
                       (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gy)) % 16 == 0;
-    const bool x3 = h->x3 && rows, x2 = h->x2d && rows;
+    const bool x3 = h->x3 && rows, xi = h->xi && rows;
     kg_args    a{};
     a.total  = (long long)total;
     int grid = (int)std::min<size_t>(total, (size_t)h->sms);
+    const auto run_xci = [&]() -> int {
+        xci_kg_args b{};
+        b.base = a;
+        b.tw   = h->xi_tw;
+        return h->log_n == 14 ? launch_xci_kg<14>(b, st, h->sms, &grid) : launch_xci_kg<13>(b, st, h->sms, &grid);
+    };
     if (x3) {
         if (int rc = dispatch_xc3_kg(h->log_n, a, nullptr, st, h->sms, &grid)) return rc;
+    } else if (xi) {
+        if (int rc = run_xci()) return rc;
     }
     // sums of the blocks, the general form's spectra, the sum and its inverse
-    const size_t rows_s = (size_t)grid * (x3 || x2 ? 1 : 2);
+    const size_t rows_s = (size_t)grid * (x3 || xi ? 1 : 2);
     const size_t need   = (rows_s + 2) * n * eb;
     if (h->gscratch_bytes < need) {
         if (h->gscratch) cudaFree(h->gscratch);
@@ -670,13 +654,8 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
     int rc;
     if (x3) {
         rc = dispatch_xc3_kg(h->log_n, a, h->plan->stwL, st, h->sms, &grid);
-    } else if (x2) {
-        xc2_kg_args b{};
-        b.base = a;
-        b.stw1 = h->x2_stw1;
-        b.stw2 = h->x2_stw2;
-        b.tws  = h->x2_tws;
-        rc     = h->log_n == 14 ? launch_xc2_kg<14>(b, st, grid, false) : launch_xc2_kg<13>(b, st, grid, false);
+    } else if (xi) {
+        rc = run_xci();
     } else {
         rc = h->dtype == PCX_F64 ? dispatch_kg<double>(h->log_n, a, h->tw, st, grid, false)
                                  : dispatch_kg<float>(h->log_n, a, h->tw, st, grid, false);

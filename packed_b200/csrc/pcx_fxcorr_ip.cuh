@@ -335,4 +335,208 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
     if (tid < 32) tmem_dealloc(tbase, F::TCOLS);
 }
 
+// ---------------------------------------------------------------------------
+// Kernel gradient in the same form: per block the gy block (zero beyond its
+// outputs) and then the x window are transformed by the three forward steps.
+// A thread's 32 values of FFT(gy) and of the running sum of FFT(x) *
+// conj(FFT(gy)) fill its 128 words of tensor memory; its W_N^(ka(16b+c)) are
+// products of two of ten factors (u^1..u^3, u^4, u^8..u^28, u = W_N^(16b+c)) in
+// shared memory.  Both inputs land in the same window, the next one once the
+// last step has read its rows.  Blocks go round the launch, so the sums do not
+// depend on timing.  16 channels x 2^20, blocks of 16384 and 8192 points: 271 and
+// 318 us in the two-step form, 193 and 189 us.
+struct xci_kg_args {
+    kg_args     base;
+    const void* tw;    // k_xci_twiddles
+};
+
+template<int LOGN>
+struct xci_kg_cfg {
+    using F                   = xci_cfg<LOGN>;
+    static constexpr int UB   = 10 * F::NT * 8;    // factors of the first twiddle
+    static constexpr int SMEM = F::SMEM + UB;
+    static_assert(F::MINB * (SMEM + 1024 + 256) <= 233472, "blocks per SM");
+};
+
+template<int LOGN>
+__global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxcorr_ip_kgrad(xci_kg_args A) {
+    using F            = xci_cfg<LOGN>;
+    constexpr int N    = F::N;
+    constexpr int B    = F::B;
+    constexpr int NT   = F::NT;
+    constexpr int RL   = F::RL;
+    const kg_args& a   = A.base;
+    extern __shared__ __align__(128) unsigned char smem[];
+    cpx<float>*         win = reinterpret_cast<cpx<float>*>(smem);
+    float*              raw = reinterpret_cast<float*>(smem);
+    cpx<float>*         tw2 = reinterpret_cast<cpx<float>*>(smem + F::WIN);
+    cpx<float>*         uf  = tw2 + 16 * B;    // [10][NT]
+    __shared__ uint64_t full;
+    __shared__ uint32_t s_tmem;
+    const int           tid   = threadIdx.x;
+    const int           lane  = tid % 32;
+    const unsigned      total = (unsigned)a.total, nblk = (unsigned)a.nblk;    // < 2^31 (host check)
+    const cpx<float>*   tw    = reinterpret_cast<const cpx<float>*>(A.tw);
+
+    if (tid < 32) {
+        tmem_alloc(&s_tmem, F::TCOLS);
+        tmem_relinquish();
+    }
+    tw2[tid] = ldg_cpx(tw + N + tid);
+    static_for<10>([&](auto qc) {
+        constexpr int q   = decltype(qc)::value;
+        uf[q * NT + tid] = ldg_cpx(tw + (q < 3 ? q + 1 : 4 * (q - 2)) * NT + tid);    // row ka of the table: u^ka
+    });
+    if (tid == 0) {
+        mbar_init(&full, 1);
+        fence_barrier_init();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tbase = s_tmem;
+    const uint32_t tcol  = tbase + ((uint32_t)(32 * ((tid / 32) % 4)) << 16) + (uint32_t)(tid / 128) * 128;
+    {
+        uint32_t z[32];
+        static_for<32>([&](auto jc) { z[decltype(jc)::value] = 0u; });
+        tmem_st32(tcol + 64, z);
+        tmem_st32(tcol + 96, z);
+    }
+    // elements of input s (0: gy block, 1: x window) of an item that count
+    auto valid = [&](unsigned item, int s, long long& off) -> int {
+        const unsigned  ch = item / nblk;
+        const long long b  = (long long)(item - ch * nblk) * a.step;
+        off                = ch * a.stride + 2 * b;
+        return (int)min((long long)(s ? N : a.step), a.len - b);
+    };
+    // warp 0: the packed samples, in pieces of 32 KB
+    auto copy = [&](unsigned item, int s) {
+        if (item >= total) return;
+        long long      off;
+        const uint32_t bytes = (uint32_t)((valid(item, s, off) + 7) / 8) * 64;
+        if (lane == 0) mbar_arrive_expect_tx(&full, bytes);
+        __syncwarp();
+        const uint32_t q = lane * 32768u;
+        if (q < bytes) {
+            bulk_g2s(smem + q, reinterpret_cast<const char*>(reinterpret_cast<const float*>(s ? a.x : a.gy) + off) + q,
+                     min(32768u, bytes - q), &full);
+        }
+    };
+    if (tid < 32) copy(blockIdx.x, 0);
+
+    const int   c  = tid % 16;
+    cpx<float>* p1 = win + tid + 2 * (tid / 16);
+    cpx<float>* p2 = win + (tid / 16) * (B * RL) + c;
+    cpx<float>* p3 = win + tid * RL;
+    uint32_t    phase = 0;
+    bool        fail  = false;
+    for (unsigned item = blockIdx.x; item < total && !fail; item += gridDim.x) {
+        for (int s = 0; s < 2; ++s) {
+            long long  off;
+            const int  n  = valid(item, s, off);
+            const bool ok = mbar_wait_bounded(&full, phase);
+            cpx<float> v[32];
+            static_for<32>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                v[i]            = lds_swapped<float, 16>(raw, 2 * i * 16 * B + pk<3>(tid), 8);
+            });
+            if (n < N) {
+                static_for<32>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    if (i * 16 * B + tid >= n) v[i] = {0.f, 0.f};
+                });
+            }
+            if (__syncthreads_or(!ok)) {
+                // give up: record it and let the copies in flight land first
+                if (tid == 0) {
+                    atomicExch(a.error, 1);
+                    mbar_wait_bounded(&full, phase, 100000000ull);
+                }
+                fail = true;
+                break;
+            }
+            phase ^= 1;
+            dft<32, 1, 0>(v);
+            static_for<31>([&](auto ic) {
+                constexpr int i = decltype(ic)::value + 1, lo = i & 3, hi = i >> 2;
+                cpx<float>    w;
+                if constexpr (hi == 0) w = uf[(lo - 1) * NT + tid];
+                else if constexpr (lo == 0) w = uf[(2 + hi) * NT + tid];
+                else w = cmul(uf[(2 + hi) * NT + tid], uf[(lo - 1) * NT + tid]);
+                v[i] = cmul(v[i], w);
+            });
+            static_for<32>([&](auto ic) { p1[decltype(ic)::value * B * RL] = v[decltype(ic)::value]; });
+            __syncthreads();
+            static_for<32>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                v[i]            = p2[(i / B) * (NT / 16) * (B * RL) + (i % B) * RL];
+            });
+            xci_dft_b<B>(v);
+            static_for<32>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                p2[(i / B) * (NT / 16) * (B * RL) + (i % B) * RL] = i % B ? cmul(v[i], tw2[(i % B) * 16 + c]) : v[i];
+            });
+            __syncthreads();
+            static_for<16>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                const float4  x = *reinterpret_cast<const float4*>(p3 + (i / 8) * NT * RL + 2 * (i % 8));
+                v[2 * i]        = {x.x, x.y};
+                v[2 * i + 1]    = {x.z, x.w};
+            });
+            fence_proxy_async_smem();
+            __syncthreads();    // the window is read: the next input may land
+            if (tid < 32) copy(s ? item + gridDim.x : item, s ^ 1);
+            dft<16, 1, 0>(v);
+            dft<16, 1, 16>(v);
+            __syncwarp();
+            if (s == 0) {
+                static_for<2>([&](auto hc) {
+                    constexpr int h = decltype(hc)::value;
+                    uint32_t      r[32];
+                    static_for<16>([&](auto jc) {
+                        constexpr int j = decltype(jc)::value;
+                        r[2 * j]        = __float_as_uint(v[16 * h + j].re);
+                        r[2 * j + 1]    = __float_as_uint(v[16 * h + j].im);
+                    });
+                    tmem_st32(tcol + 32 * h, r);
+                });
+            } else {
+                // sum += X * conj(GY), eight values at a time
+                static_for<4>([&](auto hc) {
+                    constexpr int h = decltype(hc)::value;
+                    uint32_t      gq[16], sq[16];
+                    tmem_ld16(tcol + 16 * h, gq);
+                    tmem_ld16(tcol + 64 + 16 * h, sq);
+                    static_for<8>([&](auto jc) {
+                        constexpr int    j = decltype(jc)::value;
+                        const cpx<float> p = cmulc(v[8 * h + j], cpx<float>{__uint_as_float(gq[2 * j]),
+                                                                             __uint_as_float(gq[2 * j + 1])});
+                        sq[2 * j]          = __float_as_uint(__uint_as_float(sq[2 * j]) + p.re);
+                        sq[2 * j + 1]      = __float_as_uint(__uint_as_float(sq[2 * j + 1]) + p.im);
+                    });
+                    tmem_st16(tcol + 64 + 16 * h, sq);
+                });
+            }
+        }
+    }
+    if (!fail) {
+        // this block's sums in natural order: k = ka + 32*kb + 32B*kc, row r = ka*B + kb
+        cpx<float>* acc = reinterpret_cast<cpx<float>*>(a.acc) + (long long)blockIdx.x * N;
+        __syncwarp();
+        static_for<2>([&](auto hc) {
+            constexpr int h = decltype(hc)::value;
+            uint32_t      sq[32];
+            tmem_ld32(tcol + 64 + 32 * h, sq);
+            const int r = tid + h * NT;
+            static_for<16>([&](auto jc) {
+                constexpr int kc                           = decltype(jc)::value;
+                acc[r / B + 32 * (r % B) + 32 * B * kc] = {__uint_as_float(sq[2 * kc]), __uint_as_float(sq[2 * kc + 1])};
+            });
+        });
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (tid < 32) tmem_dealloc(tbase, F::TCOLS);
+}
+
 }    // namespace pcxg
