@@ -157,13 +157,11 @@ namespace {
 
 template<int LOGN>
 int launch_xci(const xci_args& a, cudaStream_t st, int sms, bool attr_only) {
-    using C    = xci_cfg<LOGN>;
-    auto kern  = k_fxcorr_ip<LOGN>;
-    int per_sm = 0;
+    using C   = xci_cfg<LOGN>;
+    auto kern = k_fxcorr_ip<LOGN>;
     PCX_CUDA_TRY(smem_attr_cached(reinterpret_cast<const void*>(kern), C::SMEM));
-    PCX_CUDA_TRY(occupancy_cached(reinterpret_cast<const void*>(kern), C::NT, C::SMEM, &per_sm));
     if (attr_only) return PCX_OK;
-    const long long grid = std::max<long long>(1, std::min<long long>(a.base.total, (long long)std::max(per_sm, 1) * sms));
+    const long long grid = std::max<long long>(1, std::min<long long>(a.base.total, (long long)C::MINB * sms));
     kern<<<(unsigned)grid, C::NT, C::SMEM, st>>>(a);
     PCX_CUDA_TRY(cudaGetLastError());
     return PCX_OK;
@@ -172,12 +170,10 @@ int launch_xci(const xci_args& a, cudaStream_t st, int sms, bool attr_only) {
 // grid: given a.acc == nullptr only returned (the rows of the accumulator)
 template<int LOGN>
 int launch_xci_kg(const xci_kg_args& a, cudaStream_t st, int sms, int* grid) {
-    using C    = xci_cfg<LOGN>;
-    auto kern  = k_fxcorr_ip_kgrad<LOGN>;
-    int per_sm = 0;
+    using C   = xci_cfg<LOGN>;
+    auto kern = k_fxcorr_ip_kgrad<LOGN>;
     PCX_CUDA_TRY(smem_attr_cached(reinterpret_cast<const void*>(kern), xci_kg_cfg<LOGN>::SMEM));
-    PCX_CUDA_TRY(occupancy_cached(reinterpret_cast<const void*>(kern), C::NT, xci_kg_cfg<LOGN>::SMEM, &per_sm));
-    *grid = (int)std::max<long long>(1, std::min<long long>(a.base.total, (long long)std::max(per_sm, 1) * sms));
+    *grid = (int)std::max<long long>(1, std::min<long long>(a.base.total, (long long)C::MINB * sms));
     if (!a.base.acc) return PCX_OK;
     kern<<<(unsigned)*grid, C::NT, xci_kg_cfg<LOGN>::SMEM, st>>>(a);
     PCX_CUDA_TRY(cudaGetLastError());
@@ -185,14 +181,17 @@ int launch_xci_kg(const xci_kg_args& a, cudaStream_t st, int sms, int* grid) {
 }
 
 // The whole-window form (pcx_fxcorr3.cuh): blocks of a launch over `total` windows.
+// Two blocks per SM by shared memory and registers (xc3_cfg); the occupancy
+// query answers one for a kernel that allocates tensor memory, whatever it
+// needs of the 512 columns (64 and 128 here).  Out of place, one block an SM and
+// two: 4096 points, 16 x 250008 samples, 504 taps 41.7 and 35.4 us, 32 x 2^20,
+// 1024 taps 335 and 265 us; 1024 points, 32 x 250000, 250 taps 89 and 73 us.
 template<int LOGN, class K>
 int grid_xc3(K kern, long long total, int sms, int* grid) {
-    using C    = xc3_cfg<LOGN>;
-    int per_sm = 0;
+    using C = xc3_cfg<LOGN>;
     PCX_CUDA_TRY(smem_attr_cached(reinterpret_cast<const void*>(kern), C::SMEM));
-    PCX_CUDA_TRY(occupancy_cached(reinterpret_cast<const void*>(kern), C::NT, C::SMEM, &per_sm));
     const long long tiles = (total + C::M - 1) / C::M;
-    *grid = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)std::max(per_sm, 1) * sms));
+    *grid = (int)std::max<long long>(1, std::min<long long>(tiles, 2LL * sms));
     return PCX_OK;
 }
 template<int LOGN>
@@ -662,10 +661,10 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
     }
     if (rc) return rc;
     if (h->dtype == PCX_F64) {
-        k_kgrad_reduce<double><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
+        k_kgrad_reduce<double><<<(unsigned)((n + 15) / 16), 256, 0, st>>>(
             static_cast<const cpx<double>*>(a.acc), grid, (int)n, static_cast<cpx<double>*>(sum));
     } else {
-        k_kgrad_reduce<float><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
+        k_kgrad_reduce<float><<<(unsigned)((n + 15) / 16), 256, 0, st>>>(
             static_cast<const cpx<float>*>(a.acc), grid, (int)n, static_cast<cpx<float>*>(sum));
     }
     PCX_CUDA_TRY(cudaGetLastError());

@@ -16,8 +16,8 @@
 // would be, against 16 bytes of HBM per sample.  16 channels x 250008 samples,
 // 504 taps, 4096-point windows: the general kernel (plain loads, no copy in
 // flight during a block, sub-transform twiddles and kernel spectrum from
-// global memory) 98 us, this one 41 us; kernel gradient 182 and
-// 40 us (device times).
+// global memory) 98 us, this one 34 us; kernel gradient 182 and
+// 34 us (device times).
 //
 // In place, a tile's outputs overwrite samples that the windows of earlier
 // tiles still read, so tiles are claimed in order from a counter, a block

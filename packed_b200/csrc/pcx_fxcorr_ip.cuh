@@ -24,7 +24,7 @@
 // the next one as soon as the last step has read this one.
 // Bound by issue and the shared-memory pipe.  32 channels x 2^20 samples, 4096
 // taps, in place: 395 us with the two-step form, 260 us; relative error against
-// FP64 4.0e-7 and 2.8e-7.  8192 points, 16 x 2^20, 2048 taps: 220 and 140 us.
+// FP64 4.0e-7 and 2.8e-7.  8192 points, 16 x 2^20, 2048 taps: 220 and 115 us.
 //
 // In place, a window's outputs overwrite samples that earlier blocks' windows
 // read: blocks are claimed in order, each publishes "window loaded" (the call's
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
 // shared memory.  Both inputs land in the same window, the next one once the
 // last step has read its rows.  Blocks go round the launch, so the sums do not
 // depend on timing.  16 channels x 2^20, blocks of 16384 and 8192 points: 271 and
-// 318 us in the two-step form, 193 and 189 us.
+// 318 us in the two-step form, 190 and 157 us.
 struct xci_kg_args {
     kg_args     base;
     const void* tw;    // k_xci_twiddles

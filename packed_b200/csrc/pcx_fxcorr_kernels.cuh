@@ -301,25 +301,25 @@ __global__ void __launch_bounds__(splan<LOGN, EPT>::TT) k_fxcorr_kgrad(kg_args a
     }
 }
 
-// Sum the per-CTA spectra: 32 frequencies per block of 256 threads, every
-// eighth CTA per thread, so that a sum is a chain of ctas / 8 loads and the
-// whole chip takes part (4096 points, 148 CTAs: one thread per frequency in 16
-// blocks took 9.2 us, this 5.2).
+// Sum the per-CTA spectra: 16 frequencies per block of 256 threads, every
+// sixteenth CTA per thread, so that a sum is a chain of ctas / 16 loads and the
+// whole chip takes part (4096 points: one thread per frequency in 16 blocks
+// took 9.2 us for 148 CTAs, this 4.1 for 296).
 template<class T>
 __global__ void __launch_bounds__(256) k_kgrad_reduce(const cpx<T>* __restrict__ acc, int ctas, int n,
                                                       cpx<T>* __restrict__ out) {
-    __shared__ cpx<T> part[8][32];
-    const int         x = threadIdx.x % 32, y = threadIdx.x / 32;
-    const int         k = blockIdx.x * 32 + x;
+    __shared__ cpx<T> part[16][16];
+    const int         x = threadIdx.x % 16, y = threadIdx.x / 16;
+    const int         k = blockIdx.x * 16 + x;
     cpx<T>            s = {T(0), T(0)};
     if (k < n) {
-#pragma unroll 4
-        for (int c = y; c < ctas; c += 8) s = s + acc[(long long)c * n + k];
+#pragma unroll 8
+        for (int c = y; c < ctas; c += 16) s = s + acc[(long long)c * n + k];
     }
     part[y][x] = s;
     __syncthreads();
     if (y == 0 && k < n) {
-        for (int j = 1; j < 8; ++j) s = s + part[j][x];
+        for (int j = 1; j < 16; ++j) s = s + part[j][x];
         out[k] = s;
     }
 }
