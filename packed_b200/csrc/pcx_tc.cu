@@ -649,74 +649,57 @@ __device__ __forceinline__ bool tcp_run(const tcp_args& a, int rows, const float
         }
     };
     load_f(1 << R0B);
-    // rows in natural order (conjugated for the inverse); missing rows are
-    // zero.  Two 8-point packs per thread, all loads first.
-    static_assert(T * N / 8 == 2 * TP_NT, "two packs per thread");
-    {
-        float4 v[2][4];
-        static_for<2>([&](auto uc) {
-            constexpr int u   = decltype(uc)::value;
-            const int     q   = tid + u * TP_NT;
-            const int     r   = q / (N / 8), pk8 = q % (N / 8);
-            v[u][0] = v[u][1] = v[u][2] = v[u][3] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < rows) {
-                const float4* s = reinterpret_cast<const float4*>(s_src[r] + pk8 * 16);
-                static_for<4>([&](auto hc) { v[u][decltype(hc)::value] = __ldg(s + decltype(hc)::value); });
-            }
+    // this thread's row, read before the first barrier (the next item's rows
+    // are written after the last one)
+    const float* src_row = tr < rows ? s_src[tr] : nullptr;
+    float*       dst_row = tr < rows ? s_dst[tr] : nullptr;
+    // element e of a row in natural order, conjugated for the inverse; zeros for a missing row
+    auto in = [&](const float* row, int e) -> cpx<float> {
+        if (!row) return {0.f, 0.f};
+        return {__ldg(row + pk<3>(e)), cj * __ldg(row + pk<3>(e) + 8)};
+    };
+    cpx<float> x[16];
+    if constexpr (R0B == 0) {
+        static_for<16>([&](auto jc) {
+            constexpr int j = decltype(jc)::value;
+            x[j]            = in(src_row, bl + j * (N / 16));
         });
-        static_for<2>([&](auto uc) {
-            constexpr int u   = decltype(uc)::value;
-            const int     q   = tid + u * TP_NT;
-            const int     r   = q / (N / 8), pk8 = q % (N / 8);
-            const float4 &r0 = v[u][0], &r1 = v[u][1], &i0 = v[u][2], &i1 = v[u][3];
-            float4*       w   = reinterpret_cast<float4*>(work + tcp_wp(r * N + pk8 * 8));    // 8 contiguous elements
-            w[0]              = make_float4(r0.x, cj * i0.x, r0.y, cj * i0.y);
-            w[1]              = make_float4(r0.z, cj * i0.z, r0.w, cj * i0.w);
-            w[2]              = make_float4(r1.x, cj * i1.x, r1.y, cj * i1.y);
-            w[3]              = make_float4(r1.z, cj * i1.z, r1.w, cj * i1.w);
-        });
-    }
-    __syncthreads();
-    int ns = 1;
-    // remainder stage (radix 2, 4 or 8) on the CUDA cores, in place
-    if constexpr (R0B > 0) {
+    } else {
+        // remainder stage (radix 2, 4 or 8) on the CUDA cores, into the work buffer
         constexpr int R = 1 << R0B;
         constexpr int U = 16 / R;    // butterflies per thread
-        cpx<float>    x[16];
         static_for<U>([&](auto uc) {
             constexpr int u  = decltype(uc)::value;
             const int     b  = tid + u * TP_NT;
-            const int     tr = b / (N / R), bl = b % (N / R);
+            const int     r  = b / (N / R);
+            const float*  g  = r < rows ? s_src[r] : nullptr;
             static_for<R>([&](auto jc) {
                 constexpr int j = decltype(jc)::value;
-                x[u * R + j]    = work[tcp_wp(tr * N + bl + j * (N / R))];
+                x[u * R + j]    = in(g, b % (N / R) + j * (N / R));
             });
         });
-        __syncthreads();
         static_for<U>([&](auto uc) {
-            constexpr int u  = decltype(uc)::value;
-            const int     b  = tid + u * TP_NT;
-            const int     tr = b / (N / R), bl = b % (N / R);
+            constexpr int u = decltype(uc)::value;
+            const int     b = tid + u * TP_NT;
             dft<R, 1, u * R>(x);
             static_for<R>([&](auto jc) {
-                constexpr int j                     = decltype(jc)::value;
-                work[tcp_wp(tr * N + bl * R + j)] = x[u * R + j];
+                constexpr int j                                                  = decltype(jc)::value;
+                work[tcp_wp((b / (N / R)) * N + (b % (N / R)) * R + j)] = x[u * R + j];
             });
         });
-        ns = R;
         __syncthreads();
     }
-    for (int st = 0; st < NTC; ++st) {
-        const int  k = bl & (ns - 1);
-        cpx<float> x[16];
+    // a radix-16 stage; false when the products did not come
+    auto stage = [&](auto stc) -> bool {
+        constexpr int  st   = decltype(stc)::value;
+        constexpr int  ns   = 1 << (R0B + 4 * st);
+        constexpr bool LAST = st == NTC - 1;
+        const int      k    = bl & (ns - 1);
         // twiddle j of the butterfly: W_{16 ns}^(jk), from the six factors
         static_for<16>([&](auto jc) {
             constexpr int j = decltype(jc)::value;
-            cpx<float>    v = work[tcp_wp(tr * N + bl + j * (N / 16))];
-            if constexpr (j > 0) {
-                if (ns > 1) v = cmul(v, stw_factor<4, j>(fn));
-            }
-            x[j] = v;
+            if constexpr (R0B > 0 || st > 0) x[j] = work[tcp_wp(tr * N + bl + j * (N / 16))];
+            if constexpr (j > 0 && ns > 1) x[j] = cmul(x[j], stw_factor<4, j>(fn));
         });
         // operand row tid (reals 0..15 then imaginaries 16..31) into this
         // thread's tensor-memory lane, four columns at a time
@@ -774,7 +757,7 @@ __device__ __forceinline__ bool tcp_run(const tcp_args& a, int rows, const float
             });
             umma_commit(mbar);
         }
-        if (st + 1 < NTC) load_f(ns * 16);
+        if constexpr (!LAST) load_f(ns * 16);
         const bool ok = mbar_wait_bounded(mbar, phase);
         if (__syncthreads_or(!ok)) {
             // give up: record it and let the products in flight finish before TMEM is freed
@@ -788,43 +771,46 @@ __device__ __forceinline__ bool tcp_run(const tcp_args& a, int rows, const float
         tc_fence_after();
         uint32_t r[32];
         tmem_ld32(taddr + ((uint32_t)(32 * (warp % 4)) << 16) + 32 * (warp / 4), r);
-        // outputs of this butterfly, Stockham placement, in place
-        const int base = tr * N + (bl / ns) * ns * 16 + k;
-        if (ns == 1) {
-            // sixteen contiguous outputs: eight 16-byte stores
-            float4* w = reinterpret_cast<float4*>(work + tcp_wp(base));
-            static_for<8>([&](auto jc) {
-                constexpr int j = decltype(jc)::value;
-                w[j]            = make_float4(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 16]),
-                                              __uint_as_float(r[2 * j + 1]), __uint_as_float(r[2 * j + 17]));
-            });
+        if constexpr (LAST) {
+            // frequencies bl + j*N/16 of the row, natural order out (conjugated and scaled for the inverse)
+            const float sc = a.scale, sim = a.conj ? -a.scale : a.scale;
+            if (dst_row) {
+                static_for<16>([&](auto jc) {
+                    constexpr int j = decltype(jc)::value;
+                    __stcs(dst_row + pk<3>(bl + j * (N / 16)), __uint_as_float(r[j]) * sc);
+                    __stcs(dst_row + pk<3>(bl + j * (N / 16)) + 8, __uint_as_float(r[j + 16]) * sim);
+                });
+            }
+            // the next products, and the next use of the work buffer, lie
+            // behind barriers that this thread reaches with its reads done
+            tc_fence_before();
         } else {
-            static_for<16>([&](auto jc) {
-                constexpr int j                = decltype(jc)::value;
-                work[tcp_wp(base + j * ns)] = {__uint_as_float(r[j]), __uint_as_float(r[j + 16])};
-            });
+            // outputs of this butterfly, Stockham placement, in place
+            const int base = tr * N + (bl / ns) * ns * 16 + k;
+            if constexpr (ns == 1) {
+                // sixteen contiguous outputs: eight 16-byte stores
+                float4* w = reinterpret_cast<float4*>(work + tcp_wp(base));
+                static_for<8>([&](auto jc) {
+                    constexpr int j = decltype(jc)::value;
+                    w[j]            = make_float4(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 16]),
+                                                  __uint_as_float(r[2 * j + 1]), __uint_as_float(r[2 * j + 17]));
+                });
+            } else {
+                static_for<16>([&](auto jc) {
+                    constexpr int j                = decltype(jc)::value;
+                    work[tcp_wp(base + j * ns)] = {__uint_as_float(r[j]), __uint_as_float(r[j + 16])};
+                });
+            }
+            tc_fence_before();
+            __syncthreads();    // operands, accumulator and work free for the next stage
         }
-        tc_fence_before();
-        __syncthreads();    // operands, accumulator and work free for the next stage
-        ns *= 16;
-    }
-    // natural order out (conjugated and scaled for the inverse)
-    const float sc = a.scale, sim = a.conj ? -a.scale : a.scale;
-    static_for<2>([&](auto uc) {
-        const int q = tid + decltype(uc)::value * TP_NT;
-        const int r = q / (N / 8), pk8 = q % (N / 8);
-        if (r < rows) {
-            const float4* w  = reinterpret_cast<const float4*>(work + tcp_wp(r * N + pk8 * 8));
-            const float4  w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
-            float4*       d  = reinterpret_cast<float4*>(s_dst[r] + pk8 * 16);
-            d[0]             = make_float4(w0.x * sc, w0.z * sc, w1.x * sc, w1.z * sc);
-            d[1]             = make_float4(w2.x * sc, w2.z * sc, w3.x * sc, w3.z * sc);
-            d[2]             = make_float4(w0.y * sim, w0.w * sim, w1.y * sim, w1.w * sim);
-            d[3]             = make_float4(w2.y * sim, w2.w * sim, w3.y * sim, w3.w * sim);
-        }
+        return true;
+    };
+    bool done = true;
+    static_for<NTC>([&](auto stc) {
+        if (done) done = stage(stc);
     });
-    __syncthreads();    // the work buffer and row pointers are free for the next item
-    return true;
+    return done;
 }
 
 template<int PREC>
