@@ -668,16 +668,50 @@ __device__ __forceinline__ bool tcp_run(const tcp_args& a, int rows, const float
         // remainder stage (radix 2, 4 or 8) on the CUDA cores, into the work buffer
         constexpr int R = 1 << R0B;
         constexpr int U = 16 / R;    // butterflies per thread
-        static_for<U>([&](auto uc) {
-            constexpr int u  = decltype(uc)::value;
-            const int     b  = tid + u * TP_NT;
-            const int     r  = b / (N / R);
-            const float*  g  = r < rows ? s_src[r] : nullptr;
-            static_for<R>([&](auto jc) {
-                constexpr int j = decltype(jc)::value;
-                x[u * R + j]    = in(g, b % (N / R) + j * (N / R));
+        if constexpr (R0B <= 2) {
+            // 512 and 1024 points: eight or four butterflies from as many rows a
+            // thread, whose 32 loads of 4 bytes
+            // cost more than a copy in 16-byte units through the work buffer
+            // (bf16 x6, 2^24 points: 152 and 128 us, this way 111 and 111)
+            float4 v[2][4];
+            static_for<2>([&](auto uc) {
+                constexpr int u = decltype(uc)::value;
+                const int     q = tid + u * TP_NT, r = q / (N / 8), pk8 = q % (N / 8);
+                v[u][0] = v[u][1] = v[u][2] = v[u][3] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < rows) {
+                    const float4* g = reinterpret_cast<const float4*>(s_src[r] + pk8 * 16);
+                    static_for<4>([&](auto hc) { v[u][decltype(hc)::value] = __ldg(g + decltype(hc)::value); });
+                }
             });
-        });
+            static_for<2>([&](auto uc) {
+                constexpr int u = decltype(uc)::value;
+                const int     q = tid + u * TP_NT, r = q / (N / 8), pk8 = q % (N / 8);
+                const float4 &r0 = v[u][0], &r1 = v[u][1], &i0 = v[u][2], &i1 = v[u][3];
+                float4*       w  = reinterpret_cast<float4*>(work + tcp_wp(r * N + pk8 * 8));    // 8 contiguous elements
+                w[0]             = make_float4(r0.x, cj * i0.x, r0.y, cj * i0.y);
+                w[1]             = make_float4(r0.z, cj * i0.z, r0.w, cj * i0.w);
+                w[2]             = make_float4(r1.x, cj * i1.x, r1.y, cj * i1.y);
+                w[3]             = make_float4(r1.z, cj * i1.z, r1.w, cj * i1.w);
+            });
+            __syncthreads();
+            static_for<16>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                const int     b = tid + (i / R) * TP_NT;
+                x[i]            = work[tcp_wp((b / (N / R)) * N + b % (N / R) + (i % R) * (N / R))];
+            });
+            __syncthreads();
+        } else {
+            static_for<U>([&](auto uc) {
+                constexpr int u  = decltype(uc)::value;
+                const int     b  = tid + u * TP_NT;
+                const int     r  = b / (N / R);
+                const float*  g  = r < rows ? s_src[r] : nullptr;
+                static_for<R>([&](auto jc) {
+                    constexpr int j = decltype(jc)::value;
+                    x[u * R + j]    = in(g, b % (N / R) + j * (N / R));
+                });
+            });
+        }
         static_for<U>([&](auto uc) {
             constexpr int u = decltype(uc)::value;
             const int     b = tid + u * TP_NT;
