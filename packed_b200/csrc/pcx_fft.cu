@@ -957,10 +957,9 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
             if (p->fs_ctr) cudaFree(p->fs_ctr);
             p->fs_ctr   = nullptr;
             p->fs_ctr_n = 0;
-            PCX_CUDA_TRY(cudaMalloc(&p->fs_ctr, (2 * batch + 1) * sizeof(int)));
+            // every launch leaves them zero
+            PCX_CUDA_TRY(alloc_zeroed(reinterpret_cast<void**>(&p->fs_ctr), (2 * batch + 1) * sizeof(int)));
             p->fs_ctr_n = 2 * batch;
-            // from here on every launch leaves them zero
-            PCX_CUDA_TRY(cudaMemsetAsync(p->fs_ctr, 0, (2 * batch + 1) * sizeof(int), st));
         }
         fs_args a{};
         a.src        = src;

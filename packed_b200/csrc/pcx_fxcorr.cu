@@ -264,8 +264,7 @@ int ensure_flags(pcx_fxcorr_s* h, size_t items) {
     h->ctl       = nullptr;
     h->flags_cap = 0;
     const size_t cap = std::max<size_t>(items, 1024);
-    PCX_CUDA_TRY(cudaMalloc(&h->ctl, (cap + 3) * sizeof(unsigned)));
-    PCX_CUDA_TRY(cudaMemset(h->ctl, 0, (cap + 3) * sizeof(unsigned)));
+    PCX_CUDA_TRY(alloc_zeroed(reinterpret_cast<void**>(&h->ctl), (cap + 3) * sizeof(unsigned)));
     h->flags_cap = cap;
     h->epoch     = 0;
     return PCX_OK;

@@ -53,6 +53,24 @@ inline cudaError_t smem_attr_cached(const void* kern, int bytes) {
     return e;
 }
 
+// Zeroed device memory for counters that every launch leaves zero.  Filled and
+// waited for on a stream of its own: on the caller's stream the fill could
+// become part of a capture that is never replayed, and on the default one a
+// launch on another stream could overtake it.
+inline cudaError_t alloc_zeroed(void** out, size_t bytes) {
+    void*        p = nullptr;
+    cudaStream_t s = nullptr;
+    cudaError_t  e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess) return e;
+    e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, bytes, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (s) cudaStreamDestroy(s);
+    if (e == cudaSuccess) *out = p;
+    else cudaFree(p);
+    return e;
+}
+
 struct v2_args;
 struct v3_args;
 
