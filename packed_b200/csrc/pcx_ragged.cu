@@ -170,7 +170,8 @@ struct args {
 
 // What the compute warps need of the item in each stage, filled by the
 // producer while earlier items are computed, so that no chain of dependent
-// global loads opens an item.
+// global loads opens an item.  It is the next item's as soon as the last warp
+// has released the stage: a warp reads what it needs of it before it does that.
 struct stage_meta {
     item   it;
     xc_req xq;    // XR, XC: the correlation request
@@ -281,13 +282,14 @@ __device__ __forceinline__ bool single_items(const args& A, const stage_meta& mt
     // also votes on `bad`
     if (bar1_any<NT>(bad)) return false;
     run_stages_tab<P, typename G::X, false, NT>(v, reinterpret_cast<cpx<float>*>(buf), m, t, stw);
+    const int first = it.a, count = it.b;
     fence_proxy_async_smem();    // the stage is read: it may be refilled
     __syncwarp();
     if (tid % 32 == 0) mbar_arrive(empty_bar);
-    if (m < it.b) {
+    if (m < count) {
         // element t + i*TT; its packed offset splits into a base and a
         // constant only when TT is a multiple of the pack width
-        float*      d  = A.req[it.a + m].dst;
+        float*      d  = A.req[first + m].dst;
         const float sc = s_scale, sim = conj ? -sc : sc;
         static_for<E>([&](auto ic) {
             constexpr int i = decltype(ic)::value;
@@ -371,10 +373,10 @@ __device__ __forceinline__ bool row_item(const stage_meta& mt, unsigned char* bu
                                                                    bad)) {
         return false;
     }
+    float* dst = const_cast<float*>(static_cast<const float*>(mt.it.p0)) + pk<LPK>(t * N1 + k1);
     fence_proxy_async_smem();
     __syncwarp();
     if (tid % 32 == 0) mbar_arrive(empty_bar);
-    float*      dst = const_cast<float*>(static_cast<const float*>(mt.it.p0)) + pk<LPK>(t * N1 + k1);
     const float sc = s_scale, sim = s_conj ? -sc : sc;
     static_for<E>([&](auto ic) {
         constexpr int i = decltype(ic)::value;
@@ -678,11 +680,11 @@ __device__ __noinline__ bool xrw_window(const args& A, const stage_meta& mt, uns
         });
         stage_compute_tab<P1, 0>(v, t, tw1);
         run_stages_full<P1, XC, true, -1>(v, col, n2, t, tw1);
+        float* drow = q.dst + 2 * b0 + 2 * t * N2 + ((n2 >> 3) << 4) + (n2 & 7);
         // the windows are read: the stage may be refilled while the outputs go out
         fence_proxy_async_smem();
         __syncwarp();
         if (tid % 32 == 0) mbar_arrive(empty_bar);
-        float* drow = q.dst + 2 * b0 + 2 * t * N2 + ((n2 >> 3) << 4) + (n2 & 7);
         static_for<E>([&](auto ic) {
             constexpr int i = decltype(ic)::value;
             if ((t + i * TT1) * N2 + n2 < hi) {
@@ -740,14 +742,15 @@ __device__ __noinline__ bool xr_items(const args& A, const stage_meta& mt, unsig
     });
     stage_compute_tab<P, 0>(v, t, fst);
     run_stages_full<P, typename G::X, TS, NT, PT>(v, xch, m, t, fst);
+    // outputs t + i*TT < min(step, samples left), none past the item (lim is 0
+    // there); the window starts on a whole pack, so the packed offset is a base
+    // plus a constant
+    const int olim = lim < q.step ? lim : q.step;
+    float*    d    = q.dst + 2 * b0 + pk<LPK>(t);
     fence_proxy_async_smem();    // the stage is read: it may be refilled
     __syncwarp();
     if (tid % 32 == 0) mbar_arrive(empty_bar);
-    if (m < it.c) {
-        // outputs t + i*TT < min(step, samples left); the window starts on a
-        // whole pack, so the packed offset is a base plus a constant
-        const int olim = lim < q.step ? lim : q.step;
-        float*    d    = q.dst + 2 * b0 + pk<LPK>(t);
+    if (olim > 0) {
         static_for<E>([&](auto ic) {
             constexpr int i = decltype(ic)::value;
             if (t + i * TT < olim) {
@@ -762,12 +765,17 @@ __device__ __noinline__ bool xr_items(const args& A, const stage_meta& mt, unsig
 // ---------------------------------------------------------------- producer
 // Bytes and copies of an item into stage `buf` (lane 0 registers the bytes
 // on `bar` first; the lanes issue the copies).  XC items copy nothing.
+// The tensor maps are in global memory that an earlier batch's may have been
+// in: `seen` is the map that this block acquired for the tensor-map proxy last.
 template<int L1, int L2>
-__device__ void issue_col(const args& A, const item& it, unsigned char* buf, uint64_t* bar, int lane, uint64_t pol) {
+__device__ void issue_col(const args& A, const item& it, unsigned char* buf, uint64_t* bar, int lane, uint64_t pol,
+                          int& seen) {
     using F = fsg<L1, L2>;
     if (lane == 0) {
         mbar_arrive_expect_tx(bar, F::N1 * F::SEG * 4);
         const CUtensorMap* map = A.tmaps + it.tmap;
+        if (seen != it.tmap) fence_tensormap_acquire(map);
+        seen = it.tmap;
 #pragma unroll
         for (int y = 0; y < F::N1; y += F::BOXY) {
             tma_load_3d_hint(buf + y * F::SEG * 4, map, 2 * it.b * F::C, y, it.tz, bar, pol);
@@ -1058,6 +1066,7 @@ __global__ void __launch_bounds__(NT + 64, 1) k_ragged(const args* __restrict__ 
         const uint64_t pol    = l2_evict_first_policy();
         bool           fail   = false;
         long long      issued = 0;
+        int            seen   = -1;
         long long      drain_until = -1;    // after an XC item: wait for it before the next item
         auto           wait_empty = [&](long long q) -> bool {    // stage of item q released
             int ok = 1;
@@ -1142,7 +1151,7 @@ __global__ void __launch_bounds__(NT + 64, 1) k_ragged(const args* __restrict__ 
             } else if (it.kind == K_COL) {
                 switch (it.lg) {
 #define PCX_RG_ISSUE_C(LG, A1, A2) \
-    case LG: issue_col<A1, A2>(A, it, buf, &s_full[s], lane, pol); break;
+    case LG: issue_col<A1, A2>(A, it, buf, &s_full[s], lane, pol, seen); break;
                     PCX_RG_FOURSTEP(PCX_RG_ISSUE_C)
 #undef PCX_RG_ISSUE_C
                 default: break;
