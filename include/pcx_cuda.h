@@ -279,6 +279,8 @@ int pcx_fft_vjp(pcx_plan plan, void* g_in, const void* g_out, int pack, int dire
  * (reference fxcorr.hpp:62-92): g is a DEVICE pointer to k elements at pack
  * width pack_g; kernel spectrum K = FFT(g zero-padded to n_fft) / n_fft is
  * computed on the device.  Requires k <= n_fft - pack + 1 so that step > 0.
+ * Waits for the device before it reads g (which may have been written on any
+ * stream) and until g has been read.
  */
 int pcx_fxcorr_create(pcx_fxcorr* h, const void* g, size_t k, int pack_g, size_t n_fft, int dtype);
 int pcx_fxcorr_destroy(pcx_fxcorr h);

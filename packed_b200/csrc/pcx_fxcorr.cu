@@ -34,13 +34,7 @@ struct pcx_fxcorr_s {
     // FP32, N = 2^13 or 2^14: three-step form (pcx_fxcorr_ip.cuh)
     void*       xi             = nullptr;    // one allocation: K in its order | twiddles
     const void* xi_tw          = nullptr;
-    // for reuse (see handle_pool): created with PCX_XC_GENERAL; the last call's
-    // end on its stream, unless calls went to several streams or into a capture
-    bool         general = false;
-    cudaEvent_t  done    = nullptr;
-    cudaStream_t last    = nullptr;
-    bool         used    = false;
-    bool         unsure  = false;
+    bool        general        = false;    // created with PCX_XC_GENERAL
 };
 
 namespace {
@@ -349,7 +343,6 @@ void free_handle(pcx_fxcorr_s* h) {
     if (h->ctl) cudaFree(h->ctl);
     if (h->gscratch) cudaFree(h->gscratch);
     if (h->xi) cudaFree(h->xi);
-    if (h->done) cudaEventDestroy(h->done);
     delete h;
 }
 
@@ -418,23 +411,6 @@ handle_pool& pool() {
     return *p;
 }
 
-// Remember where the handle's last call ends.
-void note_call(pcx_fxcorr_s* h, cudaStream_t st) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-        (void)cudaGetLastError();
-        h->unsure = true;
-        return;
-    }
-    if (h->used && st != h->last) h->unsure = true;
-    if (cudaEventRecord(h->done, st) != cudaSuccess) {
-        (void)cudaGetLastError();
-        h->unsure = true;
-    }
-    h->last = st;
-    h->used = true;
-}
-
 // K = FFT(g zero-padded to N) / N, natural order, interleaved (fxcorr.hpp:62-69),
 // and its reordered copy for the three-step form.
 int set_kernel(pcx_fxcorr_s* h, const void* g) {
@@ -456,7 +432,6 @@ int init_handle(pcx_fxcorr_s* h) {
     const bool   f64   = h->dtype == PCX_F64;
     const size_t eb    = f64 ? 16 : 8;
     PCX_CUDA_TRY(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device));
-    PCX_CUDA_TRY(cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming));
     if (int rc = pcx_plan_create(&h->plan, h->n, h->dtype, PCX_ORDER_NORMAL, 2048)) return rc;
     PCX_CUDA_TRY(cudaMalloc(&h->tw, h->n * eb));
     PCX_CUDA_TRY(cudaMalloc(&h->kspec, h->n * eb));
@@ -507,15 +482,7 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
         PCX_CUDA_TRY(cudaGetDevice(&device));
         auto make = [&](pcx_fxcorr_s*& h) -> int {
             h = pool().take(device, dtype, n_fft, general);
-            if (h) {
-                // its last owner's kernels may still read what is set below
-                cudaError_t e = cudaSuccess;
-                if (h->unsure) e = cudaDeviceSynchronize();
-                else if (h->used) e = cudaStreamWaitEvent(0, h->done, 0);
-                if (e == cudaSuccess && h->ctl) e = cudaMemsetAsync(h->ctl, 0, 3 * sizeof(unsigned), 0);
-                PCX_CUDA_TRY(e);
-                h->used = h->unsure = false;
-            } else {
+            if (!h) {
                 h          = new pcx_fxcorr_s{};
                 h->dtype   = dtype;
                 h->n       = n_fft;
@@ -526,6 +493,11 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
             }
             h->k      = k;
             h->pack_g = pack_g;
+            // g may have been written on any stream, and a reused handle's last
+            // owner may still be running: what follows is on the default
+            // stream, which no non-blocking stream is ordered with
+            PCX_CUDA_TRY(cudaDeviceSynchronize());
+            if (h->ctl) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, 3 * sizeof(unsigned), 0));
             if (int rc = set_kernel(h, g)) return rc;
             PCX_CUDA_TRY(cudaStreamSynchronize(0));    // g is read, the tables and K are there
             return PCX_OK;
@@ -567,10 +539,8 @@ extern "C" int pcx_fxcorr_exec(pcx_fxcorr h, void* dst, const void* src, size_t 
                                size_t dst_stride, size_t src_stride, void* stream) {
     return pcx_guard([&]() -> int {
         if (!h) return pcx_fail(PCX_ERR_INVALID, "handle is null");
-        const cudaStream_t st = static_cast<cudaStream_t>(stream);
-        const int          rc = run_xc(h, dst, src, len, pack, channels, dst_stride, src_stride, false, st);
-        note_call(h, st);
-        return rc;
+        return run_xc(h, dst, src, len, pack, channels, dst_stride, src_stride, false,
+                      static_cast<cudaStream_t>(stream));
     });
 }
 
@@ -686,9 +656,6 @@ extern "C" int pcx_fxcorr_vjp(pcx_fxcorr h, void* gx, void* gg, const void* gy, 
                               size_t channels, size_t stride, void* stream) {
     return pcx_guard([&]() -> int {
         if (!h) return pcx_fail(PCX_ERR_INVALID, "handle is null");
-        const cudaStream_t st = static_cast<cudaStream_t>(stream);
-        const int          rc = run_vjp(h, gx, gg, gy, x, len, pack, channels, stride, st);
-        note_call(h, st);
-        return rc;
+        return run_vjp(h, gx, gg, gy, x, len, pack, channels, stride, static_cast<cudaStream_t>(stream));
     });
 }
