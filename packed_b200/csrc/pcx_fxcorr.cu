@@ -23,9 +23,8 @@ struct pcx_fxcorr_s {
     pcx_plan_s* plan   = nullptr;    // natural-order N-point FFT (kernel spectrum, gradient inverse)
     void*       tw     = nullptr;    // W_N^i, i < N
     void*       kspec  = nullptr;    // FFT(g)/N, interleaved complex, natural order
-    unsigned*   ctl    = nullptr;    // [0] work counter, [1] error flag, [2] ticket, [3..] flags
+    unsigned*   ctl    = nullptr;    // [0] error flag, [1] work counter, [2] ticket, [3..] "window loaded" flags
     size_t      flags_cap = 0;
-    unsigned    epoch     = 0;
     void*       gscratch  = nullptr;    // kernel-gradient accumulators
     size_t      gscratch_bytes = 0;
     int         sms            = 0;
@@ -260,7 +259,6 @@ int ensure_flags(pcx_fxcorr_s* h, size_t items) {
     const size_t cap = std::max<size_t>(items, 1024);
     PCX_CUDA_TRY(alloc_zeroed(reinterpret_cast<void**>(&h->ctl), (cap + 3) * sizeof(unsigned)));
     h->flags_cap = cap;
-    h->epoch     = 0;
     return PCX_OK;
 }
 
@@ -284,10 +282,10 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     const bool inplace = dst == src;
     if (inplace && convolve) return pcx_fail(PCX_ERR_INVALID, "the adjoint needs distinct input and output buffers");
     if (int rc = ensure_flags(h, inplace ? total : 1)) return rc;
-    if (++h->epoch == 0) {
-        PCX_CUDA_TRY(cudaMemsetAsync(h->ctl + 3, 0, h->flags_cap * sizeof(unsigned), st));
-        h->epoch = 1;
-    }
+    // In place, the flags (and the counter before them) are cleared on the
+    // call's own stream, so that every run of a captured call finds them clear
+    // too: a flag value that the host chooses per call is the same in each run.
+    if (inplace) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl + 1, 0, (2 + total) * sizeof(unsigned), st));
 
     xc_args a{};
     a.src         = src;
@@ -310,11 +308,10 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     a.conj_kernel = convolve ? 0 : 1;
     a.inplace     = inplace ? 1 : 0;
     a.hwait       = (int)((n + step - 1) / step) - 1;
-    a.epoch       = h->epoch;
     a.flags       = h->ctl + 3;
-    a.counter     = h->ctl;
+    a.counter     = h->ctl + 1;
     a.ticket      = h->ctl + 2;
-    a.error       = reinterpret_cast<int*>(h->ctl + 1);
+    a.error       = reinterpret_cast<int*>(h->ctl);
     a.kspec       = h->kspec;
     // whole-window and three-step forms: FP32, pack 8, windows on whole
     // packs, rows of packs 16-byte aligned
@@ -549,9 +546,9 @@ extern "C" int pcx_fxcorr_status(pcx_fxcorr h) {
         if (!h) return pcx_fail(PCX_ERR_INVALID, "handle is null");
         if (!h->ctl) return PCX_OK;
         unsigned err = 0;
-        PCX_CUDA_TRY(cudaMemcpy(&err, h->ctl + 1, sizeof(unsigned), cudaMemcpyDeviceToHost));
+        PCX_CUDA_TRY(cudaMemcpy(&err, h->ctl, sizeof(unsigned), cudaMemcpyDeviceToHost));
         if (err) {
-            PCX_CUDA_TRY(cudaMemset(h->ctl + 1, 0, sizeof(unsigned)));
+            PCX_CUDA_TRY(cudaMemset(h->ctl, 0, sizeof(unsigned)));
             return pcx_fail(PCX_ERR_TIMEOUT, "a correlation block gave up a bounded wait (for its input copy or, in place, for its predecessor)");
         }
         return PCX_OK;
@@ -612,9 +609,9 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
     a.lp      = __builtin_ctz(pack);
     a.step    = (int)step;
     a.nblk    = (int)nblk;
-    a.counter = h->ctl;
+    a.counter = h->ctl + 1;
     a.ticket  = h->ctl + 2;
-    a.error   = reinterpret_cast<int*>(h->ctl + 1);
+    a.error   = reinterpret_cast<int*>(h->ctl);
     a.acc     = base;
     a.xspec   = base + (size_t)grid * n * eb;
     void* sum = base + rows_s * n * eb;

@@ -21,8 +21,8 @@
 //
 // In place, a tile's outputs overwrite samples that the windows of earlier
 // tiles still read, so tiles are claimed in order from a counter, a block
-// publishes "tile loaded" (the call's epoch in flags[tile]) as it starts on a
-// tile and, before it writes, waits (bounded, about a second) for the tiles
+// publishes "tile loaded" (flags[tile], cleared before each launch) as it starts
+// on a tile and, before it writes, waits (bounded, about a second) for the tiles
 // that hold the hwait blocks before its own.  A block's claimed tiles are
 // published in order and every wait is for lower tiles, so the lowest
 // unpublished tile always gets there.  Out of place, tiles go round the
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
             break;
         }
         if (a.inplace && tid == 0) {
-            st_release(a.flags + tile, a.epoch);    // this tile's windows are loaded
+            st_release(a.flags + tile, 1u);    // this tile's windows are loaded
         }
         const xc3_window x  = win[s][m];
         const float*     in = in0 + s * F::TILE + m * RS;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
         // has to read one
         const int lane = tid % 32;
         bool      seen = true;
-        if (a.inplace && lane < htile && lane < tile) seen = ld_acquire(a.flags + (tile - 1 - lane)) == a.epoch;
+        if (a.inplace && lane < htile && lane < tile) seen = ld_acquire(a.flags + (tile - 1 - lane)) != 0u;
         stage_compute_tab<P, 0>(v, t, stw);
         run_stages_tab<P, X, true, BAR>(v, xch, m, t, stw);
         if (a.inplace) {
@@ -230,9 +230,9 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
             bool late = false;
             for (long long d = lane; d < htile && d < tile && !late; d += 32) {
                 const unsigned* f = a.flags + (tile - 1 - d);
-                if ((d == lane && seen) || ld_acquire(f) == a.epoch) continue;
+                if ((d == lane && seen) || ld_acquire(f) != 0u) continue;
                 const unsigned long long t0 = globaltimer_ns();
-                while (ld_acquire(f) != a.epoch) {
+                while (ld_acquire(f) == 0u) {
                     if (globaltimer_ns() - t0 > XC_WAIT_NS) {
                         late = true;
                         break;

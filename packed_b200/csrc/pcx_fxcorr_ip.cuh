@@ -27,8 +27,8 @@
 // FP64 4.0e-7 and 2.8e-7.  8192 points, 16 x 2^20, 2048 taps: 220 and 115 us.
 //
 // In place, a window's outputs overwrite samples that earlier blocks' windows
-// read: blocks are claimed in order, each publishes "window loaded" (the call's
-// epoch in flags[item]), and every warp waits (bounded, about a second) for its
+// read: blocks are claimed in order, each publishes "window loaded" (flags[item],
+// cleared before each launch), and every warp waits (bounded, about a second) for its
 // predecessors before it writes, as in the other forms.
 #pragma once
 
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
         }
         phase ^= 1;
         if (tid == 0) {
-            if (a.inplace) st_release(a.flags + item, a.epoch);    // this window is loaded
+            if (a.inplace) st_release(a.flags + item, 1u);    // this window is loaded
             s_item = atomicAdd(a.counter, 1u);
         }
         dft<32, 1, 0>(v);
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
         // in place: the first look at the flags, so that the wait below rarely has to read one
         const unsigned blk  = item - ch * nblk;
         bool           seen = true;
-        if (a.inplace && lane < a.hwait && lane < blk) seen = ld_acquire(a.flags + (item - 1 - lane)) == a.epoch;
+        if (a.inplace && lane < a.hwait && lane < blk) seen = ld_acquire(a.flags + (item - 1 - lane)) != 0u;
         __syncthreads();
         // ---------------- times W_16B^(c kb), back over kb
         static_for<32>([&](auto ic) {
@@ -296,9 +296,9 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
             bool late = false;
             for (unsigned d = lane; d < (unsigned)a.hwait && d < blk && !late; d += 32) {
                 const unsigned* f = a.flags + (item - 1 - d);
-                if ((d == (unsigned)lane && seen) || ld_acquire(f) == a.epoch) continue;
+                if ((d == (unsigned)lane && seen) || ld_acquire(f) != 0u) continue;
                 const unsigned long long t0 = globaltimer_ns();
-                while (ld_acquire(f) != a.epoch) {
+                while (ld_acquire(f) == 0u) {
                     if (globaltimer_ns() - t0 > XC_WAIT_NS) {
                         late = true;
                         break;

@@ -9,8 +9,8 @@
 //
 // Work is claimed in order from a device counter by persistent CTAs.  In
 // place, block b's outputs overwrite samples that the windows of blocks
-// b-1 .. b-h still read, so each block publishes "window read" (the call's
-// epoch in flags[item]) and waits for its h predecessors before writing.
+// b-1 .. b-h still read, so each block publishes "window read" (flags[item],
+// cleared before each launch) and waits for its h predecessors before writing.
 // Predecessors were claimed earlier by resident CTAs that never wait before
 // publishing, so the wait always ends; it is still bounded (about one second
 // of %globaltimer), after which the block records an error and gives up.
@@ -35,8 +35,7 @@ struct xc_args {
     int           conj_kernel;   // 1: multiply by conj(K) (correlation); 0: by K (convolution)
     int           inplace;       // publish / wait on window reads
     int           hwait;         // predecessors whose windows overlap this block's outputs
-    unsigned      epoch;
-    unsigned*     flags;
+    unsigned*     flags;         // zero before an in-place launch
     unsigned*     counter;       // work counter, zero outside a launch
     unsigned*     ticket;        // blocks done claiming, likewise
     int*          error;
@@ -129,7 +128,7 @@ __global__ void __launch_bounds__(M * splan<LOGN, EPT>::TT) k_fxcorr(xc_args a, 
         __syncthreads();
         if (a.inplace && tid == 0) {
             __threadfence();
-            for (int mm = 0; mm < M && item0 + mm < a.total; ++mm) st_release(a.flags + item0 + mm, a.epoch);
+            for (int mm = 0; mm < M && item0 + mm < a.total; ++mm) st_release(a.flags + item0 + mm, 1u);
         }
         cpx<T> v[E];
         static_for<E>([&](auto ic) {
@@ -156,9 +155,9 @@ __global__ void __launch_bounds__(M * splan<LOGN, EPT>::TT) k_fxcorr(xc_args a, 
                     const long long blk = it % a.nblk;
                     for (int d = 1; d <= a.hwait && d <= blk; ++d) {
                         const unsigned* f = a.flags + (it - d);
-                        if (ld_acquire(f) == a.epoch) continue;
+                        if (ld_acquire(f) != 0u) continue;
                         const unsigned long long t0 = globaltimer_ns();
-                        while (ld_acquire(f) != a.epoch) {
+                        while (ld_acquire(f) == 0u) {
                             if (globaltimer_ns() - t0 > XC_WAIT_NS) {
                                 atomicExch(a.error, 1);
                                 s_abort = 1;
