@@ -297,6 +297,9 @@ int pcx_fxcorr_release_idle(void);
  * fxcorr_unit::operator()(vec) (fxcorr.hpp:102-136, block loop with the
  * block offset taken as a packed element index) and the empty out-of-place
  * operator()(dest, src) (fxcorr.hpp:138-140).  dst == src is in place.
+ * Out-of-place calls of one handle share nothing but the error flag and may
+ * overlap on several streams; in-place calls share the handle's flags, and
+ * calls of pcx_fxcorr_vjp with gg its scratch: no two of those may overlap.
  */
 int pcx_fxcorr_exec(pcx_fxcorr h, void* dst, const void* src, size_t len, int pack, size_t channels,
                     size_t dst_stride, size_t src_stride, void* stream);

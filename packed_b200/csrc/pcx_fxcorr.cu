@@ -23,7 +23,7 @@ struct pcx_fxcorr_s {
     pcx_plan_s* plan   = nullptr;    // natural-order N-point FFT (kernel spectrum, gradient inverse)
     void*       tw     = nullptr;    // W_N^i, i < N
     void*       kspec  = nullptr;    // FFT(g)/N, interleaved complex, natural order
-    unsigned*   ctl    = nullptr;    // [0] error flag, [1] work counter, [2] ticket, [3..] "window loaded" flags
+    unsigned*   ctl    = nullptr;    // [0] error flag, [1] work counter, [2..] "window loaded" flags
     size_t      flags_cap = 0;
     void*       gscratch  = nullptr;    // kernel-gradient accumulators
     size_t      gscratch_bytes = 0;
@@ -257,7 +257,7 @@ int ensure_flags(pcx_fxcorr_s* h, size_t items) {
     h->ctl       = nullptr;
     h->flags_cap = 0;
     const size_t cap = std::max<size_t>(items, 1024);
-    PCX_CUDA_TRY(alloc_zeroed(reinterpret_cast<void**>(&h->ctl), (cap + 3) * sizeof(unsigned)));
+    PCX_CUDA_TRY(alloc_zeroed(reinterpret_cast<void**>(&h->ctl), (cap + 2) * sizeof(unsigned)));
     h->flags_cap = cap;
     return PCX_OK;
 }
@@ -285,7 +285,7 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     // In place, the flags (and the counter before them) are cleared on the
     // call's own stream, so that every run of a captured call finds them clear
     // too: a flag value that the host chooses per call is the same in each run.
-    if (inplace) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl + 1, 0, (2 + total) * sizeof(unsigned), st));
+    if (inplace) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl + 1, 0, (1 + total) * sizeof(unsigned), st));
 
     xc_args a{};
     a.src         = src;
@@ -308,9 +308,8 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     a.conj_kernel = convolve ? 0 : 1;
     a.inplace     = inplace ? 1 : 0;
     a.hwait       = (int)((n + step - 1) / step) - 1;
-    a.flags       = h->ctl + 3;
+    a.flags       = h->ctl + 2;
     a.counter     = h->ctl + 1;
-    a.ticket      = h->ctl + 2;
     a.error       = reinterpret_cast<int*>(h->ctl);
     a.kspec       = h->kspec;
     // whole-window and three-step forms: FP32, pack 8, windows on whole
@@ -494,7 +493,7 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
             // owner may still be running: what follows is on the default
             // stream, which no non-blocking stream is ordered with
             PCX_CUDA_TRY(cudaDeviceSynchronize());
-            if (h->ctl) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, 3 * sizeof(unsigned), 0));
+            if (h->ctl) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), 0));
             if (int rc = set_kernel(h, g)) return rc;
             PCX_CUDA_TRY(cudaStreamSynchronize(0));    // g is read, the tables and K are there
             return PCX_OK;
@@ -609,8 +608,6 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
     a.lp      = __builtin_ctz(pack);
     a.step    = (int)step;
     a.nblk    = (int)nblk;
-    a.counter = h->ctl + 1;
-    a.ticket  = h->ctl + 2;
     a.error   = reinterpret_cast<int*>(h->ctl);
     a.acc     = base;
     a.xspec   = base + (size_t)grid * n * eb;

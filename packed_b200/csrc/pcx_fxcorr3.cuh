@@ -257,7 +257,6 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
             }
         });
     }
-    if (a.inplace && tid == 0) xc_done(a.counter, a.ticket);
     tc_fence_before();
     __syncthreads();
     if (tid < 32) tmem_dealloc(tbase, 64);

@@ -26,10 +26,11 @@
 // taps, in place: 395 us with the two-step form, 260 us; relative error against
 // FP64 4.0e-7 and 2.8e-7.  8192 points, 16 x 2^20, 2048 taps: 220 and 115 us.
 //
-// In place, a window's outputs overwrite samples that earlier blocks' windows
-// read: blocks are claimed in order, each publishes "window loaded" (flags[item],
-// cleared before each launch), and every warp waits (bounded, about a second) for its
-// predecessors before it writes, as in the other forms.
+// Out of place, windows go round the blocks.  In place, a window's outputs
+// overwrite samples that earlier blocks' windows read: they are claimed in
+// order, each block publishes "window loaded" (flags[item], cleared before each
+// launch), and every warp waits (bounded, about a second) for its predecessors
+// before it writes, as in the other forms.
 #pragma once
 
 #include "pcx_fft_v2.cuh"
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
     }
     tw2[tid] = ldg_cpx(reinterpret_cast<const cpx<float>*>(A.tw) + N + tid);
     if (tid == 0) {
-        s_item = atomicAdd(a.counter, 1u);
+        s_item = a.inplace ? atomicAdd(a.counter, 1u) : blockIdx.x;
         mbar_init(&full, 1);
         fence_barrier_init();
     }
@@ -228,8 +229,12 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
         }
         phase ^= 1;
         if (tid == 0) {
-            if (a.inplace) st_release(a.flags + item, 1u);    // this window is loaded
-            s_item = atomicAdd(a.counter, 1u);
+            if (a.inplace) {
+                st_release(a.flags + item, 1u);    // this window is loaded
+                s_item = atomicAdd(a.counter, 1u);
+            } else {
+                s_item = item + gridDim.x;
+            }
         }
         dft<32, 1, 0>(v);
         xci_mul<false>(v, tcol, false);
@@ -329,7 +334,6 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
         }
         item = next;
     }
-    if (tid == 0) xc_done(a.counter, a.ticket);
     tc_fence_before();
     __syncthreads();
     if (tid < 32) tmem_dealloc(tbase, F::TCOLS);

@@ -7,8 +7,8 @@
 // element pattern the inverse's first stage reads — so no exchange separates
 // the two transforms.
 //
-// Work is claimed in order from a device counter by persistent CTAs.  In
-// place, block b's outputs overwrite samples that the windows of blocks
+// Persistent CTAs take items in turn; in place they claim them in order from a
+// device counter: block b's outputs overwrite samples that the windows of blocks
 // b-1 .. b-h still read, so each block publishes "window read" (flags[item],
 // cleared before each launch) and waits for its h predecessors before writing.
 // Predecessors were claimed earlier by resident CTAs that never wait before
@@ -36,8 +36,7 @@ struct xc_args {
     int           inplace;       // publish / wait on window reads
     int           hwait;         // predecessors whose windows overlap this block's outputs
     unsigned*     flags;         // zero before an in-place launch
-    unsigned*     counter;       // work counter, zero outside a launch
-    unsigned*     ticket;        // blocks done claiming, likewise
+    unsigned*     counter;       // work counter, likewise
     int*          error;
     const void*   kspec;         // K / N_fft, natural order, interleaved complex
 };
@@ -54,18 +53,6 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 }
 __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// One thread of a block that claims no more work: the last block of the launch
-// leaves the work counter (and the ticket it counts blocks with) zero for the
-// next one.
-__device__ __forceinline__ void xc_done(unsigned* counter, unsigned* ticket) {
-    __threadfence();
-    if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
-        __threadfence();
-        *counter = 0u;
-        *ticket  = 0u;
-    }
 }
 
 constexpr unsigned long long XC_WAIT_NS = 1000000000ull;    // 1 s
@@ -113,17 +100,14 @@ __global__ void __launch_bounds__(M * splan<LOGN, EPT>::TT) k_fxcorr(xc_args a, 
     T*        dst = reinterpret_cast<T*>(a.dst);
     const int Pk  = 1 << a.lp;
 
-    for (;;) {
+    for (long long turn = (long long)blockIdx.x * M;; turn += (long long)gridDim.x * M) {
         if (tid == 0) {
-            s_item  = (long long)atomicAdd(a.counter, (unsigned)M);
+            s_item  = a.inplace ? (long long)atomicAdd(a.counter, (unsigned)M) : turn;
             s_abort = 0;
         }
         __syncthreads();
         const long long item0 = s_item;
-        if (item0 >= a.total) {
-            if (tid == 0) xc_done(a.counter, a.ticket);
-            break;
-        }
+        if (item0 >= a.total) break;
         xc_load<T, L, NT>(buf, a, item0, M);
         __syncthreads();
         if (a.inplace && tid == 0) {
@@ -171,10 +155,7 @@ __global__ void __launch_bounds__(M * splan<LOGN, EPT>::TT) k_fxcorr(xc_args a, 
                 }
             }
             __syncthreads();
-            if (s_abort) {    // every thread of the CTA leaves together
-                if (tid == 0) xc_done(a.counter, a.ticket);
-                return;
-            }
+            if (s_abort) return;    // every thread of the CTA leaves together
         }
         if (item < a.total) {
             const long long ch  = item / a.nblk;
@@ -215,8 +196,6 @@ struct kg_args {
     int         step;
     int         nblk;
     long long   total;
-    unsigned*   counter;      // work counter, zero outside a launch
-    unsigned*   ticket;       // blocks done claiming, likewise
     void*       acc;          // [gridDim.x][N] complex
     void*       xspec;        // [gridDim.x][N] complex, per-CTA spectrum scratch
     int*        error;        // set when a bounded wait gave up (forms with bulk copies)
@@ -230,11 +209,10 @@ __global__ void __launch_bounds__(splan<LOGN, EPT>::TT) k_fxcorr_kgrad(kg_args a
     constexpr int TT = P::TT;
     using X          = xch_blocked<L, 1>;
     extern __shared__ __align__(16) unsigned char smem[];
-    cpx<T>*              buf = reinterpret_cast<cpx<T>*>(smem);
-    __shared__ long long s_item;
-    const int            t   = threadIdx.x;
-    cpx<T>*              acc = reinterpret_cast<cpx<T>*>(a.acc) + (long long)blockIdx.x * L;
-    cpx<T>*              xs  = reinterpret_cast<cpx<T>*>(a.xspec) + (long long)blockIdx.x * L;
+    cpx<T>*   buf = reinterpret_cast<cpx<T>*>(smem);
+    const int t   = threadIdx.x;
+    cpx<T>*   acc = reinterpret_cast<cpx<T>*>(a.acc) + (long long)blockIdx.x * L;
+    cpx<T>*   xs  = reinterpret_cast<cpx<T>*>(a.xspec) + (long long)blockIdx.x * L;
     for (int e = t; e < L; e += TT) acc[e] = {T(0), T(0)};
 
     xc_args la{};
@@ -245,14 +223,7 @@ __global__ void __launch_bounds__(splan<LOGN, EPT>::TT) k_fxcorr_kgrad(kg_args a
     la.total      = a.total;
     la.src_stride = a.stride;
     la.src        = a.x;
-    for (;;) {
-        if (t == 0) s_item = (long long)atomicAdd(a.counter, 1u);
-        __syncthreads();
-        const long long item = s_item;
-        if (item >= a.total) {
-            if (t == 0) xc_done(a.counter, a.ticket);
-            break;
-        }
+    for (long long item = blockIdx.x; item < a.total; item += gridDim.x) {
         // x window [b*step, b*step + N)
         xc_load<T, L, TT>(buf, la, item, 1);
         __syncthreads();
