@@ -237,6 +237,9 @@ static int fs_select(pcx_plan_s* p, const fs_variant& v) {
 }
 
 // The built-in variants of the one-launch four-step for this plan's size.
+// Transforms that a plan's four-step counters are made for at its creation.
+constexpr size_t FS_BATCH = 4096;
+
 static std::vector<fs_variant> fs_candidates(const pcx_plan_s* p) {
     std::vector<fs_variant> out;
     if (p->dtype == PCX_F64) {
@@ -329,6 +332,11 @@ static int plan_init_tables(pcx_plan_s* p) {
             // one launch for a whole batch: the size's first built-in variant
             for (const fs_variant& v: fs_candidates(p)) {
                 if (fs_select(p, v) == PCX_OK) break;
+            }
+            if (p->fs.tc > 0) {    // counters of a usual batch, so that no call has to allocate them
+                PCX_CUDA_TRY(cudaMalloc(&p->fs_ctr, (2 * FS_BATCH + 1) * sizeof(int)));
+                PCX_CUDA_TRY(cudaMemsetAsync(p->fs_ctr, 0, (2 * FS_BATCH + 1) * sizeof(int), 0));
+                p->fs_ctr_n = 2 * FS_BATCH;
             }
             // its forms for other packs, short sources and permuted orders (where built)
             for (auto form: {pcx_fs_any, pcx_fs_out, pcx_fs_in}) {
@@ -957,9 +965,10 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
             if (p->fs_ctr) cudaFree(p->fs_ctr);
             p->fs_ctr   = nullptr;
             p->fs_ctr_n = 0;
-            // every launch leaves them zero
-            PCX_CUDA_TRY(alloc_zeroed(reinterpret_cast<void**>(&p->fs_ctr), (2 * batch + 1) * sizeof(int)));
-            p->fs_ctr_n = 2 * batch;
+            // every launch leaves them zero; room for twice the batch, so that
+            // slowly growing batches seldom come here
+            PCX_CUDA_TRY(alloc_zeroed(reinterpret_cast<void**>(&p->fs_ctr), (4 * batch + 1) * sizeof(int)));
+            p->fs_ctr_n = 4 * batch;
         }
         fs_args a{};
         a.src        = src;

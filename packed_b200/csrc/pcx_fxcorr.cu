@@ -23,7 +23,8 @@ struct pcx_fxcorr_s {
     pcx_plan_s* plan   = nullptr;    // natural-order N-point FFT (kernel spectrum, gradient inverse)
     void*       tw     = nullptr;    // W_N^i, i < N
     void*       kspec  = nullptr;    // FFT(g)/N, interleaved complex, natural order
-    unsigned*   ctl    = nullptr;    // [0] error flag, [1] work counter, [2..] "window loaded" flags
+    int*        err    = nullptr;    // error flag, behind kspec
+    unsigned*   ctl    = nullptr;    // in-place calls: [0] work counter, [1..] "window loaded" flags
     size_t      flags_cap = 0;
     void*       gscratch  = nullptr;    // kernel-gradient accumulators
     size_t      gscratch_bytes = 0;
@@ -257,7 +258,7 @@ int ensure_flags(pcx_fxcorr_s* h, size_t items) {
     h->ctl       = nullptr;
     h->flags_cap = 0;
     const size_t cap = std::max<size_t>(items, 1024);
-    PCX_CUDA_TRY(alloc_zeroed(reinterpret_cast<void**>(&h->ctl), (cap + 2) * sizeof(unsigned)));
+    PCX_CUDA_TRY(cudaMalloc(&h->ctl, (cap + 1) * sizeof(unsigned)));
     h->flags_cap = cap;
     return PCX_OK;
 }
@@ -281,11 +282,13 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     if (total >= (size_t(1) << 31)) return pcx_fail(PCX_ERR_UNSUPPORTED, "too many blocks in one call");
     const bool inplace = dst == src;
     if (inplace && convolve) return pcx_fail(PCX_ERR_INVALID, "the adjoint needs distinct input and output buffers");
-    if (int rc = ensure_flags(h, inplace ? total : 1)) return rc;
-    // In place, the flags (and the counter before them) are cleared on the
-    // call's own stream, so that every run of a captured call finds them clear
-    // too: a flag value that the host chooses per call is the same in each run.
-    if (inplace) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl + 1, 0, (1 + total) * sizeof(unsigned), st));
+    if (inplace) {
+        // The flags (and the counter before them) are cleared on the call's own
+        // stream, so that every run of a captured call finds them clear too: a
+        // flag value that the host chooses per call is the same in each run.
+        if (int rc = ensure_flags(h, total)) return rc;
+        PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, (1 + total) * sizeof(unsigned), st));
+    }
 
     xc_args a{};
     a.src         = src;
@@ -308,9 +311,9 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     a.conj_kernel = convolve ? 0 : 1;
     a.inplace     = inplace ? 1 : 0;
     a.hwait       = (int)((n + step - 1) / step) - 1;
-    a.flags       = h->ctl + 2;
-    a.counter     = h->ctl + 1;
-    a.error       = reinterpret_cast<int*>(h->ctl);
+    a.flags       = inplace ? h->ctl + 1 : nullptr;
+    a.counter     = h->ctl;
+    a.error       = h->err;
     a.kspec       = h->kspec;
     // whole-window and three-step forms: FP32, pack 8, windows on whole
     // packs, rows of packs 16-byte aligned
@@ -430,7 +433,8 @@ int init_handle(pcx_fxcorr_s* h) {
     PCX_CUDA_TRY(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device));
     if (int rc = pcx_plan_create(&h->plan, h->n, h->dtype, PCX_ORDER_NORMAL, 2048)) return rc;
     PCX_CUDA_TRY(cudaMalloc(&h->tw, h->n * eb));
-    PCX_CUDA_TRY(cudaMalloc(&h->kspec, h->n * eb));
+    PCX_CUDA_TRY(cudaMalloc(&h->kspec, h->n * eb + sizeof(int)));
+    h->err = reinterpret_cast<int*>(static_cast<char*>(h->kspec) + h->n * eb);
     PCX_CUDA_TRY(pcx_gen_twiddles(h->tw, (int)h->n, log_n, 1, f64, 0));
     if (int rc = f64 ? dispatch_xc<double>(log_n, xc_args{}, nullptr, 0, 0, true)
                      : dispatch_xc<float>(log_n, xc_args{}, nullptr, 0, 0, true)) {
@@ -493,7 +497,7 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
             // owner may still be running: what follows is on the default
             // stream, which no non-blocking stream is ordered with
             PCX_CUDA_TRY(cudaDeviceSynchronize());
-            if (h->ctl) PCX_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(unsigned), 0));
+            PCX_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), 0));
             if (int rc = set_kernel(h, g)) return rc;
             PCX_CUDA_TRY(cudaStreamSynchronize(0));    // g is read, the tables and K are there
             return PCX_OK;
@@ -543,11 +547,10 @@ extern "C" int pcx_fxcorr_exec(pcx_fxcorr h, void* dst, const void* src, size_t 
 extern "C" int pcx_fxcorr_status(pcx_fxcorr h) {
     return pcx_guard([&]() -> int {
         if (!h) return pcx_fail(PCX_ERR_INVALID, "handle is null");
-        if (!h->ctl) return PCX_OK;
-        unsigned err = 0;
-        PCX_CUDA_TRY(cudaMemcpy(&err, h->ctl, sizeof(unsigned), cudaMemcpyDeviceToHost));
+        int err = 0;
+        PCX_CUDA_TRY(cudaMemcpy(&err, h->err, sizeof(int), cudaMemcpyDeviceToHost));
         if (err) {
-            PCX_CUDA_TRY(cudaMemset(h->ctl, 0, sizeof(unsigned)));
+            PCX_CUDA_TRY(cudaMemset(h->err, 0, sizeof(int)));
             return pcx_fail(PCX_ERR_TIMEOUT, "a correlation block gave up a bounded wait (for its input copy or, in place, for its predecessor)");
         }
         return PCX_OK;
@@ -599,7 +602,6 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
         PCX_CUDA_TRY(cudaMalloc(&h->gscratch, need));
         h->gscratch_bytes = need;
     }
-    if (int rc = ensure_flags(h, 1)) return rc;
     char* base = static_cast<char*>(h->gscratch);
     a.x       = x;
     a.gy      = gy;
@@ -608,7 +610,7 @@ static int run_vjp(pcx_fxcorr_s* h, void* gx, void* gg, const void* gy, const vo
     a.lp      = __builtin_ctz(pack);
     a.step    = (int)step;
     a.nblk    = (int)nblk;
-    a.error   = reinterpret_cast<int*>(h->ctl);
+    a.error   = h->err;
     a.acc     = base;
     a.xspec   = base + (size_t)grid * n * eb;
     void* sum = base + rows_s * n * eb;

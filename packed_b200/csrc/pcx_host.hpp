@@ -54,18 +54,28 @@ inline cudaError_t smem_attr_cached(const void* kern, int bytes) {
 }
 
 // Zeroed device memory for counters that every launch leaves zero.  Filled and
-// waited for on a stream of its own: on the caller's stream the fill could
-// become part of a capture that is never replayed, and on the default one a
-// launch on another stream could overtake it.
+// waited for on a stream of its own, one per device and kept: on the caller's
+// stream the fill could become part of a capture that is never replayed, and on
+// the default one a launch on another stream could overtake it.
 inline cudaError_t alloc_zeroed(void** out, size_t bytes) {
-    void*        p = nullptr;
-    cudaStream_t s = nullptr;
-    cudaError_t  e = cudaMalloc(&p, bytes);
+    static std::mutex                  mu;
+    static std::map<int, cudaStream_t> streams;
+    int          dev = 0;
+    void*        p   = nullptr;
+    cudaStream_t s   = nullptr;
+    cudaError_t  e   = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, bytes, s);
+    {
+        std::lock_guard<std::mutex> g(mu);
+        cudaStream_t&               kept = streams[dev];
+        if (!kept) e = cudaStreamCreateWithFlags(&kept, cudaStreamNonBlocking);
+        if (e != cudaSuccess) return e;
+        s = kept;
+    }
+    e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync(p, 0, bytes, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (s) cudaStreamDestroy(s);
     if (e == cudaSuccess) *out = p;
     else cudaFree(p);
     return e;
