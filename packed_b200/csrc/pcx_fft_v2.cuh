@@ -118,6 +118,13 @@ __device__ __forceinline__ void load_stage_tw(cpx<T>* f, int t, const cpx<T>* __
     });
 }
 
+// The transform of a butterfly's R values.
+template<int R, class T>
+__device__ __forceinline__ void stage_dft(cpx<T> (&a)[R]) {
+    if constexpr (R == 32) dft32_4x8(a);
+    else dft<R, 1, 0>(a);
+}
+
 // Butterflies of stage S >= 1 with preloaded table factors.
 template<class P, int S, class T, int E>
 __device__ __forceinline__ void stage_apply_tw(cpx<T> (&v)[E], const cpx<T>* f) {
@@ -133,7 +140,7 @@ __device__ __forceinline__ void stage_apply_tw(cpx<T> (&v)[E], const cpx<T>* f) 
             constexpr int j = decltype(jc)::value + 1;
             a[j]            = cmul(v[g + j * G], stw_factor<RB, j>(f + g * Q));
         });
-        dft<R, 1, 0>(a);
+        stage_dft(a);
         static_for<R>([&](auto jc) {
             constexpr int j = decltype(jc)::value;
             v[g + j * G]    = a[j];
@@ -158,7 +165,7 @@ __device__ __forceinline__ void stage_compute_tab(cpx<T> (&v)[E], int t, const c
                 constexpr int j = decltype(jc)::value;
                 a[j]            = v[g + j * G];
             });
-            dft<R, 1, 0>(a);
+            stage_dft(a);
             static_for<R>([&](auto jc) {
                 constexpr int j = decltype(jc)::value;
                 v[g + j * G]    = a[j];
