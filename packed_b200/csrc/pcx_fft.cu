@@ -831,6 +831,7 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         t3.order_out  = io.order_out;
         t3.scale      = io.scale;
         t3.stw        = stw;
+        t3.rows       = p->stw_rows;
         t3.error      = p->err;
         t3.lp_src     = io.lp_src;
         t3.lp_dst     = io.lp_dst;
@@ -843,9 +844,7 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         // natural order from 256 points on (FP64: 128) goes straight through
         // registers; k_single3 is faster below and takes the other orders
         if (natural && p->log_n >= 7 && (f64 || p->log_n >= 8 || !tma)) {
-            if (p->stw_rows) t3.stw = p->stw_rows;
             const cudaError_t e = (plain ? pcx_rows : pcx_rows_any)(f64, p->log_n, t3, st, false);
-            t3.stw              = stw;
             if (e != cudaErrorNotSupported) return e;
         }
         if (!tma) return cudaErrorNotSupported;

@@ -238,6 +238,15 @@ __host__ __device__ constexpr int stage_tw_smem_bytes() {
     return stage_tw_size<P>() * (int)sizeof(cpx<T>);
 }
 
+// Copy a table of BYTES bytes into shared memory (16-byte units; the caller syncs).
+template<int BYTES, class T>
+__device__ __forceinline__ void copy_table_to_smem(cpx<T>* dst, const void* src, int tid, int nt) {
+    static_assert(BYTES % 16 == 0, "table in 16-byte units");
+    const uint4* sp = reinterpret_cast<const uint4*>(src);
+    uint4*       dp = reinterpret_cast<uint4*>(dst);
+    for (int i = tid; i < BYTES / 16; i += nt) dp[i] = __ldg(sp + i);
+}
+
 // Whether a kernel whose own shared memory is `base` bytes (MINB resident CTAs
 // per SM wanted) can also hold a `tab`-byte stage table without losing
 // residency: 228 KB per SM, 227 KB per CTA, 1 KB reserved per CTA.
@@ -348,7 +357,8 @@ struct v3_args {
     int         order_in;
     int         order_out;
     double      scale;
-    const void* stw;
+    const void* stw;      // factors of the stage twiddles
+    const void* rows;     // the tables of pcx_rows_twiddles
     int*        error;    // set when a bounded wait gives up
     // the any-pack forms only (k_rows and k_single3 with ANY):
     int         lp_src;     // log2 pack widths
@@ -356,6 +366,73 @@ struct v3_args {
     int         src_len;    // valid source elements per row (zero-extended to N)
     int         pairs;      // interleaved rows may be moved a complex number at a time (aligned)
 };
+
+// Full stage tables of the any-pack forms (every twiddle an entry of its own,
+// generated in FP64 and rounded once; as products of two factors they cost 5 %
+// more error in FP32, 2 % in FP64): stage S >= 1 has Ns * R entries, those of butterfly
+// position k in pairs W^(2qk), W^((2q+1)k) at [q][k], so that a warp's loads are
+// contiguous.
+template<class P>
+__host__ __device__ constexpr int rows_tw_offset(int S) {
+    int off = 0;
+    for (int s = 1; s < S; ++s) off += 1 << (P::nsbits(s) + P::rbits(s));
+    return off;
+}
+template<class P>
+__host__ __device__ constexpr int rows_tw_size() {
+    return rows_tw_offset<P>(P::NST);
+}
+template<class T>
+__global__ void k_rows_twiddles(cpx<T>* out, int nsb, int rb) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= 1 << (nsb + rb)) return;
+    const int       k = (q >> 1) & ((1 << nsb) - 1), j = 2 * (q >> (nsb + 1)) + (q & 1);
+    const long long e = (long long)j * k;
+    double          s, c;
+    sincospi(2.0 * (double)e / (double)(1LL << (nsb + rb)), &s, &c);
+    out[q] = {T(c), T(-s)};
+}
+
+// Stages 1..NST-1 with these tables (SH: in shared memory).
+template<class P, class X, bool SH, int BARN, class T, int E>
+__device__ __forceinline__ void run_stages_rows(cpx<T> (&v)[E], cpx<T>* xch, int m, int t,
+                                                const cpx<T>* __restrict__ tab) {
+    static_for<P::NST - 1>([&](auto sc) {
+        constexpr int S = decltype(sc)::value;
+        constexpr int G = E / (1 << P::rbits(S));
+        xch_sync<BARN>();
+        static_for<E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            xch[X::idx(m, stage_out_index<P, S>(t, i % G, i / G))] = v[i];
+        });
+        xch_sync<BARN>();
+        static_for<E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            v[i]            = xch[X::idx(m, t + i * P::TT)];
+        });
+        constexpr int NSB = P::nsbits(S + 1);
+        constexpr int R   = 1 << P::rbits(S + 1);
+        constexpr int GN  = E / R;
+        static_for<GN>([&](auto gc) {
+            constexpr int g  = decltype(gc)::value;
+            const int     k  = (t + g * P::TT) & ((1 << NSB) - 1);
+            const cpx<T>* tw = tab + rows_tw_offset<P>(S + 1) + 2 * k;
+            cpx<T>        a[R];
+            static_for<R / 2>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                cpx<T>        w0, w1;
+                ld2<SH>(tw + (q << (NSB + 1)), w0, w1);
+                a[2 * q]     = q == 0 ? v[g] : cmul(v[g + 2 * q * GN], w0);
+                a[2 * q + 1] = cmul(v[g + (2 * q + 1) * GN], w1);
+            });
+            stage_dft(a);
+            static_for<R>([&](auto jc) {
+                constexpr int j = decltype(jc)::value;
+                v[g + j * GN]   = a[j];
+            });
+        });
+    });
+}
 
 // Exchange layout of 32-point stages: one slot of padding per 32.
 template<int L, int M>
@@ -398,7 +475,25 @@ struct rows_cfg {
     static constexpr int MINB = (sizeof(T) == 8 || W ? 512 : 1024) / NT;
     using X                   = std::conditional_t<W, xch_blocked32<P::L, M>, xch_blocked<P::L, M>>;
     static constexpr int SMEM = X::size * (int)sizeof(cpx<T>);
+    // v3_args::rows: with 32 points per thread the factors, then the full
+    // tables of 16 points per thread (k_single3's) and, at FULL, of its own
+    static constexpr int FULL16 = W ? stage_tw_size<P>() : 0;
+    static constexpr int FULL   = W ? FULL16 + rows_tw_size<splan<LOGL>>() : 0;
 };
+
+// Loads of interleaved data, past L1, where the full tables are (1 -> 8 at 8192
+// points 4980 GB/s so and 4760 through L1; the two halves of wider packs share
+// lines and lose by it).
+__device__ __forceinline__ float2 ld_once(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double2 ld_once(const double2* p) {
+    double2 v;
+    asm volatile("ld.global.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
 
 template<class T, int LOGL, int LP, bool ANY>
 __global__ void __launch_bounds__(rows_cfg<T, LOGL>::NT, rows_cfg<T, LOGL>::MINB) k_rows(v3_args a) {
@@ -411,7 +506,6 @@ __global__ void __launch_bounds__(rows_cfg<T, LOGL>::NT, rows_cfg<T, LOGL>::MINB
     static_assert(TT % (1 << LP) == 0, "pack must divide threads per row");
     extern __shared__ __align__(16) unsigned char smem[];
     cpx<T>*         xch  = reinterpret_cast<cpx<T>*>(smem);
-    const auto*     stw  = reinterpret_cast<const cpx<T>*>(a.stw);
     const int       m    = threadIdx.x / TT;
     const int       t    = threadIdx.x - m * TT;
     const long long row  = (long long)blockIdx.x * F::M + m;
@@ -432,7 +526,7 @@ __global__ void __launch_bounds__(rows_cfg<T, LOGL>::NT, rows_cfg<T, LOGL>::MINB
     } else if (ANY && lps == 0 && a.pairs) {
         static_for<E>([&](auto ic) {
             constexpr int i = decltype(ic)::value;
-            const V2      x = reinterpret_cast<const V2*>(src)[t + i * TT];
+            const V2      x = ld_once(reinterpret_cast<const V2*>(src) + t + i * TT);
             v[i]            = {x.x, x.y};
         });
     } else {
@@ -443,8 +537,13 @@ __global__ void __launch_bounds__(rows_cfg<T, LOGL>::NT, rows_cfg<T, LOGL>::MINB
         });
     }
     if (a.conj_in) static_for<E>([&](auto ic) { v[decltype(ic)::value].im = -v[decltype(ic)::value].im; });
-    stage_compute_tab<P, 0>(v, t, stw);
-    run_stages_tab<P, typename F::X, false, (TT <= 32 ? -1 : 0)>(v, xch, m, t, stw);
+    constexpr int BAR = TT <= 32 ? -1 : 0;
+    stage_compute_tab<P, 0>(v, t, static_cast<const cpx<T>*>(nullptr));
+    if constexpr (ANY) {
+        run_stages_rows<P, typename F::X, false, BAR>(v, xch, m, t, static_cast<const cpx<T>*>(a.rows) + F::FULL);
+    } else {
+        run_stages_tab<P, typename F::X, false, BAR>(v, xch, m, t, static_cast<const cpx<T>*>(F::W ? a.rows : a.stw));
+    }
     if (!live) return;
     const T sc  = T(a.scale);
     const T sim = a.conj_out ? -sc : sc;
@@ -614,7 +713,7 @@ __host__ __device__ constexpr int single3_pad() {
 // Shape of the TMA-fed one-pass kernel at a size: four warps a block at 32
 // and 64 points (GB/s, 512 MB, 128 and 256 threads: FP32 4784 and 3411, 5877
 // and 4820; FP64 5085 and 3360, 6098 and 5518), else eight.
-template<class T, int LOGL>
+template<class T, int LOGL, bool ANY>
 struct s3_cfg {
     using P                    = splan<LOGL>;
     static constexpr bool F64  = sizeof(T) == 8;
@@ -630,8 +729,11 @@ struct s3_cfg {
     static constexpr int  STAGE = M * RS * (int)sizeof(T);
     static constexpr int  XB   = X::size * (int)sizeof(cpx<T>);
     static constexpr int  BASE = smem_align16(2 * STAGE + XB);
-    static constexpr int  TAB  = stage_tw_smem_bytes<P, T>();
-    static constexpr bool SH   = stw_fits(BASE, TAB, MINB);    // stage factors in shared memory
+    // stage factors, in shared memory where they fit; the any-pack form has full
+    // tables instead where products would enter (a radix above 4 after the first)
+    static constexpr bool FULL = ANY && LOGL > 6;
+    static constexpr int  TAB  = FULL ? rows_tw_size<P>() * (int)sizeof(cpx<T>) : stage_tw_smem_bytes<P, T>();
+    static constexpr bool SH   = stw_fits(BASE, TAB, MINB);
     static constexpr int  SMEM = SH ? BASE + TAB : BASE;
     static_assert(XB >= STAGE, "staging fits the exchange buffer");
     static_assert((RS * (int)sizeof(T)) % 16 == 0, "rows stay 16-byte aligned");
@@ -644,8 +746,8 @@ struct s3_cfg {
 // natural order with packs of at most TT elements: one base per thread).
 // Bound by the load/store pipe and HBM like the default form.
 template<class T, int LOGL, int LP, bool ANY>
-__global__ void __launch_bounds__(s3_cfg<T, LOGL>::NT, s3_cfg<T, LOGL>::MINB) k_single3(v3_args a) {
-    using F             = s3_cfg<T, LOGL>;
+__global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>::MINB) k_single3(v3_args a) {
+    using F             = s3_cfg<T, LOGL, ANY>;
     using P             = typename F::P;
     using X             = typename F::X;
     constexpr int L     = P::L;
@@ -665,7 +767,9 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL>::NT, s3_cfg<T, LOGL>::MINB) k_
     __shared__ uint64_t full[2];
     cpx<T>*          xch = reinterpret_cast<cpx<T>*>(smem + 2 * F::STAGE);
     cpx<T>*          tws = reinterpret_cast<cpx<T>*>(smem + F::BASE);
-    const auto*      stw = SH ? tws : reinterpret_cast<const cpx<T>*>(a.stw);
+    const cpx<T>*    tab = static_cast<const cpx<T>*>(F::FULL ? a.rows : a.stw);
+    if constexpr (F::FULL) tab += rows_cfg<T, LOGL>::FULL16;
+    const cpx<T>*    stw = SH ? tws : tab;
     const T*         src = reinterpret_cast<const T*>(a.src);
     T*               dst = reinterpret_cast<T*>(a.dst);
     const int        tid = threadIdx.x;
@@ -683,7 +787,7 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL>::NT, s3_cfg<T, LOGL>::MINB) k_
     const bool       contig_in  = RS == 2 * L && a.src_stride == 2 * L && !cut;
     const bool       contig_out = RS == 2 * L && a.dst_stride == 2 * L;
 
-    if constexpr (SH) stage_tw_to_smem<P, T>(tws, a.stw, tid, NT);
+    if constexpr (SH) copy_table_to_smem<F::TAB>(tws, tab, tid, NT);
     if (tid == 0) {
         mbar_init(&full[0], 1);
         mbar_init(&full[1], 1);
@@ -754,7 +858,8 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL>::NT, s3_cfg<T, LOGL>::MINB) k_
         stage_compute_tab<P, 0>(v, t, stw);
         // a transform's TT <= 32 threads share one warp and its own exchange
         // block: its exchanges need only that warp's barrier
-        run_stages_tab<P, X, SH, (TT <= 32 ? -1 : 0)>(v, xch, m, t, stw);
+        if constexpr (F::FULL) run_stages_rows<P, X, SH, (TT <= 32 ? -1 : 0)>(v, xch, m, t, stw);
+        else run_stages_tab<P, X, SH, (TT <= 32 ? -1 : 0)>(v, xch, m, t, stw);
         const T sc  = T(a.scale);
         const T sim = a.conj_out ? -sc : sc;
         if (F::DIRECT && a.order_out == 0) {
@@ -831,15 +936,6 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL>::NT, s3_cfg<T, LOGL>::MINB) k_
 }    // namespace pcxg
 
 namespace pcxg {
-
-// Copy a table of BYTES bytes into shared memory (16-byte units; the caller syncs).
-template<int BYTES, class T>
-__device__ __forceinline__ void copy_table_to_smem(cpx<T>* dst, const void* src, int tid, int nt) {
-    static_assert(BYTES % 16 == 0, "table in 16-byte units");
-    const uint4* sp = reinterpret_cast<const uint4*>(src);
-    uint4*       dp = reinterpret_cast<uint4*>(dst);
-    for (int i = tid; i < BYTES / 16; i += nt) dp[i] = __ldg(sp + i);
-}
 
 // ---- full stage tables of the sub-transforms -------------------------------
 // For stage S >= 1 of splan P (Ns = 2^nsbits(S) butterfly positions, radix R)

@@ -20,19 +20,35 @@ static cudaError_t dispatch_rows(int log_n, const v3_args& a, cudaStream_t st, b
     }
 }
 
-template<class T, int LOGL>
-static cudaError_t rows_twiddles(void* out, cudaStream_t st, int* entries) {
-    using P  = typename rows_cfg<T, LOGL>::P;
-    *entries = rows_cfg<T, LOGL>::W ? stage_tw_size<P>() : 0;
-    if (!out || *entries == 0) return cudaSuccess;
+// Full tables of plan P at `out`.
+template<class P, class T>
+static cudaError_t full_tables(cpx<T>* out, cudaStream_t st) {
     for (int s = 1; s < P::NST; ++s) {
-        const int ns = 1 << P::nsbits(s), nq = stw_q(P::rbits(s));
-        k_stage_twiddles<T><<<(ns * nq + 255) / 256, 256, 0, st>>>(static_cast<cpx<T>*>(out) + stage_tw_offset<P>(s), ns,
-                                                                  P::rbits(s), P::nsbits(s) + P::rbits(s));
+        const int nsb = P::nsbits(s), rb = P::rbits(s);
+        k_rows_twiddles<T><<<((1 << (nsb + rb)) + 255) / 256, 256, 0, st>>>(out + rows_tw_offset<P>(s), nsb, rb);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+template<class T, int LOGL>
+static cudaError_t rows_twiddles(void* out, cudaStream_t st, int* entries) {
+    using F  = rows_cfg<T, LOGL>;
+    using P  = typename F::P;
+    *entries = F::FULL + rows_tw_size<P>();
+    if (!out) return cudaSuccess;
+    auto* o = static_cast<cpx<T>*>(out);
+    if constexpr (F::W) {
+        for (int s = 1; s < P::NST; ++s) {
+            const int ns = 1 << P::nsbits(s), rb = P::rbits(s), nq = stw_q(rb) * ns;
+            k_stage_twiddles<T><<<(nq + 255) / 256, 256, 0, st>>>(o + stage_tw_offset<P>(s), ns, rb, P::nsbits(s) + rb);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+        }
+        const cudaError_t e = full_tables<splan<LOGL>>(o + F::FULL16, st);
+        if (e != cudaSuccess) return e;
+    }
+    return full_tables<P>(o + F::FULL, st);
 }
 template<class T>
 static cudaError_t dispatch_twiddles(int log_n, void* out, cudaStream_t st, int* entries) {

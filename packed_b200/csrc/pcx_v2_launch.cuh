@@ -44,7 +44,7 @@ cudaError_t launch_rows(const v3_args& a, cudaStream_t st, bool attr_only) {
 
 template<class T, int LOGL, bool ANY>
 cudaError_t launch_single3(const v3_args& a, cudaStream_t st, int sms, bool attr_only) {
-    using F             = s3_cfg<T, LOGL>;
+    using F             = s3_cfg<T, LOGL, ANY>;
     constexpr int NT    = F::NT;
     constexpr int M     = F::M;
     constexpr int bytes = F::SMEM;

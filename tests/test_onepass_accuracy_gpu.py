@@ -34,3 +34,18 @@ def test_radix_32_stages(lg):
     pos = torch.as_tensor(np.asarray(O.order_pos(n, 1)).astype(np.int64), device="cuda")
     wide = _error(fft_unit(n), x, n, 8, 8)
     assert wide <= _error(fft_unit(n, order=fft_order.bit_reversed), x, n, 8, 8, pos)
+
+
+@pytest.mark.parametrize("dtype,lg", [(F32, lg) for lg in range(7, 14)] + [(F64, lg) for lg in range(7, 13)])
+@pytest.mark.parametrize("order", [fft_order.normal, fft_order.unordered])
+def test_other_packs(dtype, lg, order):
+    """Packs other than the default have full twiddle tables, as the general kernel had: a
+    smaller error than the default pack's, whose twiddles are products."""
+    n, p = 1 << lg, default_pack_size(dtype)
+    pos = torch.as_tensor(np.asarray(O.order_pos(n, int(order))).astype(np.int64), device="cuda")
+    x = torch.randn((1 << 21) >> lg, 2 * n, device="cuda", dtype=dtype, generator=torch.Generator("cuda").manual_seed(lg))
+    xp = x.reshape(x.shape[0], -1, 2, p).transpose(2, 3).reshape(x.shape).contiguous()    # the same elements interleaved
+    unit = fft_unit(n, dtype=dtype, order=order)
+    plain = _error(unit, x, n, p, p, pos)
+    for ps, pd in ((1, p), (p, 1), (1, 1)):
+        assert _error(unit, xp if ps == 1 else x, n, ps, pd, pos) < 0.998 * plain, (ps, pd)
