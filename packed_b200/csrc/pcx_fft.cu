@@ -202,7 +202,7 @@ static int fs_select(pcx_plan_s* p, const fs_variant& v) {
         // the default variant, which the kernel's other forms run, has their
         // twiddle table as well, plans of a permuted order a second one by
         // bit-reversed column
-        const size_t tw = (size_t)(n1 / 16 + 5) * n2;
+        const size_t tw = (size_t)(f64 ? fs_tw_rows<double>(v.l1, p->log_n) : fs_tw_rows<float>(v.l1, p->log_n)) * n2;
         const size_t nt = p->fs_def.mem ? 0 : (p->order != PCX_ORDER_NORMAL ? 2 : 1);
         PCX_CUDA_TRY(cudaMalloc(&c.mem, ((size_t)n1 + 2 * (size_t)n2 + f1 + f2 + nt * tw) * eb));
         char* b = static_cast<char*>(c.mem);
@@ -220,8 +220,8 @@ static int fs_select(pcx_plan_s* p, const fs_variant& v) {
             const unsigned grid = (unsigned)((tw + 255) / 256);
             void*          o    = b + ((size_t)n1 + 2 * (size_t)n2 + f1 + f2 + i * tw) * eb;
             (i ? c.twr : c.tw)  = o;
-            if (f64) k_fs_twiddles<double><<<grid, 256>>>(static_cast<cpx<double>*>(o), n1 / 16, v.l2, p->log_n, i);
-            else k_fs_twiddles<float><<<grid, 256>>>(static_cast<cpx<float>*>(o), n1 / 16, v.l2, p->log_n, i);
+            if (f64) k_fs_twiddles<double><<<grid, 256>>>(static_cast<cpx<double>*>(o), v.l1, v.l2, i);
+            else k_fs_twiddles<float><<<grid, 256>>>(static_cast<cpx<float>*>(o), v.l1, v.l2, i);
             e = cudaGetLastError();
         }
         if (e != cudaSuccess) {

@@ -298,19 +298,13 @@ __device__ __forceinline__ void apply_fourstep_tw(const cpx<T> (&v)[E], cpx<T> b
     });
 }
 
-// The same with u^1, u^2, u^4, u^8 and u^12 given (16 values): at most three
-// products per twiddle.
-template<class T, class F>
-__device__ __forceinline__ void apply_fourstep_tw5(const cpx<T> (&v)[16], cpx<T> base, const cpx<T> (&u)[5], F&& out) {
-    static_for<4>([&](auto ac) {
-        constexpr int a  = decltype(ac)::value;
-        cpx<T>        wa = base;
-        if constexpr (a > 0) wa = cmul(base, u[a + 1]);
-        const cpx<T>  w1 = cmul(wa, u[0]);
-        out(std::integral_constant<int, 4 * a>{}, cmul(v[4 * a], wa));
-        out(std::integral_constant<int, 4 * a + 1>{}, cmul(v[4 * a + 1], w1));
-        out(std::integral_constant<int, 4 * a + 2>{}, cmul(v[4 * a + 2], cmul(wa, u[1])));
-        out(std::integral_constant<int, 4 * a + 3>{}, cmul(v[4 * a + 3], cmul(w1, u[1])));
+// The same (16 values) with base*u^(B*a), a < 16/B, and then u^1..u^(B-1) given:
+// every twiddle an entry or the product of two.
+template<int B, class T, class F>
+__device__ __forceinline__ void apply_fourstep_ent(const cpx<T> (&v)[16], const cpx<T> (&w)[16 / B + B - 1], F&& out) {
+    static_for<16>([&](auto ic) {
+        constexpr int i = decltype(ic)::value, a = i / B, b = i % B;
+        out(ic, cmul(v[i], b == 0 ? w[a] : cmul(w[a], w[16 / B + b - 1])));
     });
 }
 

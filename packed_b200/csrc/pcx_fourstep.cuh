@@ -247,21 +247,32 @@ __device__ __forceinline__ void red_release_add(int* p, int v) {
     asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Twiddles of the forms other than FS_PLAIN: W_N^(k1*n2), k1 = t + i*TT, as one
-// table entry W_N^(t*n2) (row t) times powers of u = W_N^(TT*n2) (rows TT..
-// hold u^1, u^2, u^4, u^8 and u^12), all generated in FP64 and rounded once; a
-// row of N2 entries is read by neighbouring columns at once.  Against
-// FS_PLAIN's chains (two half-size tables and one power) this has the error of
-// the general kernels or less (2^15, there and back: 2.2e-7 for 3.6e-7 with
-// the chains and 3.0e-7 before) at the same speed; in FS_PLAIN it cost 0.7 %.
+// Twiddles of the forms other than FS_PLAIN: W_N^(k1*n2), k1 = t + i*TT, i =
+// B*a + b, as W_N^((t + B*a*TT)*n2) (row a*TT + t) times u^b, u = W_N^(TT*n2)
+// (row N1/B + b - 1), all generated in FP64 and rounded once; a row of N2 entries
+// is read by neighbouring columns at once.  The fewer of them are products the
+// smaller the error and the more entries a thread reads (9 with B = 2, 7 with
+// 4): B = 2 where B = 4 would be less accurate than the general kernels (product
+// of two half-size tables).  Error against FP64, interleaved to packed: 2^15
+// general 1.439e-7, B = 4 1.447e-7, B = 2 1.434e-7, one entry times powers of u
+// 1.472e-7; 2^17 1.573e-7, 1.573e-7, -, 1.597e-7.  GB/s, 512 MB: 2^15 3292
+// with powers of u, 3231 with B = 4 and 3210 with 2; 2^20 2800, 2672 and 2542.
 template<class T>
-__global__ void k_fs_twiddles(cpx<T>* out, int tt, int log_n2, int log_n, int permuted) {
+__host__ __device__ constexpr int fs_tw_group(int log_n) {
+    return sizeof(T) == 4 && log_n <= 16 ? 2 : 4;
+}
+template<class T>
+__host__ __device__ constexpr int fs_tw_rows(int log_n1, int log_n) {
+    return (1 << log_n1) / fs_tw_group<T>(log_n) + fs_tw_group<T>(log_n) - 1;
+}
+template<class T>
+__global__ void k_fs_twiddles(cpx<T>* out, int log_n1, int log_n2, int permuted) {
+    const int log_n = log_n1 + log_n2, tt = 1 << (log_n1 - 4), grp = fs_tw_group<T>(log_n);
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (tt + 5) << log_n2) return;
-    const int       row = q >> log_n2, r = q & ((1 << log_n2) - 1);
+    if (q >= fs_tw_rows<T>(log_n1, log_n) << log_n2) return;
+    const int       row = q >> log_n2, r = q & ((1 << log_n2) - 1), bases = 16 / grp * tt;
     const long long n2   = permuted ? (int)brev(r, log_n2) : r;
-    const int       j    = row - tt;
-    const long long mult = j < 0 ? row : (long long)tt * (j == 4 ? 12 : 1 << j);
+    const long long mult = row < bases ? row % tt + grp * tt * (row / tt) : tt * (row - bases + 1);
     const long long e    = (n2 * mult) & ((1LL << log_n) - 1);
     double          s, c;
     sincospi(2.0 * (double)e / (double)(1LL << log_n), &s, &c);
@@ -553,7 +564,8 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
         };
         // column tile: the four-step twiddle inputs are requested before the
         // tile's data is waited for, and used after the stages
-        cpx<T> th{}, tl{}, tu[FORM == FS_PLAIN ? 1 : 5]{};
+        constexpr int B = fs_tw_group<T>(LOGN1 + LOGN2), NE = 16 / B + B - 1;
+        cpx<T> th{}, tl{}, tu[FORM == FS_PLAIN ? 1 : NE]{};
         if (!it.row) {
             const int n2 = it.tile * C + tid % C;    // FS_IN: the column's place in the scratch
             if constexpr (FORM == FS_PLAIN) {
@@ -563,10 +575,9 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
                 tu[0]             = ldg_cpx(reinterpret_cast<const cpx<T>*>(a.tw_b) + n2);
             } else {
                 const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw) + n2;
-                th               = ldg_cpx(tw + (tid / C) * N2);
-                static_for<5>([&](auto qc) {
+                static_for<NE>([&](auto qc) {
                     constexpr int q = decltype(qc)::value;
-                    tu[q]           = ldg_cpx(tw + (P1::TT + q) * N2);
+                    tu[q] = ldg_cpx(tw + (q < 16 / B ? q * P1::TT + tid / C : 16 / B * P1::TT + q - 16 / B) * N2);
                 });
             }
         }
@@ -629,7 +640,7 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
                 // exchange layout is the box the publisher stores
                 auto put = [&](auto ic, cpx<T> o) { xch[F::X1::idx(c, t + decltype(ic)::value * TT)] = o; };
                 if constexpr (FORM == FS_PLAIN) apply_fourstep_tw(v, cmul(th, tl), tu[0], put);
-                else apply_fourstep_tw5(v, th, tu, put);
+                else apply_fourstep_ent<B>(v, tu, put);
                 staged();
             } else {
                 if (!mbar_wait_bounded(&slotok[s], (colpar >> s) & 1u)) {
@@ -646,7 +657,7 @@ __global__ void __launch_bounds__(fs_cfg<T, LOGN1, LOGN2, MINB, ST_>::NT + 64, M
                         dst[(long long)i * TT * N2] = o;
                     };
                     if constexpr (FORM == FS_PLAIN) apply_fourstep_tw(v, cmul(th, tl), tu[0], put);
-                    else apply_fourstep_tw5(v, th, tu, put);
+                    else apply_fourstep_ent<B>(v, tu, put);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&written[s]);
                 }

@@ -1,4 +1,4 @@
-"""Error of the one-pass FFT's faster forms against FP64, on the same data as the
+"""Error of the faster FFT forms against FP64, on the same data as the
 forms that they stand beside: it may be no larger."""
 import numpy as np
 import pytest
@@ -49,3 +49,17 @@ def test_other_packs(dtype, lg, order):
     plain = _error(unit, x, n, p, p, pos)
     for ps, pd in ((1, p), (p, 1), (1, 1)):
         assert _error(unit, xp if ps == 1 else x, n, ps, pd, pos) < 0.998 * plain, (ps, pd)
+
+
+@pytest.mark.parametrize("lg", range(15, 21))
+@pytest.mark.parametrize("order", [fft_order.normal, fft_order.unordered])
+def test_fourstep_forms(lg, order, monkeypatch):
+    """The one-launch four-step's forms against the general two-launch kernels, whose twiddles are
+    one entry or the product of two (0.4 % for the data's chance)."""
+    n = 1 << lg
+    pos = torch.as_tensor(np.asarray(O.order_pos(n, int(order))).astype(np.int64), device="cuda")
+    x = torch.randn((1 << 22) >> lg, 2 * n, device="cuda", generator=torch.Generator("cuda").manual_seed(lg))
+    unit = fft_unit(n, order=order)
+    one = _error(unit, x, n, 1, 1, pos)
+    monkeypatch.setenv("PCX_FOURSTEP", "chunked")
+    assert one < 1.004 * _error(unit, x, n, 1, 1, pos)
