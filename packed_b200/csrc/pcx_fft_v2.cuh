@@ -733,6 +733,17 @@ struct s3_cfg {
     static_assert((RS * (int)sizeof(T)) % 16 == 0, "rows stay 16-byte aligned");
 };
 
+// Bytes that a short row of `len` elements at pack width 2^lp is copied with: up
+// to the 16-byte unit of its last real, which lies inside its last pack; but FP32
+// rows at width 1 of odd length end half a unit earlier, and their last element is
+// read by its thread.
+template<class T>
+__host__ __device__ constexpr uint32_t single3_row_bytes(int len, int lp) {
+    const uint32_t last = ((((uint32_t)len - 1) >> lp) << (lp + 1)) + (((uint32_t)len - 1) & ((1u << lp) - 1u));
+    const uint32_t end  = (last + (1u << lp) + 1) * (uint32_t)sizeof(T);
+    return lp == 0 ? end & ~15u : (end + 15) & ~15u;
+}
+
 // ANY: source and destination packs of any width up to N (each its own, given
 // at run time) and rows shorter than N.  The row is the same 2*N contiguous
 // reals at every width and lds_swapped / sts_swapped stay free of bank
@@ -774,10 +785,10 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>
     const int        lpd  = ANY ? a.lp_dst : LP;
     const int        pks  = 1 << lps;
     const int        pkd  = 1 << lpd;
-    // short rows: copied up to the 16-byte unit of the last valid real
+    // short rows end where the caller's storage may end
     const bool       cut  = ANY && a.src_len < L;
-    const uint32_t   rowb = cut ? ((pk_re((uint32_t)a.src_len - 1, lps) + pks + 1) * (uint32_t)sizeof(T) + 15) & ~15u
-                                : (uint32_t)ROWB;
+    const uint32_t   rowb = cut ? single3_row_bytes<T>(a.src_len, lps) : (uint32_t)ROWB;
+    const bool       tail = cut && lps == 0 && rowb < (uint32_t)a.src_len * 2 * (uint32_t)sizeof(T);
     const bool       contig_in  = RS == 2 * L && a.src_stride == 2 * L && !cut;
     const bool       contig_out = RS == 2 * L && a.dst_stride == 2 * L;
 
@@ -796,7 +807,7 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>
         mbar_arrive_expect_tx(&full[s], (uint32_t)rows * rowb);
         if (contig_in) {
             bulk_g2s(buf, g, (uint32_t)rows * rowb, &full[s]);
-        } else {
+        } else if (!ANY || rowb > 0) {
             for (int r = 0; r < rows; ++r) bulk_g2s(buf + r * RS, g + r * a.src_stride, rowb, &full[s]);
         }
     };
@@ -832,6 +843,10 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>
             static_for<E>([&](auto ic) {
                 constexpr int i = decltype(ic)::value;
                 if (t + i * TT >= a.src_len) v[i] = {T(0), T(0)};
+                if (tail && t + i * TT == a.src_len - 1 && tile * M + m < a.batch) {
+                    const T* g = src + (tile * M + m) * a.src_stride + 2 * (t + i * TT);
+                    v[i]       = {g[0], g[1]};
+                }
             });
         }
         fence_proxy_async_smem();
