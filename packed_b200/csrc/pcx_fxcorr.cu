@@ -152,7 +152,7 @@ namespace {
 template<int LOGN>
 int launch_xci(const xci_args& a, cudaStream_t st, int sms, bool attr_only) {
     using C   = xci_cfg<LOGN>;
-    auto kern = k_fxcorr_ip<LOGN>;
+    auto kern = a.base.inplace ? k_fxcorr_ip<LOGN, true> : k_fxcorr_ip<LOGN, false>;
     PCX_CUDA_TRY(smem_attr_cached(reinterpret_cast<const void*>(kern), C::SMEM));
     if (attr_only) return PCX_OK;
     const long long grid = std::max<long long>(1, std::min<long long>(a.base.total, (long long)C::MINB * sms));
@@ -242,7 +242,10 @@ int init_xci(pcx_fxcorr_s* h) {
     h->xi_tw = tw;
     int grid = 0;
     if (int rc = launch_xci_kg<LOGN>(xci_kg_args{}, 0, h->sms, &grid)) return rc;
-    return launch_xci<LOGN>(xci_args{}, 0, 0, true);
+    xci_args a{};
+    if (int rc = launch_xci<LOGN>(a, 0, 0, true)) return rc;
+    a.base.inplace = 1;
+    return launch_xci<LOGN>(a, 0, 0, true);
 }
 
 int check_pack(int pack) {

@@ -24,10 +24,11 @@
 // the next one as soon as the last step has read this one.
 // Bound by issue and the shared-memory pipe.  32 channels x 2^20 samples, 4096
 // taps, in place: 395 us with the two-step form, 260 us; relative error against
-// FP64 4.0e-7 and 2.8e-7.  8192 points, 16 x 2^20, 2048 taps: 220 and 115 us.
+// FP64 4.0e-7 and 2.8e-7.  8192 points, 16 x 2^20, 2048 taps: 220 and 121 us.
 //
-// Out of place, windows go round the blocks.  In place, a window's outputs
-// overwrite samples that earlier blocks' windows read: they are claimed in
+// Out of place, windows go round the blocks: calls that overlap share nothing
+// (claimed from a counter 260 us, so 272 us, 18.6 rounds being 19).  In place
+// (compiled apart: in one kernel 264 us), a window's outputs overwrite samples that earlier blocks' windows read: they are claimed in
 // order, each block publishes "window loaded" (flags[item], cleared before each
 // launch), and every warp waits (bounded, about a second) for its predecessors
 // before it writes, as in the other forms.
@@ -128,7 +129,7 @@ __device__ __forceinline__ void xci_dft_b(cpx<float> (&v)[32]) {
     }
 }
 
-template<int LOGN>
+template<int LOGN, bool INPLACE>
 __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxcorr_ip(xci_args A) {
     using F            = xci_cfg<LOGN>;
     constexpr int N    = F::N;
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
     }
     tw2[tid] = ldg_cpx(reinterpret_cast<const cpx<float>*>(A.tw) + N + tid);
     if (tid == 0) {
-        s_item = a.inplace ? atomicAdd(a.counter, 1u) : blockIdx.x;
+        s_item = INPLACE ? atomicAdd(a.counter, 1u) : blockIdx.x;
         mbar_init(&full, 1);
         fence_barrier_init();
     }
@@ -228,13 +229,9 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
             break;    // every thread leaves together; nothing else is in flight
         }
         phase ^= 1;
-        if (tid == 0) {
-            if (a.inplace) {
-                st_release(a.flags + item, 1u);    // this window is loaded
-                s_item = atomicAdd(a.counter, 1u);
-            } else {
-                s_item = item + gridDim.x;
-            }
+        if (INPLACE && tid == 0) {
+            st_release(a.flags + item, 1u);    // this window is loaded
+            s_item = atomicAdd(a.counter, 1u);
         }
         dft<32, 1, 0>(v);
         xci_mul<false>(v, tcol, false);
@@ -272,7 +269,7 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
         // in place: the first look at the flags, so that the wait below rarely has to read one
         const unsigned blk  = item - ch * nblk;
         bool           seen = true;
-        if (a.inplace && lane < a.hwait && lane < blk) seen = ld_acquire(a.flags + (item - 1 - lane)) != 0u;
+        if (INPLACE && lane < a.hwait && lane < blk) seen = ld_acquire(a.flags + (item - 1 - lane)) != 0u;
         __syncthreads();
         // ---------------- times W_16B^(c kb), back over kb
         static_for<32>([&](auto ic) {
@@ -290,11 +287,11 @@ __global__ void __launch_bounds__(xci_cfg<LOGN>::NT, xci_cfg<LOGN>::MINB) k_fxco
         static_for<32>([&](auto ic) { v[decltype(ic)::value] = p1[decltype(ic)::value * B * RL]; });
         fence_proxy_async_smem();
         __syncthreads();    // the window is read: the next one may land
-        const unsigned next = s_item;
+        const unsigned next = INPLACE ? s_item : item + gridDim.x;
         if (tid < 32) copy(next);
         xci_mul<false>(v, tcol, false);
         dft<32, 1, 0>(v);
-        if (a.inplace) {
+        if constexpr (INPLACE) {
             // the outputs overwrite samples of the hwait previous blocks' windows;
             // a warp that gives up stores nothing, and the block leaves at the
             // next vote
