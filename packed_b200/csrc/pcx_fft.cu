@@ -364,11 +364,15 @@ static int plan_init_tables(pcx_plan_s* p) {
             }
         }
     }
-    int er = 0;
-    PCX_CUDA_TRY(pcx_rows_twiddles(f64, log_n, nullptr, 0, &er));
-    if (er > 0 && (!p->two_pass || p->stw_one)) {
-        PCX_CUDA_TRY(cudaMalloc(&p->stw_rows, (size_t)er * eb));
-        PCX_CUDA_TRY(pcx_rows_twiddles(f64, log_n, p->stw_rows, 0, &er));
+    rows_sections at;
+    PCX_CUDA_TRY(pcx_rows_twiddles(f64, log_n, nullptr, 0, &at));
+    if (at.entries > 0 && (!p->two_pass || p->stw_one)) {
+        PCX_CUDA_TRY(cudaMalloc(&p->stw_rows, (size_t)at.entries * eb));
+        PCX_CUDA_TRY(pcx_rows_twiddles(f64, log_n, p->stw_rows, 0, &at));
+        const char* base = static_cast<const char*>(p->stw_rows);
+        p->rows_fac      = at.factors ? base : nullptr;
+        p->s3_any        = base + (size_t)at.single3 * eb;
+        p->rows_any      = base + (size_t)at.rows * eb;
     }
     PCX_CUDA_TRY(cudaDeviceSynchronize());
     return PCX_OK;
@@ -830,8 +834,6 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         t3.order_in   = io.order_in;
         t3.order_out  = io.order_out;
         t3.scale      = io.scale;
-        t3.stw        = stw;
-        t3.rows       = p->stw_rows;
         t3.error      = p->err;
         t3.lp_src     = io.lp_src;
         t3.lp_dst     = io.lp_dst;
@@ -844,10 +846,12 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         // natural order from 256 points on (FP64: 128) goes straight through
         // registers; k_single3 is faster below and takes the other orders
         if (natural && p->log_n >= 7 && (f64 || p->log_n >= 8 || !tma)) {
+            t3.stw              = !plain ? p->rows_any : p->rows_fac ? p->rows_fac : stw;
             const cudaError_t e = (plain ? pcx_rows : pcx_rows_any)(f64, p->log_n, t3, st, false);
             if (e != cudaErrorNotSupported) return e;
         }
         if (!tma) return cudaErrorNotSupported;
+        t3.stw = !plain && p->s3_any ? p->s3_any : stw;
         return plain ? pcx_v3_single(f64, p->log_n, t3, st, p->sms, false)
                      : pcx_v3_single_any(f64, p->log_n, t3, st, p->sms, false);
     };

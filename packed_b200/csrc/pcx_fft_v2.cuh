@@ -351,8 +351,7 @@ struct v3_args {
     int         order_in;
     int         order_out;
     double      scale;
-    const void* stw;      // factors of the stage twiddles
-    const void* rows;     // the tables of pcx_rows_twiddles
+    const void* stw;      // stage twiddles: factors, or full tables (rows_cfg, s3_cfg)
     int*        error;    // set when a bounded wait gives up
     // the any-pack forms only (k_rows and k_single3 with ANY):
     int         lp_src;     // log2 pack widths
@@ -469,8 +468,8 @@ struct rows_cfg {
     static constexpr int MINB = (sizeof(T) == 8 || W ? 512 : 1024) / NT;
     using X                   = std::conditional_t<W, xch_blocked32<P::L, M>, xch_blocked<P::L, M>>;
     static constexpr int SMEM = X::size * (int)sizeof(cpx<T>);
-    // v3_args::rows: with 32 points per thread the factors, then the full
-    // tables of 16 points per thread (k_single3's) and, at FULL, of its own
+    // sections of pcx_rows_twiddles: with 32 points per thread the factors, then
+    // the full tables of 16 points per thread (k_single3's) and, at FULL, its own
     static constexpr int FULL16 = W ? stage_tw_size<P>() : 0;
     static constexpr int FULL   = W ? FULL16 + rows_tw_size<splan<LOGL>>() : 0;
 };
@@ -533,11 +532,9 @@ __global__ void __launch_bounds__(rows_cfg<T, LOGL>::NT, rows_cfg<T, LOGL>::MINB
     if (a.conj_in) static_for<E>([&](auto ic) { v[decltype(ic)::value].im = -v[decltype(ic)::value].im; });
     constexpr int BAR = TT <= 32 ? -1 : 0;
     stage_compute_tab<P, 0>(v, t, static_cast<const cpx<T>*>(nullptr));
-    if constexpr (ANY) {
-        run_stages_rows<P, typename F::X, false, BAR>(v, xch, m, t, static_cast<const cpx<T>*>(a.rows) + F::FULL);
-    } else {
-        run_stages_tab<P, typename F::X, false, BAR>(v, xch, m, t, static_cast<const cpx<T>*>(F::W ? a.rows : a.stw));
-    }
+    const auto* stw = static_cast<const cpx<T>*>(a.stw);
+    if constexpr (ANY) run_stages_rows<P, typename F::X, false, BAR>(v, xch, m, t, stw);    // full tables
+    else run_stages_tab<P, typename F::X, false, BAR>(v, xch, m, t, stw);
     if (!live) return;
     const T sc  = T(a.scale);
     const T sim = a.conj_out ? -sc : sc;
@@ -772,9 +769,7 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>
     __shared__ uint64_t full[2];
     cpx<T>*          xch = reinterpret_cast<cpx<T>*>(smem + 2 * F::STAGE);
     cpx<T>*          tws = reinterpret_cast<cpx<T>*>(smem + F::BASE);
-    const cpx<T>*    tab = static_cast<const cpx<T>*>(F::FULL ? a.rows : a.stw);
-    if constexpr (F::FULL) tab += rows_cfg<T, LOGL>::FULL16;
-    const cpx<T>*    stw = SH ? tws : tab;
+    const cpx<T>*    stw = SH ? tws : static_cast<const cpx<T>*>(a.stw);
     const T*         src = reinterpret_cast<const T*>(a.src);
     T*               dst = reinterpret_cast<T*>(a.dst);
     const int        tid = threadIdx.x;
@@ -792,7 +787,7 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>
     const bool       contig_in  = RS == 2 * L && a.src_stride == 2 * L && !cut;
     const bool       contig_out = RS == 2 * L && a.dst_stride == 2 * L;
 
-    if constexpr (SH) copy_table_to_smem<F::TAB>(tws, tab, tid, NT);
+    if constexpr (SH) copy_table_to_smem<F::TAB>(tws, a.stw, tid, NT);
     if (tid == 0) {
         mbar_init(&full[0], 1);
         mbar_init(&full[1], 1);

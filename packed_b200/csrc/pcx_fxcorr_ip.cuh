@@ -28,10 +28,11 @@
 //
 // Out of place, windows go round the blocks: calls that overlap share nothing
 // (claimed from a counter 260 us, so 272 us, 18.6 rounds being 19).  In place
-// (compiled apart: in one kernel 264 us), a window's outputs overwrite samples that earlier blocks' windows read: they are claimed in
-// order, each block publishes "window loaded" (flags[item], cleared before each
-// launch), and every warp waits (bounded, about a second) for its predecessors
-// before it writes, as in the other forms.
+// (compiled apart: in one kernel 264 us), a window's outputs overwrite samples
+// that earlier blocks' windows read: they are claimed in order, each block
+// publishes "window loaded" (flags[item], cleared before each launch), and every
+// warp waits (bounded, about a second) for its predecessors before it writes, as
+// in the other forms.
 #pragma once
 
 #include "pcx_fft_v2.cuh"

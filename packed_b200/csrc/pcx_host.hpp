@@ -176,7 +176,10 @@ struct pcx_plan_s {
     void*  stw2     = nullptr;    // stage twiddles of the row pass (N2)
     void*  tw_b     = nullptr;    // W_{16*N2}^m, m < 16*N2
     void*  stw_one  = nullptr;    // stage twiddles of a one-pass form of a two-pass size
-    void*  stw_rows = nullptr;    // one-pass sizes from 128 points on: pcx_rows_twiddles
+    void*  stw_rows = nullptr;    // one-pass sizes from 128 points on: pcx_rows_twiddles' tables
+    const void* rows_fac = nullptr;    // factors of k_rows' default form (null: stwL serves)
+    const void* rows_any = nullptr;    // full tables of k_rows' any-pack form
+    const void* s3_any   = nullptr;    // full tables of k_single3's (null: below 128 points)
     void*  fst      = nullptr;    // one-launch four-step: full stage tables of N1 then N2 (one allocation)
     void*  fst1     = nullptr;
     void*  fst2     = nullptr;
@@ -241,10 +244,19 @@ cudaError_t pcx_tc_list_launch(int precision, const pcxg::tc_item* items, int ni
 
 // Hot-path launches (pcx_v2_*.cu); cudaErrorNotSupported when no variant exists.
 cudaError_t pcx_rows(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, bool attr_only);
-// Tables of k_rows and of k_single3's any-pack form: full stage tables and, where
-// k_rows runs 32 points per thread, its stage factors (rows_cfg; out == nullptr
-// only counts the entries).
-cudaError_t pcx_rows_twiddles(bool f64, int log_n, void* out, cudaStream_t st, int* entries);
+namespace pcxg {
+// Tables of k_rows and of k_single3's any-pack form, in one allocation (offsets
+// in complex entries): full stage tables and, where k_rows runs 32 points per
+// thread, its stage factors first.
+struct rows_sections {
+    int  entries = 0;        // 0: the size has none
+    bool factors = false;    // factors at 0
+    int  single3 = 0;        // k_single3's full tables
+    int  rows    = 0;        // k_rows'
+};
+}
+// out == nullptr only gives the sections.
+cudaError_t pcx_rows_twiddles(bool f64, int log_n, void* out, cudaStream_t st, pcxg::rows_sections* at);
 cudaError_t pcx_rows_any(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, bool attr_only);
 cudaError_t pcx_v3_single(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, int sms, bool attr_only);
 // the same kernel for any pack widths and short rows

@@ -32,10 +32,10 @@ static cudaError_t full_tables(cpx<T>* out, cudaStream_t st) {
     return cudaSuccess;
 }
 template<class T, int LOGL>
-static cudaError_t rows_twiddles(void* out, cudaStream_t st, int* entries) {
-    using F  = rows_cfg<T, LOGL>;
-    using P  = typename F::P;
-    *entries = F::FULL + rows_tw_size<P>();
+static cudaError_t rows_twiddles(void* out, cudaStream_t st, rows_sections* at) {
+    using F = rows_cfg<T, LOGL>;
+    using P = typename F::P;
+    *at     = {F::FULL + rows_tw_size<P>(), F::W, F::FULL16, F::FULL};
     if (!out) return cudaSuccess;
     auto* o = static_cast<cpx<T>*>(out);
     if constexpr (F::W) {
@@ -51,26 +51,26 @@ static cudaError_t rows_twiddles(void* out, cudaStream_t st, int* entries) {
     return full_tables<P>(o + F::FULL, st);
 }
 template<class T>
-static cudaError_t dispatch_twiddles(int log_n, void* out, cudaStream_t st, int* entries) {
-    *entries = 0;
+static cudaError_t dispatch_twiddles(int log_n, void* out, cudaStream_t st, rows_sections* at) {
+    *at = {};
     switch (log_n) {
-    case 7: return rows_twiddles<T, 7>(out, st, entries);
-    case 8: return rows_twiddles<T, 8>(out, st, entries);
-    case 9: return rows_twiddles<T, 9>(out, st, entries);
-    case 10: return rows_twiddles<T, 10>(out, st, entries);
-    case 11: return rows_twiddles<T, 11>(out, st, entries);
-    case 12: return rows_twiddles<T, 12>(out, st, entries);
-    case 13: return rows_twiddles<T, 13>(out, st, entries);
-    case 14: return rows_twiddles<T, 14>(out, st, entries);
+    case 7: return rows_twiddles<T, 7>(out, st, at);
+    case 8: return rows_twiddles<T, 8>(out, st, at);
+    case 9: return rows_twiddles<T, 9>(out, st, at);
+    case 10: return rows_twiddles<T, 10>(out, st, at);
+    case 11: return rows_twiddles<T, 11>(out, st, at);
+    case 12: return rows_twiddles<T, 12>(out, st, at);
+    case 13: return rows_twiddles<T, 13>(out, st, at);
+    case 14: return rows_twiddles<T, 14>(out, st, at);
     default: return cudaSuccess;
     }
 }
 
 }    // namespace pcxg
 
-cudaError_t pcx_rows_twiddles(bool f64, int log_n, void* out, cudaStream_t st, int* entries) {
-    return f64 ? pcxg::dispatch_twiddles<double>(log_n, out, st, entries)
-               : pcxg::dispatch_twiddles<float>(log_n, out, st, entries);
+cudaError_t pcx_rows_twiddles(bool f64, int log_n, void* out, cudaStream_t st, pcxg::rows_sections* at) {
+    return f64 ? pcxg::dispatch_twiddles<double>(log_n, out, st, at)
+               : pcxg::dispatch_twiddles<float>(log_n, out, st, at);
 }
 
 cudaError_t pcx_rows(bool f64, int log_n, const pcxg::v3_args& a, cudaStream_t st, bool attr_only) {
