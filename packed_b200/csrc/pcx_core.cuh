@@ -186,6 +186,24 @@ __device__ __forceinline__ void dft32_4x8(cpx<T> (&v)[32]) {
     static_for<32>([&](auto qc) { v[decltype(qc)::value] = t[decltype(qc)::value]; });
 }
 
+// 16 values as 4 x 4 in the same way.
+template<class T>
+__device__ __forceinline__ void dft16_4x4(cpx<T> (&v)[16]) {
+    static_for<4>([&](auto nc) { dft<4, 4, decltype(nc)::value>(v); });
+    cpx<T> t[16];
+    static_for<4>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        cpx<T>        a, b, c, d;
+        addsub_w<4 * k>(v[4 * k], v[4 * k + 2], a, b);
+        addsub_w<6 * k>(mulw<2 * k>(v[4 * k + 1]), v[4 * k + 3], c, d);
+        t[k]      = a + c;
+        t[k + 8]  = a - c;
+        t[k + 4]  = {b.re + d.im, b.im - d.re};
+        t[k + 12] = {b.re - d.im, b.im + d.re};
+    });
+    static_for<16>([&](auto qc) { v[decltype(qc)::value] = t[decltype(qc)::value]; });
+}
+
 // ---- stage plan for an L = 2^LOGL point Stockham FFT ---------------------
 // Radix-16 stages first (stage 0 carries no twiddles), remainder radix last.
 // Each thread owns E values (E = EPT, or L when smaller); in every stage

@@ -845,7 +845,7 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
         const bool tma       = batch == 1 || (sstride % vreals == 0 && dstride % vreals == 0);
         // natural order from 256 points on (FP64: 128) goes straight through
         // registers; k_single3 is faster below and takes the other orders
-        if (natural && p->log_n >= 7 && (f64 || p->log_n >= 8 || !tma)) {
+        if (natural && p->log_n >= 7 && (f64 || p->log_n >= 8 || !tma) && !(p->narrow && p->rows_fac)) {
             t3.stw              = !plain ? p->rows_any : p->rows_fac ? p->rows_fac : stw;
             const cudaError_t e = (plain ? pcx_rows : pcx_rows_any)(f64, p->log_n, t3, st, false);
             if (e != cudaErrorNotSupported) return e;

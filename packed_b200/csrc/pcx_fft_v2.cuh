@@ -118,15 +118,16 @@ __device__ __forceinline__ void load_stage_tw(cpx<T>* f, int t, const cpx<T>* __
     });
 }
 
-// The transform of a butterfly's R values.
-template<int R, class T>
+// The transform of a butterfly's R values (FINE: 16 as 4 x 4).
+template<bool FINE, int R, class T>
 __device__ __forceinline__ void stage_dft(cpx<T> (&a)[R]) {
     if constexpr (R == 32) dft32_4x8(a);
+    else if constexpr (R == 16 && FINE) dft16_4x4(a);
     else dft<R, 1, 0>(a);
 }
 
 // Butterflies of stage S >= 1 with preloaded table factors.
-template<class P, int S, class T, int E>
+template<class P, int S, bool FINE = false, class T, int E>
 __device__ __forceinline__ void stage_apply_tw(cpx<T> (&v)[E], const cpx<T>* f) {
     constexpr int RB = P::rbits(S);
     constexpr int R  = 1 << RB;
@@ -140,7 +141,7 @@ __device__ __forceinline__ void stage_apply_tw(cpx<T> (&v)[E], const cpx<T>* f) 
             constexpr int j = decltype(jc)::value + 1;
             a[j]            = cmul(v[g + j * G], stw_factor<RB, j>(f + g * Q));
         });
-        stage_dft(a);
+        stage_dft<FINE>(a);
         static_for<R>([&](auto jc) {
             constexpr int j = decltype(jc)::value;
             v[g + j * G]    = a[j];
@@ -148,13 +149,13 @@ __device__ __forceinline__ void stage_apply_tw(cpx<T> (&v)[E], const cpx<T>* f) 
     });
 }
 
-template<class P, int S, class T, int E>
+template<class P, int S, bool FINE = false, class T, int E>
 __device__ __forceinline__ void stage_compute_tab(cpx<T> (&v)[E], int t, const cpx<T>* __restrict__ stw) {
     constexpr int NSB = P::nsbits(S);
     if constexpr (NSB > 0) {
         cpx<T> f[(E >> P::rbits(S)) * stw_q(P::rbits(S))];
         load_stage_tw<P, S>(f, t, stw);
-        stage_apply_tw<P, S>(v, f);
+        stage_apply_tw<P, S, FINE>(v, f);
     } else {
         constexpr int R = 1 << P::rbits(S);
         constexpr int G = E / R;
@@ -165,7 +166,7 @@ __device__ __forceinline__ void stage_compute_tab(cpx<T> (&v)[E], int t, const c
                 constexpr int j = decltype(jc)::value;
                 a[j]            = v[g + j * G];
             });
-            stage_dft(a);
+            stage_dft<FINE>(a);
             static_for<R>([&](auto jc) {
                 constexpr int j = decltype(jc)::value;
                 v[g + j * G]    = a[j];
@@ -386,44 +387,56 @@ __global__ void k_rows_twiddles(cpx<T>* out, int nsb, int rb) {
     out[q] = {T(c), T(-s)};
 }
 
+// Butterflies of stage S >= 1 with its full table `tab` (SH: in shared memory).
+template<class P, int S, bool SH, bool FINE, class T, int E>
+__device__ __forceinline__ void stage_apply_rows(cpx<T> (&v)[E], int t, const cpx<T>* __restrict__ tab) {
+    constexpr int NSB = P::nsbits(S);
+    constexpr int R   = 1 << P::rbits(S);
+    constexpr int G   = E / R;
+    static_for<G>([&](auto gc) {
+        constexpr int g  = decltype(gc)::value;
+        const int     k  = (t + g * P::TT) & ((1 << NSB) - 1);
+        const cpx<T>* tw = tab + 2 * k;
+        cpx<T>        a[R];
+        static_for<R / 2>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            cpx<T>        w0, w1;
+            ld2<SH>(tw + (q << (NSB + 1)), w0, w1);
+            a[2 * q]     = q == 0 ? v[g] : cmul(v[g + 2 * q * G], w0);
+            a[2 * q + 1] = cmul(v[g + (2 * q + 1) * G], w1);
+        });
+        stage_dft<FINE>(a);
+        static_for<R>([&](auto jc) {
+            constexpr int j = decltype(jc)::value;
+            v[g + j * G]    = a[j];
+        });
+    });
+}
+
+// The exchange between stages S and S + 1.
+template<class P, int S, class X, int BARN, class T, int E>
+__device__ __forceinline__ void stage_exchange(cpx<T> (&v)[E], cpx<T>* xch, int m, int t) {
+    constexpr int G = E / (1 << P::rbits(S));
+    xch_sync<BARN>();
+    static_for<E>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        xch[X::idx(m, stage_out_index<P, S>(t, i % G, i / G))] = v[i];
+    });
+    xch_sync<BARN>();
+    static_for<E>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        v[i]            = xch[X::idx(m, t + i * P::TT)];
+    });
+}
+
 // Stages 1..NST-1 with these tables (SH: in shared memory).
 template<class P, class X, bool SH, int BARN, class T, int E>
 __device__ __forceinline__ void run_stages_rows(cpx<T> (&v)[E], cpx<T>* xch, int m, int t,
                                                 const cpx<T>* __restrict__ tab) {
     static_for<P::NST - 1>([&](auto sc) {
         constexpr int S = decltype(sc)::value;
-        constexpr int G = E / (1 << P::rbits(S));
-        xch_sync<BARN>();
-        static_for<E>([&](auto ic) {
-            constexpr int i = decltype(ic)::value;
-            xch[X::idx(m, stage_out_index<P, S>(t, i % G, i / G))] = v[i];
-        });
-        xch_sync<BARN>();
-        static_for<E>([&](auto ic) {
-            constexpr int i = decltype(ic)::value;
-            v[i]            = xch[X::idx(m, t + i * P::TT)];
-        });
-        constexpr int NSB = P::nsbits(S + 1);
-        constexpr int R   = 1 << P::rbits(S + 1);
-        constexpr int GN  = E / R;
-        static_for<GN>([&](auto gc) {
-            constexpr int g  = decltype(gc)::value;
-            const int     k  = (t + g * P::TT) & ((1 << NSB) - 1);
-            const cpx<T>* tw = tab + rows_tw_offset<P>(S + 1) + 2 * k;
-            cpx<T>        a[R];
-            static_for<R / 2>([&](auto qc) {
-                constexpr int q = decltype(qc)::value;
-                cpx<T>        w0, w1;
-                ld2<SH>(tw + (q << (NSB + 1)), w0, w1);
-                a[2 * q]     = q == 0 ? v[g] : cmul(v[g + 2 * q * GN], w0);
-                a[2 * q + 1] = cmul(v[g + (2 * q + 1) * GN], w1);
-            });
-            stage_dft(a);
-            static_for<R>([&](auto jc) {
-                constexpr int j = decltype(jc)::value;
-                v[g + j * GN]   = a[j];
-            });
-        });
+        stage_exchange<P, S, X, BARN>(v, xch, m, t);
+        stage_apply_rows<P, S + 1, SH, false>(v, t, tab + rows_tw_offset<P>(S + 1));
     });
 }
 

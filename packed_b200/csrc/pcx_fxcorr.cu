@@ -189,12 +189,12 @@ int grid_xc3(K kern, long long total, int sms, int* grid) {
     return PCX_OK;
 }
 template<int LOGN>
-int launch_xc3(const xc_args& a, const void* stw, cudaStream_t st, int sms) {
+int launch_xc3(const xc_args& a, const void* stw, const void* full, cudaStream_t st, int sms) {
     using C  = xc3_cfg<LOGN>;
     int grid = 0;
     if (int rc = grid_xc3<LOGN>(k_fxcorr3<LOGN>, a.total, sms, &grid)) return rc;
     if (a.total == 0) return PCX_OK;    // launch attributes only
-    k_fxcorr3<LOGN><<<(unsigned)grid, C::NT, C::SMEM, st>>>(a, stw);
+    k_fxcorr3<LOGN><<<(unsigned)grid, C::NT, C::SMEM, st>>>(a, stw, full);
     PCX_CUDA_TRY(cudaGetLastError());
     return PCX_OK;
 }
@@ -208,15 +208,15 @@ int launch_xc3_kg(const kg_args& a, const void* stw, cudaStream_t st, int sms, i
     PCX_CUDA_TRY(cudaGetLastError());
     return PCX_OK;
 }
-int dispatch_xc3(int log_n, const xc_args& a, const void* stw, cudaStream_t st, int sms) {
+int dispatch_xc3(int log_n, const xc_args& a, const void* stw, const void* full, cudaStream_t st, int sms) {
     switch (log_n) {
-    case 6: return launch_xc3<6>(a, stw, st, sms);
-    case 7: return launch_xc3<7>(a, stw, st, sms);
-    case 8: return launch_xc3<8>(a, stw, st, sms);
-    case 9: return launch_xc3<9>(a, stw, st, sms);
-    case 10: return launch_xc3<10>(a, stw, st, sms);
-    case 11: return launch_xc3<11>(a, stw, st, sms);
-    default: return launch_xc3<12>(a, stw, st, sms);
+    case 6: return launch_xc3<6>(a, stw, full, st, sms);
+    case 7: return launch_xc3<7>(a, stw, full, st, sms);
+    case 8: return launch_xc3<8>(a, stw, full, st, sms);
+    case 9: return launch_xc3<9>(a, stw, full, st, sms);
+    case 10: return launch_xc3<10>(a, stw, full, st, sms);
+    case 11: return launch_xc3<11>(a, stw, full, st, sms);
+    default: return launch_xc3<12>(a, stw, full, st, sms);
     }
 }
 int dispatch_xc3_kg(int log_n, const kg_args& a, const void* stw, cudaStream_t st, int sms, int* grid) {
@@ -322,7 +322,7 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     // packs, rows of packs 16-byte aligned
     const bool rows = pack == 8 && a.in_shift % 8 == 0 && (channels == 1 || sstride % 4 == 0) &&
                       reinterpret_cast<uintptr_t>(src) % 16 == 0;
-    if (h->x3 && rows) return dispatch_xc3(h->log_n, a, h->plan->stwL, st, h->sms);
+    if (h->x3 && rows) return dispatch_xc3(h->log_n, a, h->plan->stwL, h->plan->s3_any, st, h->sms);
     if (h->xi && rows) {
         xci_args b{};
         b.base  = a;
@@ -435,6 +435,10 @@ int init_handle(pcx_fxcorr_s* h) {
     const size_t eb    = f64 ? 16 : 8;
     PCX_CUDA_TRY(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device));
     if (int rc = pcx_plan_create(&h->plan, h->n, h->dtype, PCX_ORDER_NORMAL, 2048)) return rc;
+    // K rounds as the windows' transforms do where it has their stages, and part
+    // of the error cancels (1024 points at pack 1: 2.035e-7 so, 2.059e-7 with K
+    // in 32-point stages)
+    h->plan->narrow = log_n <= 12;
     PCX_CUDA_TRY(cudaMalloc(&h->tw, h->n * eb));
     PCX_CUDA_TRY(cudaMalloc(&h->kspec, h->n * eb + sizeof(int)));
     h->err = reinterpret_cast<int*>(static_cast<char*>(h->kspec) + h->n * eb);
@@ -451,7 +455,7 @@ int init_handle(pcx_fxcorr_s* h) {
         // its launch attributes now, not in a call that may be captured
         int grid = 0;
         if (int rc = dispatch_xc3_kg(log_n, kg_args{}, nullptr, 0, h->sms, &grid)) return rc;
-        if (int rc = dispatch_xc3(log_n, xc_args{}, nullptr, 0, h->sms)) return rc;
+        if (int rc = dispatch_xc3(log_n, xc_args{}, nullptr, nullptr, 0, h->sms)) return rc;
         h->x3 = true;
     }
     if (!f64 && log_n >= 13 && !h->general) return log_n == 14 ? init_xci<14>(h) : init_xci<13>(h);
@@ -500,8 +504,8 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
             // owner may still be running: what follows is on the default
             // stream, which no non-blocking stream is ordered with
             PCX_CUDA_TRY(cudaDeviceSynchronize());
-            PCX_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), 0));
             if (int rc = set_kernel(h, g)) return rc;
+            PCX_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), 0));
             PCX_CUDA_TRY(cudaStreamSynchronize(0));    // g is read, the tables and K are there
             return PCX_OK;
         };

@@ -18,6 +18,12 @@
 // flight during a block, sub-transform twiddles and kernel spectrum from
 // global memory) 98 us, this one 34 us; kernel gradient 182 and
 // 34 us (device times).
+// Accuracy: full tables for all stages would leave room for one block an SM.
+// With factors in all of them and butterflies by halves the error is 5 % above
+// the general kernel's; a full table for the second stage (small) and radix-16
+// butterflies as 4 x 4 bring it below at the same speed.  4096 points, 1024
+// taps, against FP64: general 2.469e-7, by halves 2.649e-7, this 2.403e-7.  (The
+// kernel gradient's sums differ anyway: 3.25e-7 in the general form, 2.78e-7.)
 //
 // In place, a tile's outputs overwrite samples that the windows of earlier
 // tiles still read, so tiles are claimed in order from a counter, a block
@@ -46,8 +52,14 @@ struct xc3_cfg {
     static constexpr int TILE = M * RS;
     static constexpr int SW   = TT >= 32 ? 16 : 0;
     using X                   = xch_blocked<N, M>;
+    // twiddles: the correlator's second stage reads a full table (from 128
+    // points on: FULL entries), later ones factors
+    static constexpr int FULL = LOGN > 6 ? 1 << (4 + P::rbits(1)) : 0;
     static constexpr int TAB  = smem_align16(stage_tw_smem_bytes<P, float>());
-    static constexpr int SMEM = 2 * TILE * 4 + X::size * 8 + TAB;
+    static constexpr int SKIP = FULL ? stage_tw_offset<P>(2) : 0;    // factors that the full table stands for
+    static constexpr int TAB2 = (FULL + stage_tw_size<P>() - SKIP) * 8;
+    static constexpr int BASE = 2 * TILE * 4 + X::size * 8;
+    static constexpr int SMEM = BASE + (TAB > TAB2 ? TAB : TAB2);
     static_assert((RS * 4) % 16 == 0 && (X::size * 8) % 16 == 0, "16-byte sections");
     static_assert(P::E == 16 && P::NST > 1, "16 points per thread");
     static_assert(2 * (SMEM + 1024 + 256) <= 233472, "two blocks per SM");
@@ -70,8 +82,29 @@ __device__ __forceinline__ void xc3_clip(cpx<float> (&v)[16], int t, int lo, int
     });
 }
 
+// A window's transform, frequency t + i*TT into v[i].
+template<int LOGN, int BAR>
+__device__ __forceinline__ void xc3_transform(cpx<float> (&v)[16], cpx<float>* xch, int m, int t, const cpx<float>* tab) {
+    using F = xc3_cfg<LOGN>;
+    using P = typename F::P;
+    using X = typename F::X;
+    stage_compute_tab<P, 0, true>(v, t, tab);
+    static_for<P::NST - 1>([&](auto sc) {
+        constexpr int S = decltype(sc)::value;
+        stage_exchange<P, S, X, BAR>(v, xch, m, t);
+        if constexpr (S == 0 && F::FULL > 0) {
+            stage_apply_rows<P, 1, true, true>(v, t, tab);
+        } else {
+            cpx<float> f[(16 >> P::rbits(S + 1)) * stw_q(P::rbits(S + 1))];
+            load_stage_tw<P, S + 1, true>(f, t, tab + F::FULL - F::SKIP);
+            stage_apply_tw<P, S + 1, true>(v, f);
+        }
+    });
+}
+
+// full_g: the second stage's full table (not read below 128 points).
 template<int LOGN>
-__global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g) {
+__global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g, const void* full_g) {
     using F           = xc3_cfg<LOGN>;
     using P           = typename F::P;
     using X           = typename F::X;
@@ -97,7 +130,11 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
     const long long       ntile = (a.total + M - 1) / M;
     const int             htile = (a.hwait + M - 1) / M;    // earlier tiles to wait for, in place
 
-    stage_tw_to_smem<P, float>(stw, stw_g, tid, NT);
+    if constexpr (F::FULL > 0) copy_table_to_smem<F::FULL * 8>(stw, full_g, tid, NT);
+    if constexpr (stage_tw_size<P>() > F::SKIP) {
+        copy_table_to_smem<(stage_tw_size<P>() - F::SKIP) * 8>(stw + F::FULL, static_cast<const cpx<float>*>(stw_g) + F::SKIP,
+                                                               tid, NT);
+    }
     if (tid < 32) {
         tmem_alloc(&s_tmem, 64);
         tmem_relinquish();
@@ -201,8 +238,7 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
         fence_proxy_async_smem();
         __syncthreads();    // stage s and its windows are read: refill them
         if (tid < 32) issue(s);
-        stage_compute_tab<P, 0>(v, t, stw);
-        run_stages_tab<P, X, true, BAR>(v, xch, m, t, stw);
+        xc3_transform<LOGN, BAR>(v, xch, m, t, stw);
         // conj(X * conj(K)) or conj(X * K), K eight values at a time
         __syncwarp();
         static_for<2>([&](auto hc) {
@@ -221,8 +257,7 @@ __global__ void __launch_bounds__(256, 2) k_fxcorr3(xc_args a, const void* stw_g
         const int lane = tid % 32;
         bool      seen = true;
         if (a.inplace && lane < htile && lane < tile) seen = ld_acquire(a.flags + (tile - 1 - lane)) != 0u;
-        stage_compute_tab<P, 0>(v, t, stw);
-        run_stages_tab<P, X, true, BAR>(v, xch, m, t, stw);
+        xc3_transform<LOGN, BAR>(v, xch, m, t, stw);
         if (a.inplace) {
             // every warp waits for itself, so that no barrier holds the outputs
             // of those that are done; one that gives up stores nothing, and the

@@ -179,6 +179,7 @@ struct pcx_plan_s {
     void*  stw_rows = nullptr;    // one-pass sizes from 128 points on: pcx_rows_twiddles' tables
     const void* rows_fac = nullptr;    // factors of k_rows' default form (null: stwL serves)
     const void* rows_any = nullptr;    // full tables of k_rows' any-pack form
+    bool        narrow   = false;      // never 32 points per thread in k_rows (a correlator's plan)
     const void* s3_any   = nullptr;    // full tables of k_single3's (null: below 128 points)
     void*  fst      = nullptr;    // one-launch four-step: full stage tables of N1 then N2 (one allocation)
     void*  fst1     = nullptr;

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import oracle as O
-from packed_b200 import default_pack_size, fft_order, fft_unit
+from packed_b200 import default_pack_size, fft_order, fft_unit, fxcorr_unit
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +63,28 @@ def test_fourstep_forms(lg, order, monkeypatch):
     one = _error(unit, x, n, 1, 1, pos)
     monkeypatch.setenv("PCX_FOURSTEP", "chunked")
     assert one < 1.004 * _error(unit, x, n, 1, 1, pos)
+
+
+@pytest.mark.parametrize("lg", range(7, 13))
+@pytest.mark.parametrize("part", [4, 2])
+def test_correlators(lg, part, monkeypatch):
+    """The whole-window correlator and its signal gradient against the general kernel that ran these
+    sizes before it, which has full twiddle tables (0.4 % for the data's chance)."""
+    n, channels, length = 1 << lg, 16, 1 << 16
+    k, m = n // part, 1 << 17
+    rng = np.random.default_rng(lg)
+    g = ((rng.standard_normal(k) + 1j * rng.standard_normal(k)) / np.sqrt(2 * k)).astype(np.complex64)
+    unit = fxcorr_unit(g, n)
+    monkeypatch.setenv("PCX_XC_GENERAL", "1")
+    general = fxcorr_unit(g, n)
+    x = torch.randn(channels, 2 * length, device="cuda", generator=torch.Generator("cuda").manual_seed(lg))
+    spec, gs = torch.fft.fft(_cx(x, length, 8), m), torch.fft.fft(torch.as_tensor(g.astype(complex), device="cuda"), m)
+    for want, run in ((torch.fft.ifft(spec * gs.conj()), lambda u, y: u.exec(y, x, length, channels=channels)),
+                      (torch.fft.ifft(spec * gs),
+                       lambda u, y: y.copy_(u.vjp(x, x, length, channels=channels, want_kernel_grad=False)[0]))):
+        want, err = want[:, :length], []
+        for u in (unit, general):
+            y = torch.empty_like(x)
+            run(u, y)
+            err.append(((_cx(y, length, 8) - want).norm() / want.norm()).item())
+        assert err[0] < 1.004 * err[1], err
