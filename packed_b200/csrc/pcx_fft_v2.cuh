@@ -851,11 +851,18 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>
             static_for<E>([&](auto ic) {
                 constexpr int i = decltype(ic)::value;
                 if (t + i * TT >= a.src_len) v[i] = {T(0), T(0)};
-                if (tail && t + i * TT == a.src_len - 1 && tile * M + m < a.batch) {
-                    const T* g = src + (tile * M + m) * a.src_stride + 2 * (t + i * TT);
-                    v[i]       = {g[0], g[1]};
-                }
             });
+            if (tail) {
+                cpx<T> z = {T(0), T(0)};
+                if (t == (a.src_len - 1) % TT && tile * M + m < a.batch) {
+                    const T* g = src + (tile * M + m) * a.src_stride + 2 * (a.src_len - 1);
+                    z          = {g[0], g[1]};
+                }
+                static_for<E>([&](auto ic) {
+                    constexpr int i = decltype(ic)::value;
+                    if (t + i * TT == a.src_len - 1) v[i] = z;
+                });
+            }
         }
         fence_proxy_async_smem();
         // every thread has read the tile (this barrier is also the vote on a
