@@ -760,7 +760,10 @@ __host__ __device__ constexpr uint32_t single3_row_bytes(int len, int lp) {
 // conflicts at widths 1..16, so the form costs an index per element (none in
 // natural order with packs of at most TT elements: one base per thread).
 // Bound by the load/store pipe and HBM like the default form.
-template<class T, int LOGL, int LP, bool ANY>
+// NAT: outputs in natural order, straight from registers (with s3_cfg::DIRECT);
+// one kernel for both kinds of order spilled registers in FP64 (4096 points,
+// into unordered order, 2770 GB/s in one kernel, 2900 apart).
+template<class T, int LOGL, int LP, bool ANY, bool NAT>
 __global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>::MINB) k_single3(v3_args a) {
     using F             = s3_cfg<T, LOGL, ANY>;
     using P             = typename F::P;
@@ -886,7 +889,7 @@ __global__ void __launch_bounds__(s3_cfg<T, LOGL, ANY>::NT, s3_cfg<T, LOGL, ANY>
         else run_stages_tab<P, X, SH, (TT <= 32 ? -1 : 0)>(v, xch, m, t, stw);
         const T sc  = T(a.scale);
         const T sim = a.conj_out ? -sc : sc;
-        if (F::DIRECT && a.order_out == 0) {
+        if constexpr (NAT) {
             // v[i] is frequency t + i*TT: neighbouring threads store neighbouring reals
             if (tile * M + m < a.batch) {
                 T* d = dst + (tile * M + m) * a.dst_stride;

@@ -48,8 +48,13 @@ cudaError_t launch_single3(const v3_args& a, cudaStream_t st, int sms, bool attr
     constexpr int NT    = F::NT;
     constexpr int M     = F::M;
     constexpr int bytes = F::SMEM;
-    auto          kern  = k_single3<T, LOGL, v2cfg<T>::LP, ANY>;
-    if (attr_only) return smem_attr_cached(reinterpret_cast<const void*>(kern), bytes);
+    const auto    nat   = k_single3<T, LOGL, v2cfg<T>::LP, ANY, F::DIRECT>;
+    const auto    perm  = k_single3<T, LOGL, v2cfg<T>::LP, ANY, false>;
+    if (attr_only) {
+        const cudaError_t e = smem_attr_cached(reinterpret_cast<const void*>(nat), bytes);
+        return e != cudaSuccess ? e : smem_attr_cached(reinterpret_cast<const void*>(perm), bytes);
+    }
+    const auto kern = a.order_out == 0 ? nat : perm;
     const long long tiles = (a.batch + M - 1) / M;
     if (tiles == 0) return cudaSuccess;
     unsigned    grid = 0;
