@@ -92,12 +92,14 @@ struct fs_args {
 //    The scratch keeps the columns in the order r, and a row tile reads its
 //    n2 from bitrev(n2), again one run of 16 per thread.
 // 2^15, 301 transforms, forward into `unordered` and inverse back: two
-// launches per chunk of general kernels 427 us, these 119 us.
-constexpr int FS_TS_ROUNDS = 12;
+// launches per chunk of general kernels 427 us, these 121 us.
 constexpr int FS_PLAIN = 0;
 constexpr int FS_ANY   = 1;
 constexpr int FS_OUT   = 2;
 constexpr int FS_IN    = 3;
+
+// Items a block from which outputs are stored by TMA (fs_cfg::TS).
+constexpr int FS_TS_ROUNDS = 12;
 
 // Register i of the 16 a thread holds (element t + i*TT) at place q of its run
 // of 16 consecutive positions: i = bitrev4(q), or bitrev4(sigma(q)) in the

@@ -75,12 +75,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // Order this thread's earlier generic-proxy shared-memory accesses before
 // later async-proxy (TMA) accesses to the same memory.  Every thread that
 // read a stage runs it before the barrier that precedes the refill.
+__device__ __forceinline__ void fence_proxy_async_smem() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 // A tensor map in global memory that the host wrote, before copies that use it.
 __device__ __forceinline__ void fence_tensormap_acquire(const void* map) {
     asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
 // 1-D bulk copy global -> shared (16-byte aligned addresses, size multiple
