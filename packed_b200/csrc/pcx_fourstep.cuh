@@ -253,15 +253,18 @@ __device__ __forceinline__ void red_release_add(int* p, int v) {
 // B*a + b, as W_N^((t + B*a*TT)*n2) (row a*TT + t) times u^b, u = W_N^(TT*n2)
 // (row N1/B + b - 1), all generated in FP64 and rounded once; a row of N2 entries
 // is read by neighbouring columns at once.  The fewer of them are products the
-// smaller the error and the more entries a thread reads (9 with B = 2, 7 with
-// 4): B = 2 where B = 4 would be less accurate than the general kernels (product
-// of two half-size tables).  Error against FP64, interleaved to packed: 2^15
-// general 1.439e-7, B = 4 1.447e-7, B = 2 1.434e-7, one entry times powers of u
-// 1.472e-7; 2^17 1.573e-7, 1.573e-7, -, 1.597e-7.  GB/s, 512 MB: 2^15 3292
-// with powers of u, 3231 with B = 4 and 3210 with 2; 2^20 2800, 2672 and 2542.
+// smaller the error and the larger the table: B = 2 (9 entries a thread) where 4
+// (7 entries) would be less accurate than the general kernels, whose twiddles
+// are products of two half-size tables' entries; 8 and 16 (9 and 16) where the
+// table would pass 2 MB, whose allocation adds 0.35 ms to a plan's creation.
+// Error against FP64, interleaved to packed, general kernels, one entry times
+// powers of u (up to three products), B = 4, B = 2: 2^15 1.439e-7 1.472e-7
+// 1.447e-7 1.434e-7; 2^17 1.573e-7 1.597e-7 1.573e-7 -; 2^20 1.691e-7 1.711e-7
+// 1.69e-7 - (B = 8 1.69e-7).  GB/s, 512 MB: 2^15 - 3292 3231 3210, 2^20 - 2800
+// 2672 - (2604).
 template<class T>
 __host__ __device__ constexpr int fs_tw_group(int log_n) {
-    return sizeof(T) == 4 && log_n <= 16 ? 2 : 4;
+    return sizeof(T) == 4 ? (log_n <= 16 ? 2 : log_n <= 19 ? 4 : 8) : (log_n <= 18 ? 4 : log_n <= 19 ? 8 : 16);
 }
 template<class T>
 __host__ __device__ constexpr int fs_tw_rows(int log_n1, int log_n) {
