@@ -465,7 +465,7 @@ struct xch_blocked32 {
 // shared memory both ways, 16 warps an SM (FP64: 8):
 //   N            256  512 1024 2048 4096 8192 16384  FP64: 128  256  512 1024 2048 4096 8192
 //   before      5917 4944 4436 4544 4526 3255  3404       4364 4982 4073 3516 3658 3860 1833
-//   this        6703 6470 6488 6026 5654 5092  3690       6726 6722 5954 5049 5309 5095 3316
+//   this        6703 6455 6530 6026 5654 5127  3690       6726 6722 5954 5049 5309 5095 3316
 //   16 points   6703 6220 5575           4228  3043
 //   256 threads 6729 5690 5720 5773                       6587 6798 5576 4557 4901
 // (8192 and 16384 before: 3500 and 3404 in the four-step's tuned form.)  4096
@@ -758,8 +758,9 @@ __host__ __device__ constexpr uint32_t single3_row_bytes(int len, int lp) {
 // at run time) and rows shorter than N.  The row is the same 2*N contiguous
 // reals at every width and lds_swapped / sts_swapped stay free of bank
 // conflicts at widths 1..16, so the form costs an index per element (none in
-// natural order with packs of at most TT elements: one base per thread).
-// Bound by the load/store pipe and HBM like the default form.
+// natural order with packs of at most TT elements: one base per thread) and, from
+// 128 points on, the loads of its full tables (s3_cfg::FULL).  Bound by the
+// load/store pipe and HBM like the default form.
 // NAT: outputs in natural order, straight from registers (with s3_cfg::DIRECT);
 // one kernel for both kinds of order spilled registers in FP64 (4096 points,
 // into unordered order, 2770 GB/s in one kernel, 2900 apart).

@@ -307,7 +307,7 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
     // output b*step, and output m of the block is circular index m + shift.
     // Any shift >= K-1 with step + shift <= N gives the same outputs; at pack 8
     // K-1 rounded up to whole packs is one (step = N - shift), and it keeps
-    // the windows on whole packs, as the four-step form below needs.
+    // the windows on whole packs, as the forms below need.
     const size_t shift = pack == 8 ? (h->k - 1 + 7) / 8 * 8 : h->k - 1;
     a.in_shift    = convolve ? (int)shift : 0;
     a.out_shift   = convolve ? (int)shift : 0;
@@ -355,8 +355,8 @@ void free_handle(pcx_fxcorr_s* h) {
 // ten times its kernels.  What is reused is memory and the tables that depend
 // on the size alone; a handle has one owner at a time, and the kernel's
 // spectrum is computed anew for each.  At most 4 idle handles and 64 MB of
-// their growing buffers are kept, the oldest goes first, and all go when an
-// allocation fails.
+// their growing buffers are kept, the oldest goes first, and all go when making
+// a handle fails for want of memory.
 class handle_pool {
 public:
     static constexpr size_t MAX_IDLE  = 4;
