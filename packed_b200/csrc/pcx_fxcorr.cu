@@ -11,6 +11,7 @@
 #include <list>
 #include <mutex>
 #include <string>
+#include <vector>
 
 using namespace pcxg;
 
@@ -23,7 +24,7 @@ struct pcx_fxcorr_s {
     pcx_plan_s* plan   = nullptr;    // natural-order N-point FFT (kernel spectrum, gradient inverse)
     void*       tw     = nullptr;    // W_N^i, i < N
     void*       kspec  = nullptr;    // FFT(g)/N, interleaved complex, natural order
-    int*        err    = nullptr;    // error flag, behind kspec
+    int*        err    = nullptr;    // error flag (host memory, see flag_words)
     unsigned*   ctl    = nullptr;    // in-place calls: [0] work counter, [1..] "window loaded" flags
     size_t      flags_cap = 0;
     void*       gscratch  = nullptr;    // kernel-gradient accumulators
@@ -338,6 +339,38 @@ int run_xc(pcx_fxcorr_s* h, void* dst, const void* src, size_t len, int pack, si
 
 namespace {
 
+// Error flags of the handles: words of page-locked host memory that a kernel
+// writes only when a wait gives up, so that neither clearing one for a new owner
+// nor reading it takes a copy (3 and 8 us of a training step).
+class flag_words {
+public:
+    cudaError_t take(int** out) {
+        std::lock_guard<std::mutex> g(mu_);
+        if (free_.empty()) {
+            int*              block = nullptr;
+            const cudaError_t e     = cudaHostAlloc(&block, 1024 * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+            if (e != cudaSuccess) return e;
+            for (int i = 0; i < 1024; i += 16) free_.push_back(block + i);    // a cache line each
+        }
+        *out = free_.back();
+        free_.pop_back();
+        return cudaSuccess;
+    }
+    void give(int* p) {
+        std::lock_guard<std::mutex> g(mu_);
+        free_.push_back(p);
+    }
+
+private:
+    std::mutex        mu_;
+    std::vector<int*> free_;
+};
+flag_words& flags() {
+    static flag_words* f = new flag_words;    // never destroyed, as the pool below
+    return *f;
+}
+
+// Its memory goes after the frees, which wait for the device.
 void free_handle(pcx_fxcorr_s* h) {
     if (h->plan) pcx_plan_destroy(h->plan);
     if (h->tw) cudaFree(h->tw);
@@ -345,6 +378,7 @@ void free_handle(pcx_fxcorr_s* h) {
     if (h->ctl) cudaFree(h->ctl);
     if (h->gscratch) cudaFree(h->gscratch);
     if (h->xi) cudaFree(h->xi);
+    if (h->err) flags().give(h->err);
     delete h;
 }
 
@@ -440,8 +474,8 @@ int init_handle(pcx_fxcorr_s* h) {
     // in 32-point stages)
     h->plan->narrow = log_n <= 12;
     PCX_CUDA_TRY(cudaMalloc(&h->tw, h->n * eb));
-    PCX_CUDA_TRY(cudaMalloc(&h->kspec, h->n * eb + sizeof(int)));
-    h->err = reinterpret_cast<int*>(static_cast<char*>(h->kspec) + h->n * eb);
+    PCX_CUDA_TRY(cudaMalloc(&h->kspec, h->n * eb));
+    PCX_CUDA_TRY(flags().take(&h->err));
     PCX_CUDA_TRY(pcx_gen_twiddles(h->tw, (int)h->n, log_n, 1, f64, 0));
     if (int rc = f64 ? dispatch_xc<double>(log_n, xc_args{}, nullptr, 0, 0, true)
                      : dispatch_xc<float>(log_n, xc_args{}, nullptr, 0, 0, true)) {
@@ -504,8 +538,8 @@ extern "C" int pcx_fxcorr_create(pcx_fxcorr* out, const void* g, size_t k, int p
             // owner may still be running: what follows is on the default
             // stream, which no non-blocking stream is ordered with
             PCX_CUDA_TRY(cudaDeviceSynchronize());
+            *h->err = 0;
             if (int rc = set_kernel(h, g)) return rc;
-            PCX_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), 0));
             PCX_CUDA_TRY(cudaStreamSynchronize(0));    // g is read, the tables and K are there
             return PCX_OK;
         };
@@ -554,10 +588,9 @@ extern "C" int pcx_fxcorr_exec(pcx_fxcorr h, void* dst, const void* src, size_t 
 extern "C" int pcx_fxcorr_status(pcx_fxcorr h) {
     return pcx_guard([&]() -> int {
         if (!h) return pcx_fail(PCX_ERR_INVALID, "handle is null");
-        int err = 0;
-        PCX_CUDA_TRY(cudaMemcpy(&err, h->err, sizeof(int), cudaMemcpyDeviceToHost));
-        if (err) {
-            PCX_CUDA_TRY(cudaMemset(h->err, 0, sizeof(int)));
+        PCX_CUDA_TRY(cudaStreamSynchronize(0));
+        if (*static_cast<volatile int*>(h->err)) {
+            *h->err = 0;
             return pcx_fail(PCX_ERR_TIMEOUT, "a correlation block gave up a bounded wait (for its input copy or, in place, for its predecessor)");
         }
         return PCX_OK;
