@@ -170,6 +170,49 @@ size_t pcx_plan_s::chunk_rows(size_t batch) const {
     return std::min(c, std::max<size_t>(batch, 1));
 }
 
+// Twiddle table of the kernel's other forms for variant `v`, by column or (twr)
+// by bit-reversed column, filled on `st`.
+static cudaError_t fs_form_table(const pcx_plan_s* p, const fs_variant& v, bool reversed, cudaStream_t st, void** out) {
+    const bool     f64     = p->dtype == PCX_F64;
+    const size_t   entries = (size_t)(f64 ? fs_tw_rows<double>(v.l1, p->log_n) : fs_tw_rows<float>(v.l1, p->log_n)) << v.l2;
+    const unsigned grid    = (unsigned)((entries + 255) / 256);
+    void*          o       = nullptr;
+    cudaError_t    e       = cudaMalloc(&o, entries * p->elem_bytes());
+    if (e != cudaSuccess) return e;
+    if (f64) k_fs_twiddles<double><<<grid, 256, 0, st>>>(static_cast<cpx<double>*>(o), v.l1, v.l2, reversed);
+    else k_fs_twiddles<float><<<grid, 256, 0, st>>>(static_cast<cpx<float>*>(o), v.l1, v.l2, reversed);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) *out = o;
+    else cudaFree(o);
+    return e;
+}
+
+// Whether the plan has the forms' tables.  Plans of a permuted order are made
+// with them, as every call of theirs is one of a form; a natural-order plan gets
+// them with the first call of other packs or a short source (they would double
+// its memory and cost its creation up to 0.35 ms), unless that call is being
+// captured or there is no memory: the two-launch kernels, which need no table,
+// serve it then.
+static bool fs_form_ready(pcx_plan_s* p, cudaStream_t st) {
+    std::lock_guard<std::mutex> g(p->mu);
+    if (p->fs_def.tw) return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStream_t            s  = nullptr;
+    cudaError_t             e  = cudaStreamIsCapturing(st, &cs);
+    if (e == cudaSuccess && cs != cudaStreamCaptureStatusNone) return false;
+    if (e == cudaSuccess) e = setup_stream(&s);
+    void* tw = nullptr;
+    if (e == cudaSuccess) e = fs_form_table(p, p->fs_def.var, false, s, &tw);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) {
+        p->fs_def.tw = tw;
+        return true;
+    }
+    if (tw) cudaFree(tw);
+    (void)cudaGetLastError();
+    return false;
+}
+
 // Make `v` the plan's one-launch four-step variant: its split's tables (W_N
 // tables, W_{16 N2}, full stage tables), generated again only when the split
 // changes, and its tile counts and resident blocks per SM.  The first variant
@@ -199,12 +242,7 @@ static int fs_select(pcx_plan_s* p, const fs_variant& v) {
         int          f1 = 0, f2 = 0;
         PCX_CUDA_TRY(pcx_fourstep_tables(v.l1, nullptr, f64, 0, &f1));
         PCX_CUDA_TRY(pcx_fourstep_tables(v.l2, nullptr, f64, 0, &f2));
-        // the default variant, which the kernel's other forms run, has their
-        // twiddle table as well, plans of a permuted order a second one by
-        // bit-reversed column
-        const size_t tw = (size_t)(f64 ? fs_tw_rows<double>(v.l1, p->log_n) : fs_tw_rows<float>(v.l1, p->log_n)) * n2;
-        const size_t nt = p->fs_def.mem ? 0 : (p->order != PCX_ORDER_NORMAL ? 2 : 1);
-        PCX_CUDA_TRY(cudaMalloc(&c.mem, ((size_t)n1 + 2 * (size_t)n2 + f1 + f2 + nt * tw) * eb));
+        PCX_CUDA_TRY(cudaMalloc(&c.mem, ((size_t)n1 + 2 * (size_t)n2 + f1 + f2) * eb));
         char* b = static_cast<char*>(c.mem);
         c.thi   = b;
         c.tlo   = b + (size_t)n1 * eb;
@@ -216,14 +254,6 @@ static int fs_select(pcx_plan_s* p, const fs_variant& v) {
         if (e == cudaSuccess) e = pcx_gen_twiddles(c.tb, n2, v.l2 + 4, 1, f64, 0);
         if (e == cudaSuccess) e = pcx_fourstep_tables(v.l1, c.st1, f64, 0, &f1);
         if (e == cudaSuccess) e = pcx_fourstep_tables(v.l2, c.st2, f64, 0, &f2);
-        for (size_t i = 0; i < nt && e == cudaSuccess; ++i) {
-            const unsigned grid = (unsigned)((tw + 255) / 256);
-            void*          o    = b + ((size_t)n1 + 2 * (size_t)n2 + f1 + f2 + i * tw) * eb;
-            (i ? c.twr : c.tw)  = o;
-            if (f64) k_fs_twiddles<double><<<grid, 256>>>(static_cast<cpx<double>*>(o), v.l1, v.l2, i);
-            else k_fs_twiddles<float><<<grid, 256>>>(static_cast<cpx<float>*>(o), v.l1, v.l2, i);
-            e = cudaGetLastError();
-        }
         if (e != cudaSuccess) {
             cudaFree(c.mem);
             PCX_CUDA_TRY(e);
@@ -236,10 +266,10 @@ static int fs_select(pcx_plan_s* p, const fs_variant& v) {
     return PCX_OK;
 }
 
-// The built-in variants of the one-launch four-step for this plan's size.
 // Transforms that a plan's four-step counters are made for at its creation.
 constexpr size_t FS_BATCH = 4096;
 
+// The built-in variants of the one-launch four-step for this plan's size.
 static std::vector<fs_variant> fs_candidates(const pcx_plan_s* p) {
     std::vector<fs_variant> out;
     if (p->dtype == PCX_F64) {
@@ -332,6 +362,10 @@ static int plan_init_tables(pcx_plan_s* p) {
             // one launch for a whole batch: the size's first built-in variant
             for (const fs_variant& v: fs_candidates(p)) {
                 if (fs_select(p, v) == PCX_OK) break;
+            }
+            if (p->fs_def.tc > 0 && p->order != PCX_ORDER_NORMAL) {
+                PCX_CUDA_TRY(fs_form_table(p, p->fs_def.var, false, 0, &p->fs_def.tw));
+                PCX_CUDA_TRY(fs_form_table(p, p->fs_def.var, true, 0, &p->fs_def.twr));
             }
             if (p->fs.tc > 0) {    // counters of a usual batch, so that no call has to allocate them
                 PCX_CUDA_TRY(cudaMalloc(&p->fs_ctr, (2 * FS_BATCH + 1) * sizeof(int)));
@@ -434,6 +468,8 @@ void pcx_plan_s::release() {
     if (fst) cudaFree(fst);
     if (fs.mem && fs.mem != fs_def.mem) cudaFree(fs.mem);
     if (fs_def.mem) cudaFree(fs_def.mem);
+    if (fs_def.tw) cudaFree(fs_def.tw);
+    if (fs_def.twr) cudaFree(fs_def.twr);
     fs     = {};
     fs_def = {};
     if (fs_ctr) cudaFree(fs_ctr);
@@ -942,7 +978,7 @@ int pcx_fft_run(pcx_plan_s* p, void* dst, const void* src, size_t src_len, int p
     const bool fs_form     = !fs_plain && p->fs_def.tc > 0 && (size_t(1) << p->fs_def.var.l2) <= src_len &&
                          (!perm || lp_perm == 0 || lp_perm == lp_def);
     if (!ws && tuned_fused && use_tma && p->fs.tc > 0 && (fs_plain || fs_form) &&
-        !(fs_env && std::strcmp(fs_env, "chunked") == 0)) {
+        !(fs_env && std::strcmp(fs_env, "chunked") == 0) && (fs_plain || fs_form_ready(p, st))) {
         const fs_choice& fc    = fs_plain ? p->fs : p->fs_def;
         const long long  per_t = fc.tc + fc.tr;
         // a row tile runs about `rounds` rounds of items (one item per CTA)

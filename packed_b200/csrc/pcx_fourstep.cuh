@@ -256,7 +256,7 @@ __device__ __forceinline__ void red_release_add(int* p, int v) {
 // smaller the error and the larger the table: B = 2 (9 entries a thread) where 4
 // (7 entries) would be less accurate than the general kernels, whose twiddles
 // are products of two half-size tables' entries; 8 and 16 (9 and 16) where the
-// table would pass 2 MB, whose allocation adds 0.35 ms to a plan's creation.
+// table would pass 2 MB, whose allocation takes 0.35 ms.
 // Error against FP64, interleaved to packed, general kernels, one entry times
 // powers of u (up to three products), B = 4, B = 2: 2^15 1.439e-7 1.472e-7
 // 1.447e-7 1.434e-7; 2^17 1.573e-7 1.597e-7 1.573e-7 -; 2^20 1.691e-7 1.711e-7

@@ -53,26 +53,29 @@ inline cudaError_t smem_attr_cached(const void* kern, int bytes) {
     return e;
 }
 
-// Zeroed device memory for counters that every launch leaves zero.  Filled and
-// waited for on a stream of its own, one per device and kept: on the caller's
-// stream the fill could become part of a capture that is never replayed, and on
-// the default one a launch on another stream could overtake it.
-inline cudaError_t alloc_zeroed(void** out, size_t bytes) {
+// A stream of the library's own, one per device and kept, for what a call has to
+// put into device memory once: on the caller's stream it could become part of a
+// capture that is never replayed, and on the default one a launch on another
+// stream could overtake it.
+inline cudaError_t setup_stream(cudaStream_t* out) {
     static std::mutex                  mu;
     static std::map<int, cudaStream_t> streams;
-    int          dev = 0;
-    void*        p   = nullptr;
-    cudaStream_t s   = nullptr;
-    cudaError_t  e   = cudaGetDevice(&dev);
+    int         dev = 0;
+    cudaError_t e   = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    {
-        std::lock_guard<std::mutex> g(mu);
-        cudaStream_t&               kept = streams[dev];
-        if (!kept) e = cudaStreamCreateWithFlags(&kept, cudaStreamNonBlocking);
-        if (e != cudaSuccess) return e;
-        s = kept;
-    }
-    e = cudaMalloc(&p, bytes);
+    std::lock_guard<std::mutex> g(mu);
+    cudaStream_t&               kept = streams[dev];
+    if (!kept) e = cudaStreamCreateWithFlags(&kept, cudaStreamNonBlocking);
+    *out = kept;
+    return e;
+}
+
+// Zeroed device memory for counters that every launch leaves zero.
+inline cudaError_t alloc_zeroed(void** out, size_t bytes) {
+    void*        p = nullptr;
+    cudaStream_t s = nullptr;
+    cudaError_t  e = setup_stream(&s);
+    if (e == cudaSuccess) e = cudaMalloc(&p, bytes);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(p, 0, bytes, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -93,11 +96,11 @@ struct fs_variant {
 // A variant with its tables (one allocation) and tile counts.
 struct fs_choice {
     fs_variant var{};                 // l1 == 0: none
-    void*      mem = nullptr;         // owns the tables below
+    void*      mem = nullptr;         // owns the tables below but the forms'
     void*      thi = nullptr;         // W_N^(i*N2), i < N1
     void*      tlo = nullptr;         // W_N^i, i < N2
     void*      tb  = nullptr;         // W_{16*N2}^i, i < N2
-    void*      tw  = nullptr;         // twiddles of the forms (the default variant only)
+    void*      tw  = nullptr;         // default variant: twiddles of the forms (natural order: made by the first call of one)
     void*      twr = nullptr;         // the same by bit-reversed column (plans of a permuted order)
     void*      st1 = nullptr;         // full stage tables of the N1- and N2-point sub-transforms
     void*      st2 = nullptr;

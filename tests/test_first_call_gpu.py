@@ -1,6 +1,6 @@
 """What the first call of a plan or correlator may still allocate: the scratch
-of a four-step transform and the flags of an in-place correlation, nothing to
-zero and wait for.  A first call, and one of a batch above what the counters
+of a four-step transform, the tables of its other forms and the flags of an
+in-place correlation, nothing to zero and wait for.  A first call, and one of a batch above what the counters
 were made for, give the results of the calls after them."""
 import numpy as np
 import pytest
@@ -43,6 +43,29 @@ def test_larger_batch_allocates_nothing():
     graph.replay()
     unit.exec(want, x, batch=500)
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("lg", [15, 20])
+def test_first_call_of_another_pack_captured(lg):
+    """The tables of the four-step's other forms are made by their first call; one that is being
+    captured, where nothing may be allocated, does without them."""
+    n, batch = 1 << lg, 3
+    x = torch.randn(batch, 2 * n, device="cuda")
+    y, direct = torch.zeros_like(x), torch.zeros_like(x)
+    unit = fft_unit(n)
+    unit.exec(y, x, batch=batch)    # the scratch is there
+    st, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st, capture_error_mode="global"):
+        unit.exec(y, x, batch=batch, pack_src=1, stream=st, check=False)
+    want = torch.fft.fft(torch.complex(*x.reshape(batch, n, 2).double().unbind(2)))
+    for _ in range(2):
+        y.fill_(float("nan"))
+        graph.replay()
+        unit.exec(direct, x, batch=batch, pack_src=1)
+        for out in (y, direct):
+            f = out.reshape(batch, -1, 2, 8).double()
+            got = torch.complex(f[:, :, 0].reshape(batch, n), f[:, :, 1].reshape(batch, n))
+            assert ((got - want).norm() / want.norm()).item() < TOL[np.float32]
 
 
 def test_more_transforms_than_the_counters_were_made_for():
